@@ -17,6 +17,7 @@
 // index, ties to the lowest indices.  The set of selected pools is the reference's whenever the k-th largest
 // score is unique; `cnt` is always the same.
 #include "internal.cuh"
+#include "sm100_prims.cuh"
 
 namespace gs {
 namespace {
@@ -28,22 +29,45 @@ __device__ __forceinline__ const float *idx_row(const float *chunk, const float 
 
 // grid (column blocks, max(1, completing pools)); thread = one column of one pool.  Only the first completing pool
 // (the one holding position p0) can reach into the rings; its threads also hand the trailing rows over afterwards.
+// A few hundred bytes per thread: the time is the chain of dependent memory round trips.  KP > 0 (kpool as a constant)
+// requests gates, keys and ape together, one round trip instead of three (a decode step, cold caches: 7.7 -> 3.0 us).
+template <int KP>
 __global__ void __launch_bounds__(128) k_idx_pool(const float *__restrict__ kc, const float *__restrict__ gc, float *rk, float *rg,
-                                                  const float *__restrict__ ape, float *__restrict__ P, int p0, int T, int Dk, int kpool) {
+                                                  const float *__restrict__ ape, float *__restrict__ P, int p0, int T, int Dk, int kpool_arg) {
+    sm100::griddep_launch_dependents();
+    const int kpool = KP > 0 ? KP : kpool_arg;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= Dk) return;
     const int end = p0 + T;
     const int jf = p0 / kpool, jl = end / kpool;
     const int64_t j = (int64_t) jf + blockIdx.y;
+    sm100::griddep_wait();
+    if (c >= Dk) return;
     if (j < jl) {
-        float mx = -INFINITY;
-        for (int m = 0; m < kpool; m++) mx = fmaxf(mx, idx_row(gc, rg, j * kpool + m, p0, Dk, kpool)[c] + ape[m * Dk + c]);
-        float sum = 0.f, acc = 0.f;
-        for (int m = 0; m < kpool; m++) {
-            const int64_t pos = j * kpool + m;
-            const float e = expf(idx_row(gc, rg, pos, p0, Dk, kpool)[c] + ape[m * Dk + c] - mx);
-            sum += e;
-            acc = fmaf(e, idx_row(kc, rk, pos, p0, Dk, kpool)[c], acc);
+        float mx = -INFINITY, sum = 0.f, acc = 0.f;
+        if (KP > 0) {
+            float g[KP > 0 ? KP : 1], k[KP > 0 ? KP : 1], a[KP > 0 ? KP : 1];
+#pragma unroll
+            for (int m = 0; m < KP; m++) {
+                g[m] = idx_row(gc, rg, j * kpool + m, p0, Dk, kpool)[c];
+                k[m] = idx_row(kc, rk, j * kpool + m, p0, Dk, kpool)[c];
+                a[m] = ape[m * Dk + c];
+            }
+#pragma unroll
+            for (int m = 0; m < KP; m++) mx = fmaxf(mx, g[m] + a[m]);
+#pragma unroll
+            for (int m = 0; m < KP; m++) {
+                const float e = expf(g[m] + a[m] - mx);
+                sum += e;
+                acc = fmaf(e, k[m], acc);
+            }
+        } else {
+            for (int m = 0; m < kpool; m++) mx = fmaxf(mx, idx_row(gc, rg, j * kpool + m, p0, Dk, kpool)[c] + ape[m * Dk + c]);
+            for (int m = 0; m < kpool; m++) {
+                const int64_t pos = j * kpool + m;
+                const float e = expf(idx_row(gc, rg, pos, p0, Dk, kpool)[c] + ape[m * Dk + c] - mx);
+                sum += e;
+                acc = fmaf(e, idx_row(kc, rk, pos, p0, Dk, kpool)[c], acc);
+            }
         }
         P[j * Dk + c] = acc / sum;
     }
@@ -101,121 +125,281 @@ __device__ __forceinline__ uint32_t f2ord(float f) {
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-constexpr int SEL_NT = 1024;
-// One block per query.  Radix select, 8 bits per pass from the top: after a pass `prefix` holds the leading bits of
-// the k-th largest value and `need` how many values are still to be taken among those that share the prefix.  The
-// 256 bins are scanned from the top by one warp (8 bins per lane, suffix sums by shuffles).  Then one ordered pass
-// over the pools writes the list: block-wide exclusive counts of "greater" and "equal" flags give every taken pool
-// its slot, so the pools appear in ascending index and ties go to the lowest indices.
+// One block per query.  Selection on the order-preserving integer image: a histogram of the top 12 bits gives the bin the
+// k-th largest value lies in; the values of that bin (about 2 % of them) go to a list, from which further digits of 10 bits
+// are taken (from all values when it does not fit) until it is short enough for every value in it to count the larger and
+// the equal ones.  Then one ordered pass writes the list of positions: ballots of "greater" and "equal" flags of 32
+// consecutive pools each, one scan over the counts, and a thread per ballot writes the pools it holds - the pools appear in
+// ascending index and ties go to the lowest indices.
+// Latency-bound (32 KB of scores at 32K positions): what counts is the number of passes and barriers and the chains within
+// them.  The image is kept in shared memory when it fits, so memory is read once, eight loads in flight per thread; the
+// first digit is wide because eight bits of a float are little more than its sign and exponent - nearly all values then
+// share a few bins and the shared-memory atomics serialise, here a warp's values spread over 50 bins and more.
+// (8192 pools, one query / 256 queries: 6.6 / 13.6 us; 17 / 36 us with four 8-bit passes over global memory and an ordered pass
+// with three barriers per 1024 pools.)
+constexpr int SEL_NT = 512, SEL_NW = SEL_NT / 32, SEL_BINS = 4096;
+constexpr int SEL_CACHE = 36864;          // scores of a query kept in shared memory (144 KB)
+constexpr int SEL_LIST = 2048;            // values of the k-th largest value's bin kept in a list
+constexpr int SEL_RANK = 128;             // a list up to this long is ranked value by value (all against all), longer ones take a digit first
+constexpr int SEL_SLAB = 4 * SEL_NT;      // groups of 32 pools the ordered pass takes at once
+struct SelSmem {
+    union {
+        alignas(16) uint32_t hist[SEL_BINS];
+        uint2 flags[SEL_SLAB];            // ordered pass: ballots of "greater" and "equal"
+    };
+    alignas(16) uint32_t list[SEL_LIST];
+    uint32_t wsum[2][32];
+    uint32_t digit, need, n_list;
+};
+static_assert(SEL_SLAB * 8 <= SEL_BINS * 4, "the ballots lie over the bins");
+
+// Inclusive sum over the lanes of a warp.
+__device__ __forceinline__ uint32_t warp_scan(uint32_t v, int lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+    }
+    return v;
+}
+
+// One digit: counts of the bins from the top, PER bins per thread; exactly one thread owns the bin in which the running
+// count reaches `need` (need >= 1) and leaves the digit and what is still needed in S.
+template <int PER>
+__device__ __forceinline__ void select_digit(SelSmem &S, uint32_t need) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int BINS = PER * SEL_NT;
+    uint32_t mine[PER], tot = 0;
+    // thread i owns bins [BINS - PER (i + 1), BINS - PER i), taken from the top
+#pragma unroll
+    for (int i = 0; i < PER; i += 2) {
+        const uint2 v = *reinterpret_cast<const uint2 *>(&S.hist[BINS - PER * (tid + 1) + PER - 2 - i]);
+        mine[i] = v.y;
+        mine[i + 1] = v.x;
+        tot += v.x + v.y;
+    }
+    const uint32_t incl = warp_scan(tot, lane);
+    if (lane == 31) S.wsum[0][warp] = incl;
+    __syncthreads();
+    const uint32_t ws = warp_scan(lane < SEL_NW ? S.wsum[0][lane] : 0u, lane);
+    const uint32_t prev = __shfl_sync(0xffffffffu, ws, warp > 0 ? warp - 1 : 0);
+    uint32_t above = incl - tot + (warp > 0 ? prev : 0u);  // values in higher bins
+    if (above < need && above + tot >= need) {
+#pragma unroll
+        for (int i = 0; i < PER; i++) {
+            if (above < need && above + mine[i] >= need) {
+                S.digit = (uint32_t) (BINS - PER * tid - 1 - i);
+                S.need = need - above;
+            }
+            above += mine[i];
+        }
+    }
+    __syncthreads();
+}
+
+template <bool CACHED>
 __global__ void __launch_bounds__(SEL_NT) k_idx_select(const float *__restrict__ score, int64_t score_stride, int pos0, int kpool,
                                                        int top_k, int *__restrict__ sel, int sel_stride, int *__restrict__ cnt) {
+    __shared__ SelSmem S;
+    extern __shared__ uint32_t sel_img[];
     const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int pos = pos0 + t;
     const int n_pool = (pos + 1) / kpool;
     int *out = sel + (int64_t) t * sel_stride;
+    for (int i = tid; i < SEL_BINS / 4; i += SEL_NT) reinterpret_cast<uint4 *>(S.hist)[i] = make_uint4(0, 0, 0, 0);
+    if (tid == 0) S.n_list = 0;
+    __syncthreads();
+    sm100::griddep_launch_dependents();
+    sm100::griddep_wait();
     if (n_pool <= top_k) {  // everything is attended (ops.cu:728-731)
         for (int i = tid; i <= pos; i += SEL_NT) out[i] = i;
         if (tid == 0) cnt[t] = pos + 1;
         return;
     }
     const float *sc = score + (int64_t) t * score_stride;
-    __shared__ uint32_t hist[256];
-    __shared__ uint32_t s_prefix, s_need;
-    __shared__ uint32_t w_gt[SEL_NT / 32], w_eq[SEL_NT / 32];
-    __shared__ uint32_t run_gt, run_eq;
-    uint32_t prefix = 0, mask = 0, need = (uint32_t) top_k;
-    for (int shift = 24; shift >= 0; shift -= 8) {
-        if (tid < 256) hist[tid] = 0;
-        __syncthreads();
-        for (int p = tid; p < n_pool; p += SEL_NT) {
-            const uint32_t u = f2ord(sc[p]);
-            if ((u & mask) == prefix) atomicAdd(&hist[(u >> shift) & 255], 1u);
+    // f(value image, valid) for every pool of this thread, eight at a time
+    auto for_all = [&](auto f) {
+        for (int p0 = tid; p0 < n_pool; p0 += 8 * SEL_NT) {
+            uint32_t u[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const int p = min(p0 + k * SEL_NT, n_pool - 1);
+                u[k] = CACHED ? sel_img[p] : f2ord(__ldcg(sc + p));
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++) f(u[k], p0 + k * SEL_NT < n_pool);
         }
-        __syncthreads();
-        if (warp == 0) {
-            // lane L owns bins 255 - 8L .. 248 - 8L (descending); above[L] = count in all bins above lane L's
-            uint32_t mine[8], tot = 0;
+    };
+    uint32_t U = 0xffffffffu, need = 0;  // top_k = 0: nothing exceeds the threshold, nothing equal to it is taken
+    if (top_k > 0) {
+        for (int p0 = tid; p0 < n_pool; p0 += 8 * SEL_NT) {
+            float v[8];
 #pragma unroll
-            for (int i = 0; i < 8; i++) {
-                mine[i] = hist[255 - (lane * 8 + i)];
-                tot += mine[i];
-            }
-            uint32_t incl = tot;
+            for (int k = 0; k < 8; k++) v[k] = __ldcg(sc + min(p0 + k * SEL_NT, n_pool - 1));
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += v;
-            }
-            uint32_t acc = incl - tot;  // values in bins above this lane's
-            // the digit: the highest bin at which the running count reaches `need`
-            int found = -1;
-            uint32_t acc_at = 0;
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                if (found < 0 && acc + mine[i] >= need) {
-                    found = 255 - (lane * 8 + i);
-                    acc_at = acc;
+            for (int k = 0; k < 8; k++) {
+                const int p = p0 + k * SEL_NT;
+                const uint32_t u = f2ord(v[k]);
+                if (p < n_pool) {
+                    if (CACHED) sel_img[p] = u;
+                    atomicAdd(&S.hist[u >> 20], 1u);
                 }
-                acc += mine[i];
-            }
-            const uint32_t has = __ballot_sync(0xffffffffu, found >= 0);
-            const int src = __ffs(has) - 1;  // the first lane (highest bins) that reached it; always exists: need <= count
-            const int d = __shfl_sync(0xffffffffu, found, src < 0 ? 0 : src);
-            const uint32_t a = __shfl_sync(0xffffffffu, acc_at, src < 0 ? 0 : src);
-            if (lane == 0) {
-                s_prefix = prefix | ((uint32_t) (d < 0 ? 0 : d) << shift);
-                s_need = need - a;
             }
         }
         __syncthreads();
-        prefix = s_prefix;
-        need = s_need;
-        mask |= 255u << shift;
+        select_digit<SEL_BINS / SEL_NT>(S, (uint32_t) top_k);
+        const uint32_t top = S.digit;
+        U = top << 20;
+        need = S.need;
+        auto push = [&](uint32_t u) {
+            const uint32_t i = atomicAdd(&S.n_list, 1u);
+            if (i < SEL_LIST) S.list[i] = u;
+        };
+        for_all([&](uint32_t u, bool valid) {
+            if (valid && u >> 20 == top) push(u);
+        });
+        __syncthreads();
+        int n = (int) S.n_list;
+        for (int shift = 20;;) {
+            if (n <= SEL_RANK) {
+                // thread i ranks value i: the k-th largest has fewer than `need` larger ones and at least `need` not smaller
+                if (tid < 8) S.list[n + tid] = 0;  // (the loop takes eight at a time: the smallest image, above nothing)
+                __syncthreads();
+                if (warp * 32 < n) {
+                    const uint32_t mine = tid < n ? S.list[tid] : 0u;
+                    uint32_t gt = 0, ge = 0;
+                    for (int j = 0; j < n; j += 8) {
+                        const uint4 a = *reinterpret_cast<const uint4 *>(&S.list[j]), b = *reinterpret_cast<const uint4 *>(&S.list[j + 4]);
+                        const uint32_t v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+                        for (int i = 0; i < 8; i++) {
+                            gt += v[i] > mine;
+                            ge += v[i] >= mine;
+                        }
+                    }
+                    if (tid < n && gt < need && ge >= need) {  // (every thread that holds this value stores the same)
+                        S.digit = mine;
+                        S.need = need - gt;
+                    }
+                }
+                __syncthreads();
+                U = S.digit;
+                need = S.need;
+                break;
+            }
+            // ten more bits of it
+            const uint32_t known = U >> shift;
+            const int sh = shift - 10;
+            *reinterpret_cast<uint2 *>(&S.hist[tid * 2]) = make_uint2(0, 0);
+            uint32_t mine[SEL_LIST / SEL_NT];
+            const bool listed = n <= SEL_LIST;
+#pragma unroll
+            for (int k = 0; k < SEL_LIST / SEL_NT; k++) mine[k] = S.list[tid + k * SEL_NT];
+            __syncthreads();
+            if (tid == 0) S.n_list = 0;
+            if (listed) {
+#pragma unroll
+                for (int k = 0; k < SEL_LIST / SEL_NT; k++)
+                    if (tid + k * SEL_NT < n) atomicAdd(&S.hist[(mine[k] >> sh) & 1023], 1u);
+            } else {
+                for_all([&](uint32_t u, bool valid) {
+                    if (valid && u >> shift == known) atomicAdd(&S.hist[(u >> sh) & 1023], 1u);
+                });
+            }
+            __syncthreads();
+            select_digit<2>(S, need);
+            U |= S.digit << sh;
+            need = S.need;
+            shift = sh;
+            if (shift == 0) break;
+            if (listed) {
+#pragma unroll
+                for (int k = 0; k < SEL_LIST / SEL_NT; k++)
+                    if (tid + k * SEL_NT < n && mine[k] >> shift == U >> shift) push(mine[k]);
+            } else {
+                for_all([&](uint32_t u, bool valid) {
+                    if (valid && u >> shift == U >> shift) push(u);
+                });
+            }
+            __syncthreads();
+            n = (int) S.n_list;
+        }
     }
-    const uint32_t U = prefix, need_eq = need;  // take every value above U and the first need_eq values equal to it
-    if (tid == 0) run_gt = run_eq = 0;
-    __syncthreads();
-    for (int p0 = 0; p0 < n_pool; p0 += SEL_NT) {
-        const int p = p0 + tid;
-        const uint32_t u = p < n_pool ? f2ord(sc[p]) : 0u;
-        const bool gt = p < n_pool && u > U, eq = p < n_pool && u == U;
-        const uint32_t b_gt = __ballot_sync(0xffffffffu, gt), b_eq = __ballot_sync(0xffffffffu, eq);
-        if (lane == 0) {
-            w_gt[warp] = __popc(b_gt);
-            w_eq[warp] = __popc(b_eq);
-        }
+    const uint32_t need_eq = need;  // take every value above U and the first need_eq values equal to it
+    const bool vec4 = kpool == 4 && !(reinterpret_cast<uintptr_t>(out) & 15);
+    uint32_t run_gt = 0, run_eq = 0;            // greater and equal values in front of the groups at hand
+    for (int slab = 0; slab < n_pool; slab += SEL_SLAB * 32) {
+        const int n = min(n_pool - slab, SEL_SLAB * 32), groups = (n + 31) >> 5;
         __syncthreads();
-        uint32_t before_gt = run_gt, before_eq = run_eq;
-        for (int w = 0; w < warp; w++) {
-            before_gt += w_gt[w];
-            before_eq += w_eq[w];
-        }
-        const uint32_t lt_mask = (1u << lane) - 1u;
-        const uint32_t my_eq = before_eq + __popc(b_eq & lt_mask);  // equal values in front of this one
-        const uint32_t my_gt = before_gt + __popc(b_gt & lt_mask);
-        const bool take = gt || (eq && my_eq < need_eq);
-        if (take) {
-            const uint32_t slot = my_gt + min(my_eq, need_eq);  // taken pools in front of this one
-            for (int m = 0; m < kpool; m++) out[(int64_t) slot * kpool + m] = p * kpool + m;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            uint32_t g = 0, e = 0;
-            for (int w = 0; w < SEL_NT / 32; w++) {
-                g += w_gt[w];
-                e += w_eq[w];
+        for (int g0 = warp; g0 < groups; g0 += 8 * SEL_NW) {
+            uint32_t u[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const int p = slab + min((g0 + k * SEL_NW) * 32 + lane, n - 1);
+                u[k] = CACHED ? sel_img[p] : f2ord(__ldcg(sc + p));
             }
-            run_gt += g;
-            run_eq += e;
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const int g = g0 + k * SEL_NW;
+                const bool valid = g * 32 + lane < n;
+                const uint32_t b_gt = __ballot_sync(0xffffffffu, valid && u[k] > U), b_eq = __ballot_sync(0xffffffffu, valid && u[k] == U);
+                if (lane == 0 && g < groups) S.flags[g] = make_uint2(b_gt, b_eq);
+            }
         }
         __syncthreads();
+        for (int gb = 0; gb < groups; gb += SEL_NT) {  // a thread per group
+            uint2 f = gb + tid < groups ? S.flags[gb + tid] : make_uint2(0u, 0u);
+            const uint32_t ig = warp_scan(__popc(f.x), lane), ie = warp_scan(__popc(f.y), lane);
+            if (lane == 31) {
+                S.wsum[0][warp] = ig;
+                S.wsum[1][warp] = ie;
+            }
+            __syncthreads();
+            const uint32_t wg = warp_scan(lane < SEL_NW ? S.wsum[0][lane] : 0u, lane), we = warp_scan(lane < SEL_NW ? S.wsum[1][lane] : 0u, lane);
+            const uint32_t pg = __shfl_sync(0xffffffffu, wg, warp > 0 ? warp - 1 : 0), pe = __shfl_sync(0xffffffffu, we, warp > 0 ? warp - 1 : 0);
+            uint32_t gt = run_gt + (warp > 0 ? pg : 0u) + ig - __popc(f.x), eq = run_eq + (warp > 0 ? pe : 0u) + ie - __popc(f.y);
+            for (uint32_t m = f.x | f.y; m; m &= m - 1) {
+                const int b = __ffs(m) - 1;
+                const bool is_gt = (f.x >> b) & 1;
+                if (is_gt || eq < need_eq) {
+                    const int64_t slot = (int64_t) (gt + min(eq, need_eq)) * kpool;  // taken pools in front of this one
+                    const int first = (slab + (gb + tid) * 32 + b) * kpool;
+                    if (vec4) *reinterpret_cast<int4 *>(out + slot) = make_int4(first, first + 1, first + 2, first + 3);
+                    else for (int i = 0; i < kpool; i++) out[slot + i] = first + i;
+                }
+                gt += is_gt;
+                eq += !is_gt;
+            }
+            run_gt += __shfl_sync(0xffffffffu, wg, 31);
+            run_eq += __shfl_sync(0xffffffffu, we, 31);
+            __syncthreads();  // wsum is written again
+        }
     }
     const int base = top_k * kpool, tail0 = n_pool * kpool;
     for (int i = tid; tail0 + i <= pos; i += SEL_NT) out[base + i] = tail0 + i;
     if (tid == 0) cnt[t] = base + (pos + 1 - tail0);
 }
 
+// The kernels of the indexer follow one another in a stream (pool, score, select, then the attention): each may be
+// scheduled while the one in front still runs and waits for its results inside.
+template <typename... KArgs, typename... Args>
+int launch_pdl(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    GS_TRY(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
+    return 0;
+}
+
 }  // namespace
+
 }  // namespace gs
 
 using namespace gs;
@@ -229,9 +413,8 @@ GS_EXPORT int gs_idx_pool(const float *kc, const float *gc, float *rk, float *rg
     const int n_pools = jl - jf;
     if (n_pools > 65535) return fail_invalid("gs_idx_pool: more than 65535 pools complete in one call");
     dim3 grid((Dk + 127) / 128, n_pools > 0 ? n_pools : 1);
-    k_idx_pool<<<grid, 128, 0, (cudaStream_t) stream>>>(kc, gc, rk, rg, ape, P, p0, T, Dk, kpool);
-    GS_TRY(cudaGetLastError());
-    return 0;
+    auto kernel = kpool == 4 ? k_idx_pool<4> : k_idx_pool<0>;
+    return launch_pdl(kernel, grid, 128, 0, (cudaStream_t) stream, kc, gc, rk, rg, ape, P, p0, T, Dk, kpool);
 }
 
 GS_EXPORT int gs_idx_score(const float *q, const float *w, const float *P, float *score, int64_t score_stride, int pos0, int T,
@@ -255,7 +438,12 @@ GS_EXPORT int gs_idx_select(const float *score, int64_t score_stride, int pos0, 
     if (T <= 0) return 0;  // ops.cu:788
     if (kpool <= 0 || top_k < 0 || pos0 < 0) return fail_invalid("gs_idx_select: need kpool > 0, top_k >= 0, pos0 >= 0");
     if (!sel || !cnt) return fail_invalid("gs_idx_select: null pointer");
-    k_idx_select<<<T, SEL_NT, 0, (cudaStream_t) stream>>>(score, score_stride, pos0, kpool, top_k, sel, sel_stride, cnt);
-    GS_TRY(cudaGetLastError());
-    return 0;
+    const int most = (pos0 + T) / kpool;  // scores of the last query
+    const bool cached = most > top_k && most <= SEL_CACHE;
+    if (!cached)
+        return launch_pdl(k_idx_select<false>, dim3(T), SEL_NT, 0, (cudaStream_t) stream, score, score_stride, pos0, kpool, top_k, sel, sel_stride, cnt);
+    GS_TRY(cudaFuncSetAttribute(k_idx_select<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SEL_CACHE * 4));
+    GS_TRY(cudaFuncSetAttribute(k_idx_select<true>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    return launch_pdl(k_idx_select<true>, dim3(T), SEL_NT, (size_t) most * 4, (cudaStream_t) stream, score, score_stride, pos0, kpool, top_k,
+                      sel, sel_stride, cnt);
 }
