@@ -135,8 +135,10 @@ GS_EXPORT int gs_mla_attn_set_impl(int impl) {
 
 GS_EXPORT int gs_mla_attn_status(int32_t *status_out, void *stream) {
     GS_TRY(cudaStreamSynchronize((cudaStream_t) stream));
-    int32_t st = 0;
+    int32_t st = 0, st_idx = 0;
     if (int e = read_list_status(&st)) return e;
+    if (int e = read_idx_status(&st_idx)) return e;
+    st |= st_idx << 8;
     if (status_out) *status_out = st;
     if (st != 0) {
         set_error("gs_mla_attn: a bounded wait inside the tcgen05 kernel gave up (status 0x%x)", st);

@@ -252,22 +252,6 @@ __device__ __forceinline__ bool next_segment(int &pos, int &b, int end, const in
     return true;
 }
 
-// barrier among the softmax group that also ORs a predicate over its threads
-__device__ __forceinline__ bool group_any(int id, int n_threads, bool pred) {
-    uint32_t out;
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p, r;\n\t"
-        "setp.ne.u32 p, %1, 0;\n\t"
-        "bar.red.or.pred r, %2, %3, p;\n\t"
-        "selp.u32 %0, 1, 0, r;\n\t"
-        "}\n"
-        : "=r"(out)
-        : "r"((uint32_t) pred), "r"(id), "r"(n_threads)
-        : "memory");
-    return out != 0;
-}
-
 // P.V for the O^T tiles [MT_LO, MT_HI): nk 16-row k-steps, fully unrolled
 template <int NQ, int MT_LO, int MT_HI, int O_SLOT0>
 __device__ __forceinline__ void issue_pv(uint32_t tmem, uint64_t d_vt, uint64_t d_pt, uint32_t kv_lo, uint32_t p_lo,

@@ -16,6 +16,8 @@
 // which of them are taken - changes from run to run there.  Here the list is deterministic: pools in ascending
 // index, ties to the lowest indices.  The set of selected pools is the reference's whenever the k-th largest
 // score is unique; `cnt` is always the same.
+#include <cuda_bf16.h>
+
 #include "internal.cuh"
 #include "sm100_prims.cuh"
 
@@ -80,43 +82,434 @@ __global__ void __launch_bounds__(128) k_idx_pool(const float *__restrict__ kc, 
     }
 }
 
-// ---- scores -------------------------------------------------------------------------------------------------
-// Block = 64 pools x 4 column parts (thread (pool, part) owns columns part, part + 4, part + 8, ... of its pool's key
-// in registers); the query's heads sit in shared memory and are read as broadcasts.  Per (pool, head): 32 FMAs per
-// thread and two shuffles to join the four parts.
-constexpr int SC_POOLS = 64, SC_PARTS = 4, SC_MAXI = 32;  // Dk <= SC_PARTS * SC_MAXI = 128
-__global__ void __launch_bounds__(SC_POOLS *SC_PARTS) k_idx_score(const float *__restrict__ q, const float *__restrict__ w,
-                                                                  const float *__restrict__ P, float *__restrict__ score,
-                                                                  int64_t score_stride, int pos0, int kpool, int Hq, int Dk, float scale) {
-    const int t = blockIdx.y;
-    const int n_pool = (pos0 + t + 1) / kpool;
-    const int p_base = blockIdx.x * SC_POOLS;
-    if (p_base >= n_pool) return;
-    extern __shared__ float sq[];  // [Hq][Dk] then w [Hq]
-    float *sw = sq + Hq * Dk;
-    const float *qt = q + (int64_t) t * Hq * Dk;
-    for (int i = threadIdx.x; i < Hq * Dk; i += blockDim.x) sq[i] = qt[i];
-    for (int i = threadIdx.x; i < Hq; i += blockDim.x) sw[i] = w[(int64_t) t * Hq + i];
+// ---- scores on the CUDA cores -------------------------------------------------------------------------------
+// Decode and MTP-verify steps (a few queries), and the shapes the tensor form below does not take.  A warp works on 32
+// pools x 32 heads at a time, a lane on 4 pools x 8 heads with four running sums each (the columns modulo 4, as two packed
+// f32 pairs): per four columns 12 16-byte reads from shared memory feed 64 packed FMAs.  What bounds it is the 128 bytes a
+// cycle that shared memory returns to the registers - a 16-byte read costs four cycles even when all lanes read the same
+// word - so the register tile decides: 1536 cycles of reads for 32 pools x 32 heads x 128 columns.  The head terms of a pool
+// then meet in shared memory and are added in ascending head order.  A block keeps its query and each of its warps walks
+// tiles, the next tile's keys in flight while it works on one.
+// (32 heads x 128 columns; 8192 pools, one query / 16384 pools, two queries: 7.5 / 13.4 us.  40 / 79 us with one 4-byte read per
+// FMA, 8.2 / 22.7 us with a pool's key in a lane's registers and the query row read as broadcast 16-byte words.)
+constexpr int SC_POOLS = 32, SC_HEADS = 32, SC_WARPS = 2, SC_C4 = 32;  // Dk <= 4 * SC_C4 = 128
+constexpr int SC_ROW = SC_C4 * 4 + 4;                   // rows padded by 16 bytes: eight consecutive rows cover all banks
+constexpr int score_smem(int Hq) {
+    return (SC_WARPS * (2 * SC_POOLS * SC_ROW + SC_HEADS * SC_POOLS) + Hq * (SC_ROW + 1)) * (int) sizeof(float);
+}
+__device__ __forceinline__ void fma_f32x2(uint64_t &d, uint64_t a, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
+__global__ void __launch_bounds__(SC_WARPS * 32) k_idx_score(const float *__restrict__ q, const float *__restrict__ w,
+                                                             const float *__restrict__ P, float *__restrict__ score,
+                                                             int64_t score_stride, int pos0, int kpool, int Hq, int Dk, float scale) {
+    extern __shared__ __align__(16) float sc_smem[];
+    const int t = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float *sq = sc_smem;                                                             // [Hq][SC_ROW]
+    float *sk = sq + Hq * SC_ROW + warp * (2 * SC_POOLS * SC_ROW + SC_HEADS * SC_POOLS);  // this warp's [2][32][SC_ROW]
+    float *sr = sk + 2 * SC_POOLS * SC_ROW;                                          // its relu terms [32 heads][32 pools]
+    float *sw = sc_smem + Hq * SC_ROW + SC_WARPS * (2 * SC_POOLS * SC_ROW + SC_HEADS * SC_POOLS);  // [Hq]
+    const int n_pool = (pos0 + t + 1) / kpool, n_tiles = (n_pool + SC_POOLS - 1) / SC_POOLS;
+    const bool vec = (Dk & 3) == 0 && !((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(P)) & 15);
+    const int n4 = (Dk + 3) >> 2;                  // columns up to a multiple of four: zeros
+    sm100::griddep_launch_dependents();
+    sm100::griddep_wait();
+    auto load_rows = [&](float *dst, const float *src, int rows, int last, int i0, int n_thr) {  // rows past `last` repeat it
+        if (vec) {
+            for (int i = i0; i < rows * n4; i += n_thr) {
+                const int r = i / n4, c = i - r * n4;
+                sm100::cp_async16(dst + r * SC_ROW + c * 4, src + (int64_t) min(r, last) * Dk + c * 4);
+            }
+        } else {
+            for (int i = i0; i < rows * n4 * 4; i += n_thr) {
+                const int r = i / (n4 * 4), c = i - r * (n4 * 4);
+                dst[r * SC_ROW + c] = c < Dk ? __ldcg(src + (int64_t) min(r, last) * Dk + c) : 0.f;
+            }
+        }
+        sm100::cp_async_commit();
+    };
+    auto load_tile = [&](int tile, int buf) {      // pools past the end work on a valid row and drop the result
+        load_rows(sk + buf * SC_POOLS * SC_ROW, P + (int64_t) tile * SC_POOLS * Dk, SC_POOLS, n_pool - 1 - tile * SC_POOLS, lane, 32);
+    };
+    const int step = gridDim.x * SC_WARPS;
+    int tile = blockIdx.x * SC_WARPS + warp;
+    load_rows(sq, q + (int64_t) t * Hq * Dk, Hq, Hq - 1, tid, SC_WARPS * 32);
+    if (tile < n_tiles) load_tile(tile, 0);
+    for (int i = tid; i < Hq; i += SC_WARPS * 32) sw[i] = w[(int64_t) t * Hq + i];
+    sm100::cp_async_wait_all();
     __syncthreads();
-    const int part = threadIdx.x & (SC_PARTS - 1);
-    const int p = p_base + (threadIdx.x >> 2);
-    const int pc = min(p, n_pool - 1);  // lanes past the end work on a valid row and drop the result
-    float kreg[SC_MAXI];
-    const float *pk = P + (int64_t) pc * Dk;
+    const int pg = lane >> 2, hg = lane & 3;       // pools pg + 8 j, heads hg + 4 i of a pass
+    for (int buf = 0; tile < n_tiles; tile += step, buf ^= 1) {
+        sm100::cp_async_wait_all();
+        __syncwarp();
+        if (tile + step < n_tiles) load_tile(tile + step, buf ^ 1);
+        const float *kt = sk + buf * SC_POOLS * SC_ROW + pg * SC_ROW;
+        float total = 0.f;
+        for (int h0 = 0; h0 < Hq; h0 += SC_HEADS) {
+            const int nh = min(SC_HEADS, Hq - h0);
+            uint64_t acc[4][8][2];
 #pragma unroll
-    for (int i = 0; i < SC_MAXI; i++) kreg[i] = (i * SC_PARTS + part) < Dk ? pk[i * SC_PARTS + part] : 0.f;
-    float total = 0.f;
-    for (int h = 0; h < Hq; h++) {
-        const float *qh = sq + h * Dk;
-        float d = 0.f;
+            for (int j = 0; j < 4; j++)
 #pragma unroll
-        for (int i = 0; i < SC_MAXI; i++)
-            if (i * SC_PARTS < Dk) d = fmaf((i * SC_PARTS + part) < Dk ? qh[i * SC_PARTS + part] : 0.f, kreg[i], d);
-        d += __shfl_xor_sync(0xffffffffu, d, 1);
-        d += __shfl_xor_sync(0xffffffffu, d, 2);
-        total = fmaf(sw[h], fmaxf(d * scale, 0.f), total);
+                for (int i = 0; i < 8; i++) acc[j][i][0] = acc[j][i][1] = 0;
+            const float *qh[8];  // heads past the last repeat it
+#pragma unroll
+            for (int i = 0; i < 8; i++) qh[i] = sq + (h0 + min(hg + 4 * i, nh - 1)) * SC_ROW;
+#pragma unroll 2
+            for (int c = 0; c < n4; c++) {
+                ulonglong2 k[4];
+#pragma unroll
+                for (int j = 0; j < 4; j++) k[j] = *reinterpret_cast<const ulonglong2 *>(kt + j * 8 * SC_ROW + c * 4);
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(qh[i] + c * 4);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        fma_f32x2(acc[j][i][0], v.x, k[j].x);
+                        fma_f32x2(acc[j][i][1], v.y, k[j].y);
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const float2 a = *reinterpret_cast<const float2 *>(&acc[j][i][0]), b = *reinterpret_cast<const float2 *>(&acc[j][i][1]);
+                    sr[(hg + 4 * i) * SC_POOLS + pg + 8 * j] = fmaxf(((a.x + a.y) + (b.x + b.y)) * scale, 0.f);
+                }
+            __syncwarp();
+#pragma unroll 8
+            for (int h = 0; h < nh; h++) total = fmaf(sw[h0 + h], sr[h * SC_POOLS + lane], total);
+            __syncwarp();
+        }
+        const int p = tile * SC_POOLS + lane;
+        if (p < n_pool) score[(int64_t) t * score_stride + p] = total;
     }
-    if (part == 0 && p < n_pool) score[(int64_t) t * score_stride + p] = total;
+}
+
+// ---- scores of a prefill block on the tensor cores ----------------------------------------------------------
+// 2 T pools Hq Dk operations: 17 GFLOP for 256 queries x 8192 pools x 32 heads x 128 columns, 0.23 ms at the f32 peak of
+// the CUDA cores.  The scores decide an exact top-k, so f32 precision has to stay: every f32 value is the sum of three
+// bf16 values (8 significand bits each, x = x1 + x2 + x3 exactly), and of the nine products of two such sums the six
+// with a weight above 2^-24 are formed on tcgen05: x1 y3, x3 y1, x2 y2, x1 y2, x2 y1, x1 y1.  The tensor core truncates at
+// every accumulation, so the large products come last, and every block of 64 columns has an f32 accumulator of its own:
+// four steps on a large sum instead of 48 (rms error against float64 of 256 x 8192 scores of rms 2.3: 3.2e-7 on the CUDA
+// cores, 1.4e-6 with one accumulator, 2.7e-7 this way).
+//   D[128 pools x 64] = P_tile[128 x Dk] . Q_unit[64 x Dk]^T   per unit; columns = the heads of 64 / Hq queries.
+// Pools fill the 128 lanes, so that the sum over a query's heads runs inside one thread and the scores of 32 consecutive
+// pools leave in one line.  A CTA walks consecutive units (pool tile major): the three parts of its pool tile stay in
+// tensor memory (192 columns), the query rows stream through a shared-memory ring of 64-column blocks (3 x 8 KB each).
+// Eight warps read the f32 query rows (bulk copies from L2), split them and write the swizzled operand blocks; two threads issue the
+// 48 MMAs of a unit (M = 128, N = 64, K = 16, A in tensor memory: 33 cycles each); four warps load and split the pool
+// tile, and read the finished accumulators (two sets in tensor memory) for scale, relu, weight and sum.
+// Why A is in tensor memory: with both operands in shared memory (128 columns per unit, 65 cycles per MMA) the MMAs alone
+// take 126 of the 128 bytes a cycle shared memory delivers, and the splitting warps' stores come on top.
+// 256 queries x 8192 pools x 32 heads x 128 columns: 78 us (2892 on the CUDA cores before); the tensor pipe is active in two
+// thirds of the cycles, the rest is the splitting of the query rows, which every pool tile repeats, and a start of 4 us.
+constexpr int ST_M = 128, ST_N = 64;                  // pools and query-head columns of a unit
+constexpr int ST_BLK = ST_N * 128;                    // bytes of one [64 rows][64 columns] bf16 block
+constexpr int ST_PARTS = 3;
+constexpr int ST_STAGE = ST_PARTS * ST_BLK;           // one 64-column block of the query rows, three parts
+constexpr int ST_STAGES = 6;
+constexpr int ST_RAW = ST_N * 128 * 4, ST_RAWS = 2;    // the query rows of a unit as they are, f32
+// warps 0-7 pool tile and epilogue (two groups, units of even / odd number), 8-15 conversion (two groups, ring stages of
+// even / odd number), 16 copies of the query rows, then one MMA-issuing warp per column block
+constexpr int ST_CONV_WARP0 = 8, ST_LOAD_WARP = 16, ST_MMA_WARP0 = 17;
+constexpr int st_threads(int kb) { return 32 * (ST_MMA_WARP0 + kb); }
+constexpr int ST_A_COL = 4 * ST_N;                    // tensor memory: two pairs of accumulators, then the pool tile's parts
+
+__device__ int32_t g_idx_status;                      // sticky: a bounded wait of the kernel below gave up
+
+struct ScoreParams {
+    const float *q, *w, *P;
+    float *score;
+    int64_t score_stride;
+    int pos0, T, kpool, Hq, Dk;
+    float scale;
+    int n_pools;        // complete pools of the last query: rows of P that may be read
+    int tok;            // queries per unit
+    int n_tg;           // units per pool tile
+    int n_units;
+};
+
+struct ScoreMisc {
+    uint64_t raw_full[ST_RAWS], raw_empty[ST_RAWS], b_full[ST_STAGES], b_empty[ST_STAGES], d_full[2], d_empty[2], a_full;
+    uint32_t tmem_base;
+    int abort_flag;
+    alignas(16) float w[2][ST_N];
+};
+constexpr int ST_SMEM = ST_RAWS * ST_RAW + ST_STAGES * ST_STAGE + (int) sizeof(ScoreMisc) + 1024;
+
+// Two f32 values -> packed pairs of the three bf16 parts.
+__device__ __forceinline__ void split3(float x, float y, uint32_t &w1, uint32_t &w2, uint32_t &w3) {
+    const __nv_bfloat162 h1 = __floats2bfloat162_rn(x, y);
+    const float2 f1 = __bfloat1622float2(h1);
+    const float rx = x - f1.x, ry = y - f1.y;      // exact
+    const __nv_bfloat162 h2 = __floats2bfloat162_rn(rx, ry);
+    const float2 f2 = __bfloat1622float2(h2);
+    const __nv_bfloat162 h3 = __floats2bfloat162_rn(rx - f2.x, ry - f2.y);
+    w1 = *reinterpret_cast<const uint32_t *>(&h1);
+    w2 = *reinterpret_cast<const uint32_t *>(&h2);
+    w3 = *reinterpret_cast<const uint32_t *>(&h3);
+}
+
+// KB: 64-column blocks of a row (Dk <= 64 * KB)
+template <int KB>
+__global__ void __launch_bounds__(st_threads(KB), 1) k_idx_score_umma(const ScoreParams S) {
+    using namespace sm100;
+    extern __shared__ uint8_t st_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(st_raw) + 1023) & ~(uintptr_t) 1023);
+    uint8_t *raw_smem = smem + ST_STAGES * ST_STAGE;
+    ScoreMisc &M = *reinterpret_cast<ScoreMisc *>(raw_smem + ST_RAWS * ST_RAW);
+    volatile int *abort_flag = &M.abort_flag;
+    int32_t *status = &g_idx_status;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int i = 0; i < ST_STAGES; i++) {
+            mbar_init(&M.b_full[i], 4);
+            mbar_init(&M.b_empty[i], 1);
+        }
+        for (int i = 0; i < ST_RAWS; i++) {
+            mbar_init(&M.raw_full[i], 1);
+            mbar_init(&M.raw_empty[i], KB * 4);
+        }
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&M.d_full[i], KB);
+            mbar_init(&M.d_empty[i], 4);
+        }
+        mbar_init(&M.a_full, 8);
+        M.abort_flag = 0;
+        fence_barrier_init();
+    }
+    if (warp == ST_MMA_WARP0) {
+        tmem_alloc(&M.tmem_base, 512);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = M.tmem_base;
+    griddep_launch_dependents();
+    griddep_wait();
+    // consecutive units, the counts of two CTAs differ by at most one
+    const int u0 = (int) ((int64_t) S.n_units * blockIdx.x / gridDim.x), u1 = (int) ((int64_t) S.n_units * (blockIdx.x + 1) / gridDim.x);
+
+    if (warp >= ST_CONV_WARP0 && warp < ST_LOAD_WARP) {
+        // ---- conversion of the query rows: f32 -> three swizzled bf16 blocks.  Group g takes the ring stages g, g + 2, ...
+        // (two column blocks per row: always column block g).  Thread = (row mod 8, 16 bytes of f32), eight rows.
+        const int g = (warp - ST_CONV_WARP0) >> 2, ct = (tid - ST_CONV_WARP0 * 32) & 127, c4 = ct & 15, r0 = ct >> 4;
+        const uint32_t off0 = (uint32_t) (r0 * 128 + (((c4 >> 1) ^ (r0 & 7)) << 4) + (c4 & 1) * 8);  // rows 8 apart share r mod 8
+        const int u_step = KB == 2 ? 1 : 2, n_u = u1 - u0;
+        const int col = (KB == 2 ? g * 64 : 0) + c4 * 4;
+        const bool col_ok = col < S.Dk;
+        const uint32_t src0 = (uint32_t) (r0 * S.Dk + col) * 4, row_step = (uint32_t) S.Dk * 32;
+        int st = g, tg = (u0 + (KB == 2 ? 0 : g)) % S.n_tg;
+        uint32_t st_ph = 1;
+        for (int i = KB == 2 ? 0 : g; i < n_u; i += u_step) {
+            const int rb = i % ST_RAWS, n_rows = min(S.tok, S.T - tg * S.tok) * S.Hq;
+            tg += u_step;
+            while (tg >= S.n_tg) tg -= S.n_tg;
+            if (!mbar_wait(&M.raw_full[rb], (i / ST_RAWS) & 1, abort_flag, status, 1)) break;
+            const uint8_t *src = raw_smem + rb * ST_RAW + src0;
+            float4 v[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+                v[k] = col_ok && r0 + k * 8 < n_rows ? *reinterpret_cast<const float4 *>(src + k * row_step) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (!mbar_wait(&M.b_empty[st], st_ph, abort_flag, status, 1)) break;
+            uint8_t *dst = smem + st * ST_STAGE + off0;
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                uint2 p1, p2, p3;
+                split3(v[k].x, v[k].y, p1.x, p2.x, p3.x);
+                split3(v[k].z, v[k].w, p1.y, p2.y, p3.y);
+                *reinterpret_cast<uint2 *>(dst + k * 8 * 128) = p1;
+                *reinterpret_cast<uint2 *>(dst + k * 8 * 128 + ST_BLK) = p2;
+                *reinterpret_cast<uint2 *>(dst + k * 8 * 128 + 2 * ST_BLK) = p3;
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&M.b_full[st]);
+                mbar_arrive(&M.raw_empty[rb]);
+            }
+            st += 2;
+            if (st >= ST_STAGES) {
+                st -= ST_STAGES;
+                st_ph ^= 1;
+            }
+        }
+    } else if (warp == ST_LOAD_WARP) {
+        // ---- the query rows of a unit are consecutive in memory: one bulk copy (loads by the converting threads took the
+        // same time, but 64 registers more each for what has to be in flight)
+        int tg = u0 % S.n_tg;
+        for (int i = 0; i < u1 - u0; i++) {
+            const int rb = i % ST_RAWS, n_rows = min(S.tok, S.T - tg * S.tok) * S.Hq;
+            if (!mbar_wait(&M.raw_empty[rb], ((i / ST_RAWS) & 1) ^ 1, abort_flag, status, 1)) break;
+            if (elect_one()) {
+                const uint32_t bytes = (uint32_t) (n_rows * S.Dk) * 4;
+                mbar_arrive_expect_tx(&M.raw_full[rb], bytes);
+                bulk_load(raw_smem + rb * ST_RAW, S.q + (int64_t) tg * S.tok * S.Hq * S.Dk, bytes, &M.raw_full[rb]);
+            }
+            __syncwarp();
+            if (++tg == S.n_tg) tg = 0;
+        }
+    } else if (warp >= ST_MMA_WARP0) {
+        // ---- MMA issue: warp kb of these takes column block kb of every unit, with an accumulator of its own (one issuing
+        // thread gets about 65 cycles per MMA here, two keep the pipe at its own rate)
+        const int kb = warp - ST_MMA_WARP0;
+        constexpr uint32_t idesc = make_idesc_bf16(ST_M, ST_N, 0, 0);
+        const uint64_t d_kmaj = make_smem_desc(0, 16, 1024, kSwizzle128B);
+        const uint32_t b_lo = smem_u32(smem) >> 4, as = tmem + ST_A_COL + kb * 32;
+        int n_a = 0, un = 0, st = kb, left = 0, tg = u0 % S.n_tg;
+        uint32_t st_ph = 0;
+        bool ok = true;
+        for (int u = u0; ok && u < u1; u++, un++) {
+            if (left == 0) {  // a new pool tile
+                left = S.n_tg - tg;
+                tg = 0;
+                ok = mbar_wait(&M.a_full, n_a & 1, abort_flag, status, 2);
+                n_a++;
+            }
+            left--;
+            ok = ok && mbar_wait(&M.d_empty[un & 1], ((un >> 1) & 1) ^ 1, abort_flag, status, 2) &&
+                 mbar_wait(&M.b_full[st], st_ph, abort_flag, status, 2);
+            if (!ok) break;
+            const uint32_t d = tmem + (un & 1) * 2 * ST_N + kb * ST_N;
+            const uint64_t bd = d_kmaj + (b_lo + st * (ST_STAGE >> 4));
+            tc_fence_after();
+            if (elect_one()) {
+#pragma unroll
+                for (int pr = 0; pr < 6; pr++) {
+                    // the small products first: (1,3) (3,1) (2,2) (1,2) (2,1) (1,1)
+                    constexpr int pa[6] = {0, 2, 1, 0, 1, 0}, pb[6] = {2, 0, 1, 1, 0, 0};
+#pragma unroll
+                    for (int ks = 0; ks < 4; ks++)
+                        umma_ts(d, as + pa[pr] * 64 + ks * 8, bd + (pb[pr] * (ST_BLK >> 4) + ks * 2), idesc, pr > 0 || ks > 0);
+                }
+                umma_commit(&M.b_empty[st]);
+                umma_commit(&M.d_full[un & 1]);
+            }
+            __syncwarp();
+            st += KB;
+            if (st >= ST_STAGES) {
+                st -= ST_STAGES;
+                st_ph ^= 1;
+            }
+        }
+    } else {
+        // ---- pool tile and epilogue: thread = one pool.  Both groups walk all units: each loads half of every new pool
+        // tile, group g finishes the units of number g, g + 2, ...
+        const int g = warp >> 2, row = tid & 127;
+        const uint32_t lane_base = (uint32_t) ((warp & 3) * 32) << 16;
+        const int n_w = S.T * S.Hq, cpt = S.Hq >> 4;  // 16-column chunks per query
+        int un = 0, pt = u0 / S.n_tg, tg = u0 - pt * S.n_tg;
+        bool new_tile = true;
+        auto weight = [&](int t_unit) {  // thread i < 64: the weight of column i of the unit
+            const int wi = t_unit * S.tok * S.Hq + row;
+            return row < ST_N && wi < n_w ? __ldcg(S.w + wi) : 0.f;
+        };
+        float w_next = weight((u0 + g) % S.n_tg);
+        for (int u = u0; u < u1; u++, un++, tg++) {
+            if (tg == S.n_tg) {
+                tg = 0;
+                pt++;
+                new_tile = true;
+            }
+            const int p = pt * ST_M + row;
+            if (new_tile) {
+                new_tile = false;
+                // the MMAs of the old tile are over when its last unit's accumulators are complete
+                if (un > 0) (void) mbar_wait(&M.d_full[(un - 1) & 1], ((un - 1) >> 1) & 1, abort_flag, status, 4);
+                const float *src = S.P + (int64_t) p * S.Dk;
+                float4 x[KB][8];
+#pragma unroll
+                for (int i = 0; i < KB; i++)
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        const int c = (g * KB + i) * 32 + j * 4;
+                        x[i][j] = p < S.n_pools && c < S.Dk ? __ldcg(reinterpret_cast<const float4 *>(src + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+#pragma unroll
+                for (int i = 0; i < KB; i++) {
+                    uint32_t p1[16], p2[16], p3[16];
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        split3(x[i][j].x, x[i][j].y, p1[2 * j], p2[2 * j], p3[2 * j]);
+                        split3(x[i][j].z, x[i][j].w, p1[2 * j + 1], p2[2 * j + 1], p3[2 * j + 1]);
+                    }
+                    const uint32_t a = tmem + lane_base + ST_A_COL + (g * KB + i) * 16;
+                    tmem_st16(a, p1);
+                    tmem_st16(a + 64, p2);
+                    tmem_st16(a + 128, p3);
+                }
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&M.a_full);
+            }
+            if ((un & 1) != g) continue;
+            const int t0 = tg * S.tok, n_tok = min(S.tok, S.T - t0);
+            // the weights of this unit's queries (each group has a buffer of its own)
+            if (group_any(1 + g, 128, *abort_flag != 0)) break;  // (one decision for the group; the old weights are read)
+            if (row < ST_N) M.w[g][row] = w_next;
+            w_next = weight(tg + 2 < S.n_tg ? tg + 2 : (tg + 2) % S.n_tg);
+            named_bar_sync(1 + g, 128);
+            const bool ok = mbar_wait(&M.d_full[g], (un >> 1) & 1, abort_flag, status, 4);
+            tc_fence_after();
+            // 16 columns of both accumulators at a time, the next 16 in flight while these are worked on
+            const uint32_t d_addr = tmem + lane_base + g * 2 * ST_N;
+            uint32_t r[2][16], e[2][16];
+            tmem_ld16(d_addr, r[0]);
+            if (KB == 2) tmem_ld16(d_addr + ST_N, e[0]);
+            float total = 0.f;
+            int k = 0, left = cpt;
+#pragma unroll
+            for (int c = 0; c < ST_N / 16; c++) {
+                tmem_wait_ld();
+                if (c + 1 < ST_N / 16) {
+                    tmem_ld16(d_addr + (c + 1) * 16, r[(c + 1) & 1]);
+                    if (KB == 2) tmem_ld16(d_addr + ST_N + (c + 1) * 16, e[(c + 1) & 1]);
+                } else {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&M.d_empty[g]);
+                }
+                const float4 *w4 = reinterpret_cast<const float4 *>(&M.w[g][c * 16]);
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const float4 wv = w4[i];
+                    auto term = [&](int j, float wj) {
+                        float d = __uint_as_float(r[c & 1][4 * i + j]);
+                        if (KB == 2) d += __uint_as_float(e[c & 1][4 * i + j]);
+                        total = fmaf(wj, fmaxf(d * S.scale, 0.f), total);
+                    };
+                    term(0, wv.x);
+                    term(1, wv.y);
+                    term(2, wv.z);
+                    term(3, wv.w);
+                }
+                if (--left == 0) {  // the query's last chunk
+                    if (ok && k < n_tok && p < (S.pos0 + t0 + k + 1) / S.kpool) S.score[(int64_t) (t0 + k) * S.score_stride + p] = total;
+                    total = 0.f;
+                    k++;
+                    left = cpt;
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (*abort_flag && tid == 0) {  // MMAs that were issued may still be reading shared memory
+        const long long c0 = clock64();
+        while (clock64() - c0 < 2000000LL) {
+        }
+    }
+    __syncthreads();
+    if (warp == ST_MMA_WARP0) {
+        tc_fence_after();
+        tmem_dealloc(tmem, 512);
+    }
 }
 
 // ---- selection ----------------------------------------------------------------------------------------------
@@ -398,7 +791,19 @@ int launch_pdl(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cu
     return 0;
 }
 
+template <int KB>
+int launch_score_umma(const ScoreParams &S, int sm_count, cudaStream_t st) {
+    // attributes are set on every call: a cached flag would go stale across a device reset
+    GS_TRY(cudaFuncSetAttribute(k_idx_score_umma<KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, ST_SMEM));
+    return launch_pdl(k_idx_score_umma<KB>, dim3(S.n_units < sm_count ? S.n_units : sm_count), st_threads(KB), ST_SMEM, st, S);
+}
+
 }  // namespace
+
+int read_idx_status(int32_t *out) {
+    GS_TRY(cudaMemcpyFromSymbol(out, g_idx_status, sizeof(int32_t)));
+    return 0;
+}
 
 }  // namespace gs
 
@@ -426,11 +831,39 @@ GS_EXPORT int gs_idx_score(const float *q, const float *w, const float *P, float
     if (Hq <= 0 || (int64_t) Hq * (Dk + 1) * 4 > 48 * 1024) return fail_invalid("gs_idx_score: Hq * Dk beyond 12288");
     if (T > 65535) return fail_invalid("gs_idx_score: T > 65535");
     if (!q || !w || !P || !score) return fail_invalid("gs_idx_score: null pointer");
-    dim3 grid((max_pool + SC_POOLS - 1) / SC_POOLS, T);
-    k_idx_score<<<grid, SC_POOLS * SC_PARTS, (size_t) Hq * (Dk + 1) * sizeof(float), (cudaStream_t) stream>>>(
-        q, w, P, score, score_stride, pos0, kpool, Hq, Dk, scale);
-    GS_TRY(cudaGetLastError());
-    return 0;
+    int sms = 0, dev = 0;
+    GS_TRY(cudaGetDevice(&dev));
+    GS_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    // The tensor form costs about 8 us plus 0.3 us a query, the CUDA-core form about 3 us a query (8192 pools, 32 heads,
+    // 128 columns): from 5 queries on the tensor form.  It reads whole float4s and sums 16 heads at a time.
+    if (T >= 5 && Hq % 16 == 0 && Hq <= ST_N && Dk % 4 == 0 && !((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(P)) & 15)) {
+        ScoreParams S{};
+        S.q = q;
+        S.w = w;
+        S.P = P;
+        S.score = score;
+        S.score_stride = score_stride;
+        S.pos0 = pos0;
+        S.T = T;
+        S.kpool = kpool;
+        S.Hq = Hq;
+        S.Dk = Dk;
+        S.scale = scale;
+        S.n_pools = max_pool;
+        S.tok = ST_N / Hq;
+        S.n_tg = (T + S.tok - 1) / S.tok;
+        const int64_t units = (int64_t) ((max_pool + ST_M - 1) / ST_M) * S.n_tg;
+        if (units < (1ll << 31)) {
+            S.n_units = (int) units;
+            return Dk <= 64 ? launch_score_umma<1>(S, sms, (cudaStream_t) stream) : launch_score_umma<2>(S, sms, (cudaStream_t) stream);
+        }
+    }
+    const int tiles = (max_pool + SC_POOLS - 1) / SC_POOLS, blocks = (tiles + SC_WARPS - 1) / SC_WARPS, want = (2 * sms + T - 1) / T;
+    const dim3 grid(blocks < want ? blocks : want, T);
+    const int smem = score_smem(Hq);
+    GS_TRY(cudaFuncSetAttribute(k_idx_score, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    GS_TRY(cudaFuncSetAttribute(k_idx_score, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+    return launch_pdl(k_idx_score, grid, SC_WARPS * 32, smem, (cudaStream_t) stream, q, w, P, score, score_stride, pos0, kpool, Hq, Dk, scale);
 }
 
 GS_EXPORT int gs_idx_select(const float *score, int64_t score_stride, int pos0, int T, int kpool, int top_k, int *sel,

@@ -76,6 +76,7 @@ bool decode_umma_supported(const DecodeProblem &p, const char **why);
 int launch_decode_umma_list(const float *q, const void *C, const __half *C_scales, const int32_t *sel, int sel_stride, const int32_t *cnt,
                             float scale, float *o, float *part, int T, int H, int R, int splits, int sm_count, cudaStream_t st);
 int read_list_status(int32_t *out);
+int read_idx_status(int32_t *out);  // the tensor form of gs_idx_score: non-zero when a bounded wait gave up
 int launch_decode_umma(const DecodeProblem &p, cudaStream_t st);
 
 int launch_prefill_simt(const __half *q, const __half *k, const __half *v, void *o, int o_f16, int S, int H, int d,

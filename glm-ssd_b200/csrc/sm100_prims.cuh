@@ -130,6 +130,11 @@ __device__ __forceinline__ void bulk_load(void *smem_dst, const void *gsrc, uint
 __device__ __forceinline__ void cp_async16_hint(void *smem_dst, const void *gsrc, uint64_t policy) {
     asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)), "l"(gsrc), "l"(policy) : "memory");
 }
+__device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_mbar_arrive(uint64_t *bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -226,6 +231,10 @@ __host__ __device__ constexpr uint32_t make_idesc_f16(int m, int n, int a_mn, in
     return (1u << 4) /* D = f32 */ | (0u << 7) /* A = f16 */ | (0u << 10) /* B = f16 */ | ((uint32_t) a_mn << 15) |
            ((uint32_t) b_mn << 16) | ((uint32_t) (n >> 3) << 17) | ((uint32_t) (m >> 4) << 24);
 }
+// The same with bf16 operands (A and B are always of one type).
+__host__ __device__ constexpr uint32_t make_idesc_bf16(int m, int n, int a_mn, int b_mn) {
+    return make_idesc_f16(m, n, a_mn, b_mn) | (1u << 7) | (1u << 10);
+}
 // D[tmem] (+)= A[smem] * B[smem]; issued by one thread.
 __device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
     asm volatile(
@@ -267,6 +276,22 @@ __device__ __forceinline__ float ex2_approx(float x) {
 
 __device__ __forceinline__ void named_bar_sync(int id, int n_threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n_threads) : "memory");
+}
+
+// The same barrier, which also ORs a predicate over its threads.
+__device__ __forceinline__ bool group_any(int id, int n_threads, bool pred) {
+    uint32_t out;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p, r;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "bar.red.or.pred r, %2, %3, p;\n\t"
+        "selp.u32 %0, 1, 0, r;\n\t"
+        "}\n"
+        : "=r"(out)
+        : "r"((uint32_t) pred), "r"(id), "r"(n_threads)
+        : "memory");
+    return out != 0;
 }
 
 }  // namespace sm100

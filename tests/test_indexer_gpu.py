@@ -94,6 +94,33 @@ def test_idx_score_vs_oracle_and_reference(pkg, cuda, oracle, T, pos0, Hq, Dk, k
         assert np.abs(got - ref).max() <= tol
 
 
+@pytest.mark.parametrize("T,pos0,Hq,Dk,kpool", [
+    (5, 510, 32, 128, 4),      # two units of queries (4 + 1), one exact pool tile
+    (4, 515, 32, 128, 4),      # the last query count below the tensor form
+    (6, 509, 48, 128, 4),      # columns past the last whole query of a unit
+    (17, 1530, 80, 64, 4),     # one query per unit, one block of columns, three pool tiles
+    (9, 3, 16, 100, 1),        # fewer pools than a tile, columns past Dk
+    (130, 20000, 64, 128, 4),  # many units per CTA: a CTA changes its pool tile
+])
+def test_idx_score_tensor_form_keeps_f32_precision(pkg, cuda, T, pos0, Hq, Dk, kpool):
+    """The three-way bf16 split against float64: no farther off than an f32 evaluation would be."""
+    rng = np.random.default_rng(pos0 + Hq)
+    pools = (pos0 + T) // kpool
+    q = (rng.standard_normal((T, Hq, Dk)) * np.exp2(rng.integers(-6, 7, (T, Hq, 1)))).astype(np.float32)
+    w = rng.standard_normal((T, Hq), dtype=np.float32)
+    P = rng.standard_normal((pools, Dk), dtype=np.float32)
+    scale = float(1 / np.sqrt(Dk))
+    got = _scores(cuda, pkg._lib.load(), q, w, P, pos0, kpool, pools + 3, scale)
+    assert pkg.mla_attn_status() == 0
+    want, mag = np.full(got.shape, -123.0), np.ones(got.shape)
+    for t in range(T):
+        n = (pos0 + t + 1) // kpool
+        d = (q[t].astype(np.float64) @ P[:n].astype(np.float64).T) * scale
+        want[t, :n] = w[t].astype(np.float64) @ np.maximum(d, 0)
+        mag[t, :n] = np.abs(w[t].astype(np.float64)) @ (np.abs(q[t]).astype(np.float64) @ np.abs(P[:n]).astype(np.float64).T * scale)
+    assert (np.abs(got - want) / mag).max() <= 1e-6  # of the sum of magnitudes; entries past a query's pools untouched
+
+
 def _select(torch, lib, score, pos0, kpool, top_k, sel_stride):
     T, stride = score.shape
     sel = torch.full((T, sel_stride), -1, dtype=torch.int32, device="cuda")
