@@ -84,7 +84,10 @@ __device__ long long g_pf_prof[32 * 8];
 #endif
 
 struct PfBarriers {
-    uint64_t q_full, k_full[K_STAGES], k_empty[K_STAGES], v_full[V_STAGES], v_empty[V_STAGES];
+    // k_full has a barrier per (stage, issuing warp): tile j lands in stage j % 3 on barrier j % 6.  Were it one per stage, the
+    // two score warps would take turns waiting on it, and a warp a tile ahead of the other (tiles may land out of order)
+    // would test for the phase after one that has not completed - which reads as complete.
+    uint64_t q_full, k_full[2 * K_STAGES], k_empty[K_STAGES], v_full[V_STAGES], v_empty[V_STAGES];
     uint64_t s_full[S_BUFS], p_full[S_BUFS], p_free[S_BUFS];  // p_free[b]: P.V has read the probabilities in buffer b
 };
 
@@ -115,10 +118,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
         tma_prefetch_desc(&P.tm_k);
         tma_prefetch_desc(&P.tm_v);
         mbar_init(&B.q_full, 1);
-        for (int i = 0; i < K_STAGES; i++) {
-            mbar_init(&B.k_full[i], 1);
-            mbar_init(&B.k_empty[i], 1);
-        }
+        for (int i = 0; i < 2 * K_STAGES; i++) mbar_init(&B.k_full[i], 1);
+        for (int i = 0; i < K_STAGES; i++) mbar_init(&B.k_empty[i], 1);
         for (int i = 0; i < V_STAGES; i++) {
             mbar_init(&B.v_full[i], 1);
             mbar_init(&B.v_empty[i], 1);
@@ -152,10 +153,11 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
             const int st = j % K_STAGES;
             if (!mbar_wait(&B.k_empty[st], ((j / K_STAGES) & 1) ^ 1, abort_flag, P.status, 1)) break;
             if (elect_one()) {
-                mbar_arrive_expect_tx(&B.k_full[st], KV_BYTES);
+                uint64_t *const full = &B.k_full[j % (2 * K_STAGES)];
+                mbar_arrive_expect_tx(full, KV_BYTES);
 #pragma unroll
                 for (int b = 0; b < NDB; b++)
-                    tma_load_2d(k_smem + st * KV_BYTES + b * KBLK, &P.tm_k, &B.k_full[st], col0 + b * 64, j * BN);
+                    tma_load_2d(k_smem + st * KV_BYTES + b * KBLK, &P.tm_k, full, col0 + b * 64, j * BN);
             }
             __syncwarp();
         }
@@ -185,7 +187,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
         // same accumulator, so that P.V is awaited explicitly.
         for (int j = warp == 1 ? 0 : 1; ok && j < n_tiles; j += 2) {
             const int st = j % K_STAGES, sb = j & (S_BUFS - 1);
-            ok = mbar_wait(&B.k_full[st], (j / K_STAGES) & 1, abort_flag, P.status, 2) &&
+            ok = mbar_wait(&B.k_full[j % (2 * K_STAGES)], (j / (2 * K_STAGES)) & 1, abort_flag, P.status, 2) &&
                  mbar_wait(&B.p_free[sb], ((j / S_BUFS) & 1) ^ 1, abort_flag, P.status, 2);
             if (!ok) break;
             tc_fence_after();

@@ -63,6 +63,26 @@ def test_prefill_run_to_run_bit_stable(pkg, cuda):
         assert cuda.equal(first, again)
 
 
+def test_prefill_many_launches_no_wait_gives_up(pkg, cuda):
+    """Alternating inputs beyond L2, so that key tiles land out of order now and then: every launch finishes its waits."""
+    torch = cuda
+    S, H = 4096, 20
+    g = torch.Generator(device="cuda").manual_seed(3)
+    mk = lambda: torch.randn((S, H, 256), generator=g, device="cuda").half()
+    sets = [(mk(), mk(), mk(), torch.empty((S, H, 256), device="cuda")) for _ in range(3)]
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    L = pkg._lib.load()
+    want = [pkg.prefill_attn(q, k, v).clone() for q, k, v, _ in sets]
+    for i in range(150):
+        q, k, v, o = sets[i % 3]
+        assert L.gs_prefill_attn_checked(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), 0, S, H, 256, 0, 1 / 16, 0,
+                                         status.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    assert int(status) == 0
+    for (_, _, _, o), w in zip(sets, want):
+        assert torch.equal(o, w)
+
+
 def test_prefill_f16_output(pkg, cuda, oracle):
     Q, K, V = _qkv(5, 200, 4, 256)
     got = pkg.prefill_attn(to_dev(cuda, Q), to_dev(cuda, K), to_dev(cuda, V), out_f16=True)
