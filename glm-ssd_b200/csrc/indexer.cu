@@ -36,13 +36,13 @@ __device__ __forceinline__ const float *idx_row(const float *chunk, const float 
 template <int KP>
 __global__ void __launch_bounds__(128) k_idx_pool(const float *__restrict__ kc, const float *__restrict__ gc, float *rk, float *rg,
                                                   const float *__restrict__ ape, float *__restrict__ P, int p0, int T, int Dk, int kpool_arg) {
-    sm100::griddep_launch_dependents();
     const int kpool = KP > 0 ? KP : kpool_arg;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int end = p0 + T;
     const int jf = p0 / kpool, jl = end / kpool;
     const int64_t j = (int64_t) jf + blockIdx.y;
     sm100::griddep_wait();
+    sm100::griddep_launch_dependents();
     if (c >= Dk) return;
     if (j < jl) {
         float mx = -INFINITY, sum = 0.f, acc = 0.f;
@@ -113,8 +113,8 @@ __global__ void __launch_bounds__(SC_WARPS * 32) k_idx_score(const float *__rest
     const int n_pool = (pos0 + t + 1) / kpool, n_tiles = (n_pool + SC_POOLS - 1) / SC_POOLS;
     const bool vec = (Dk & 3) == 0 && !((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(P)) & 15);
     const int n4 = (Dk + 3) >> 2;                  // columns up to a multiple of four: zeros
-    sm100::griddep_launch_dependents();
     sm100::griddep_wait();
+    sm100::griddep_launch_dependents();
     auto load_rows = [&](float *dst, const float *src, int rows, int last, int i0, int n_thr) {  // rows past `last` repeat it
         if (vec) {
             for (int i = i0; i < rows * n4; i += n_thr) {
@@ -290,8 +290,8 @@ __global__ void __launch_bounds__(st_threads(KB), 1) k_idx_score_umma(const Scor
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = M.tmem_base;
-    griddep_launch_dependents();
     griddep_wait();
+    griddep_launch_dependents();
     // consecutive units, the counts of two CTAs differ by at most one
     const int u0 = (int) ((int64_t) S.n_units * blockIdx.x / gridDim.x), u1 = (int) ((int64_t) S.n_units * (blockIdx.x + 1) / gridDim.x);
 
@@ -602,8 +602,8 @@ __global__ void __launch_bounds__(SEL_NT) k_idx_select(const float *__restrict__
     for (int i = tid; i < SEL_BINS / 4; i += SEL_NT) reinterpret_cast<uint4 *>(S.hist)[i] = make_uint4(0, 0, 0, 0);
     if (tid == 0) S.n_list = 0;
     __syncthreads();
-    sm100::griddep_launch_dependents();
     sm100::griddep_wait();
+    sm100::griddep_launch_dependents();
     if (n_pool <= top_k) {  // everything is attended (ops.cu:728-731)
         for (int i = tid; i <= pos; i += SEL_NT) out[i] = i;
         if (tid == 0) cnt[t] = pos + 1;
@@ -771,24 +771,6 @@ __global__ void __launch_bounds__(SEL_NT) k_idx_select(const float *__restrict__
     const int base = top_k * kpool, tail0 = n_pool * kpool;
     for (int i = tid; tail0 + i <= pos; i += SEL_NT) out[base + i] = tail0 + i;
     if (tid == 0) cnt[t] = base + (pos + 1 - tail0);
-}
-
-// The kernels of the indexer follow one another in a stream (pool, score, select, then the attention): each may be
-// scheduled while the one in front still runs and waits for its results inside.
-template <typename... KArgs, typename... Args>
-int launch_pdl(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    GS_TRY(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
-    return 0;
 }
 
 template <int KB>

@@ -85,4 +85,25 @@ bool prefill_umma_supported(int S, int H, int d, int p0, const char **why);
 int launch_prefill_umma(const __half *q, const __half *k, const __half *v, void *o, int o_f16, int S, int H, int d,
                         int p0, float scale, int32_t *status, cudaStream_t st);
 
+// Launch as a programmatic dependent of the kernel in front in the stream: the grid may be scheduled once every block of
+// that kernel has passed its launch_dependents (or ended), and waits for its results inside (griddepcontrol.wait before
+// the first access to anything another kernel writes or still reads).  The kernels let their own dependents start only after
+// that wait: triggered at entry, whole chains of waiting grids fill the SMs ahead of the running one (the six kernels of a
+// sparse decode step: 40.3 us that way, 36.8 with one grid ahead).
+template <typename... KArgs, typename... Args>
+int launch_pdl(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    GS_TRY(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
+    return 0;
+}
+
 }  // namespace gs

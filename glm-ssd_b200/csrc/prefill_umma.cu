@@ -140,6 +140,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = M.tmem_base;
+    griddep_wait();  // q, k and v may come from the kernel in front (RoPE)
+    griddep_launch_dependents();
 
     if (warp == 0) {
         // ---- Q once, then the K tiles -------------------------------------------------------------------
@@ -398,9 +400,7 @@ int launch_prefill_umma(const __half *q, const __half *k, const __half *v, void 
     P.status = status;  // may be nullptr: a wait that gives up is then not reported
     GS_TRY(cudaFuncSetAttribute(k_prefill_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
     dim3 grid((S + BM - 1) / BM, H);
-    k_prefill_umma<<<grid, PF_THREADS, PF_SMEM, st>>>(P);
-    GS_TRY(cudaGetLastError());
-    return 0;
+    return launch_pdl(k_prefill_umma, grid, PF_THREADS, PF_SMEM, st, P);
 }
 
 }  // namespace gs

@@ -8,10 +8,12 @@
 // frequencies are computed on the host in double and rounded to f32, cos/sin are the full-range
 // f32 functions (this file must not be built with fast-math).
 #include <math.h>
+#include <string.h>
 
 #include <new>
 
 #include "internal.cuh"
+#include "sm100_prims.cuh"
 
 namespace gs {
 namespace {
@@ -21,8 +23,21 @@ struct RopeTable {
     float inv_freq[ROPE_MAX_PAIRS];
 };
 
+// The table of the last (width, base) a thread asked for is kept: 32 calls of pow are 1.5 us of host time, as much as the
+// launch they precede.
 static void fill_table(RopeTable &t, int d_rope, float base) {
-    for (int i = 0; i < d_rope / 2; i++) t.inv_freq[i] = (float) pow((double) base, -2.0 * i / (double) d_rope);
+    struct Last {
+        int d_rope = -1;
+        float base = 0.f;
+        RopeTable tab;
+    };
+    static thread_local Last last;
+    if (last.d_rope != d_rope || !(last.base == base)) {
+        for (int i = 0; i < d_rope / 2; i++) last.tab.inv_freq[i] = (float) pow((double) base, -2.0 * i / (double) d_rope);
+        last.d_rope = d_rope;
+        last.base = base;
+    }
+    memcpy(t.inv_freq, last.tab.inv_freq, sizeof(float) * (d_rope / 2));
 }
 
 // Separately rounded products (no fused multiply-add) so the result matches a plain C evaluation.
@@ -31,12 +46,16 @@ __device__ __forceinline__ float2 rotate(float2 v, float cs, float sn) {
 }
 
 __global__ void k_f32_to_f16_scalar(const float *__restrict__ x, __half *__restrict__ y, int64_t n) {
+    sm100::griddep_wait();
+    sm100::griddep_launch_dependents();
     const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) y[i] = __float2half_rn(x[i]);
 }
 
 __global__ void k_f32_to_f16_rows(const float *__restrict__ x, __half *__restrict__ y, int64_t n) {
     // two values per thread, 4-byte stores
+    sm100::griddep_wait();
+    sm100::griddep_launch_dependents();
     const int64_t i = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) * 2;
     if (i + 1 < n) {
         const float2 v = *reinterpret_cast<const float2 *>(x + i);
@@ -51,6 +70,8 @@ __global__ void k_f32_to_f16_rows(const float *__restrict__ x, __half *__restric
 __global__ void k_quant_q8(const float *__restrict__ x, int8_t *__restrict__ q, __half *__restrict__ d, int64_t n_blocks) {
     const int64_t b = (int64_t) blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     const int lane = threadIdx.x & 31;
+    sm100::griddep_wait();
+    sm100::griddep_launch_dependents();
     if (b >= n_blocks) return;
     const float v = x[b * 32 + lane];
     const float amax = warp_max(fabsf(v));
@@ -76,9 +97,21 @@ struct AppendParams {
     RopeTable tab;
 };
 
-// grid (T, n_seq); thread j handles column pair (2j, 2j+1)
-__global__ void k_rope_append(const AppendParams P) {
+// grid (T, n_seq); thread j handles column pair (2j, 2j+1).  A few KB: what counts is the chain of round trips (position,
+// page, row) and the launches in front and behind, so the rows' values are requested first, and the kernel behind - the
+// attention, which sets itself up and asks its first tiles into L2 meanwhile - may start at once.
+constexpr int APPEND_NT = 128, APPEND_PRE = 3;  // column pairs per thread requested ahead (rows of up to 768 values)
+__global__ void __launch_bounds__(APPEND_NT) k_rope_append(const AppendParams P) {
     const int t = blockIdx.x, b = blockIdx.y;
+    sm100::griddep_wait();
+    sm100::griddep_launch_dependents();
+    const float *src = P.kv + ((int64_t) b * P.T + t) * P.d_row;
+    float2 pre[APPEND_PRE];
+#pragma unroll
+    for (int k = 0; k < APPEND_PRE; k++) {
+        const int j = threadIdx.x + k * APPEND_NT;
+        pre[k] = j < P.d_row / 2 ? *reinterpret_cast<const float2 *>(src + 2 * j) : make_float2(0.f, 0.f);
+    }
     if (P.len_out && t == 0 && b == 0 && threadIdx.x == 0) *P.len_out = P.len_val;
     const int64_t pos = (P.pos0 ? (int64_t) P.pos0[b] : P.pos0_host) + t;
     int64_t row;
@@ -101,12 +134,10 @@ __global__ void k_rope_append(const AppendParams P) {
         if (threadIdx.x == 0) atomicOr(P.status, 1 << 17);
         return;
     }
-    const float *src = P.kv + ((int64_t) b * P.T + t) * P.d_row;
     __half *dst = P.cache + row * P.d_row;
     const int d0 = P.d_row - P.d_rope;
-    for (int j = threadIdx.x; j < P.d_row / 2; j += blockDim.x) {
+    auto put = [&](int j, float2 v) {
         const int c = 2 * j;
-        float2 v = *reinterpret_cast<const float2 *>(src + c);
         if (c >= d0) {
             const float ang = (float) pos * P.tab.inv_freq[(c - d0) >> 1];
             float sn, cs;
@@ -114,7 +145,11 @@ __global__ void k_rope_append(const AppendParams P) {
             v = rotate(v, cs, sn);
         }
         *reinterpret_cast<__half2 *>(dst + c) = __floats2half2_rn(v.x, v.y);
-    }
+    };
+#pragma unroll
+    for (int k = 0; k < APPEND_PRE; k++)
+        if (threadIdx.x + k * APPEND_NT < P.d_row / 2) put(threadIdx.x + k * APPEND_NT, pre[k]);
+    for (int j = threadIdx.x + APPEND_PRE * APPEND_NT; j < P.d_row / 2; j += APPEND_NT) put(j, *reinterpret_cast<const float2 *>(src + 2 * j));
 }
 
 // RMSNorm of the latent columns fused into the append: y[c] = x[c] * rsqrt(mean(x[0..d0)^2) + eps) * w[c] for the
@@ -125,6 +160,8 @@ __global__ void __launch_bounds__(128) k_norm_rope_append(const AppendParams P, 
     __shared__ float red[4];
     const int t = blockIdx.x;
     const int64_t pos = P.pos0_host + t;
+    sm100::griddep_wait();
+    sm100::griddep_launch_dependents();
     const float *src = P.kv + (int64_t) t * P.d_row;
     __half *dst = P.cache + (int64_t) t * P.d_row;
     const int d0 = P.d_row - P.d_rope;
@@ -218,21 +255,53 @@ __global__ void __launch_bounds__(128) k_stage_append(const AppendParams P, vola
     }
 }
 
-// x f16 [S][H][d]: rotate the last d_rope columns of every head in place
-__global__ void k_rope_f16(__half *x, int64_t n_pairs, int H, int d, int d_rope, int64_t pos0, const RopeTable tab) {
-    const int64_t i = (int64_t) blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_pairs) return;
-    const int ppr = d_rope / 2;
-    const int pair = (int) (i % ppr);
-    const int64_t sh = i / ppr;  // s * H + h
-    const int64_t s = sh / H;
-    __half2 *p = reinterpret_cast<__half2 *>(x + sh * d + (d - d_rope)) + pair;
-    const float2 v = __half22float2(*p);
-    const float ang = (float) (pos0 + s) * tab.inv_freq[pair];
-    float sn, cs;
-    sincosf(ang, &sn, &cs);
-    const float2 r = rotate(v, cs, sn);
-    *p = __floats2half2_rn(r.x, r.y);
+// x f16 [S][H][d]: rotate the last d_rope columns of every head in place.  The angles depend on the position alone, so a
+// block takes a few positions, forms their sines and cosines once (before it waits for the kernel in front: they depend on
+// nothing) and applies them to all heads, 16 bytes (four pairs) per access where the layout allows.  What bounds it then is
+// the rotated quarter of the rows, read and written once.  (8192 positions x 20 heads x 64 of 256 columns, 42 MB: 46 us with
+// a sincosf and a 4-byte access per pair, 9 us now.)
+constexpr int ROPE_NT = 256;
+template <typename V>  // V: one access, sizeof(V) / 4 pairs
+__global__ void __launch_bounds__(ROPE_NT) k_rope_f16(__half *x, int S, int H, int d, int d_rope, int64_t pos0, int n_pos, const RopeTable tab) {
+    extern __shared__ float2 rope_cs[];  // [n_pos][d_rope / 2] (cos, sin)
+    constexpr int PV = sizeof(V) / 4;
+    const int s0 = blockIdx.x * n_pos, ns = min(n_pos, S - s0), ppr = d_rope / 2, vpr = ppr / PV;
+    for (int i = threadIdx.x; i < ns * ppr; i += ROPE_NT) {
+        const int s = i / ppr;
+        float sn, cs;
+        sincosf((float) (pos0 + s0 + s) * tab.inv_freq[i - s * ppr], &sn, &cs);
+        rope_cs[i] = make_float2(cs, sn);
+    }
+    __syncthreads();
+    sm100::griddep_wait();
+    sm100::griddep_launch_dependents();
+    const int items = ns * H * vpr;
+    __half *const base = x + (int64_t) s0 * H * d + (d - d_rope);
+    constexpr int U = 4;  // accesses in flight per thread
+    for (int i0 = threadIdx.x; i0 < items; i0 += U * ROPE_NT) {
+        V v[U];
+        V *p[U];
+        int cs_at[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int i = min(i0 + u * ROPE_NT, items - 1);
+            const int sh = i / vpr, c = i - sh * vpr;  // sh = position * H + head
+            p[u] = reinterpret_cast<V *>(base + (int64_t) sh * d) + c;
+            cs_at[u] = sh / H * ppr + c * PV;
+            v[u] = *p[u];
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            __half2 *h = reinterpret_cast<__half2 *>(&v[u]);
+#pragma unroll
+            for (int k = 0; k < PV; k++) {
+                const float2 cs = rope_cs[cs_at[u] + k];
+                const float2 r = rotate(__half22float2(h[k]), cs.x, cs.y);
+                h[k] = __floats2half2_rn(r.x, r.y);
+            }
+            if (i0 + u * ROPE_NT < items) *p[u] = v[u];
+        }
+    }
 }
 
 int check_rope(int d_row, int d_rope) {
@@ -251,23 +320,17 @@ GS_EXPORT int gs_f32_to_f16(const float *x, void *y, int64_t n, void *stream) {
     if (n <= 0) return 0;
     if ((reinterpret_cast<uintptr_t>(x) & 7) || (reinterpret_cast<uintptr_t>(y) & 3)) {
         // odd alignment: one value per thread
-        k_f32_to_f16_scalar<<<(unsigned) ((n + 255) / 256), 256, 0, (cudaStream_t) stream>>>(x, (__half *) y, n);
-        GS_TRY(cudaGetLastError());
-        return 0;
+        return launch_pdl(k_f32_to_f16_scalar, dim3((unsigned) ((n + 255) / 256)), 256, 0, (cudaStream_t) stream, x, (__half *) y, n);
     }
     const int64_t pairs = (n + 1) / 2;
-    k_f32_to_f16_rows<<<(unsigned) ((pairs + 255) / 256), 256, 0, (cudaStream_t) stream>>>(x, (__half *) y, n);
-    GS_TRY(cudaGetLastError());
-    return 0;
+    return launch_pdl(k_f32_to_f16_rows, dim3((unsigned) ((pairs + 255) / 256)), 256, 0, (cudaStream_t) stream, x, (__half *) y, n);
 }
 
 GS_EXPORT int gs_quant_q8_rows(const float *x, void *q, void *d, int64_t n, void *stream) {
     if (n % 32 != 0) return fail_invalid("gs_quant_q8_rows: n must be a multiple of 32");  // ops.cu:612
     const int64_t nb = n / 32;
     if (nb <= 0) return 0;
-    k_quant_q8<<<(unsigned) ((nb + 7) / 8), 256, 0, (cudaStream_t) stream>>>(x, (int8_t *) q, (__half *) d, nb);
-    GS_TRY(cudaGetLastError());
-    return 0;
+    return launch_pdl(k_quant_q8, dim3((unsigned) ((nb + 7) / 8)), 256, 0, (cudaStream_t) stream, x, (int8_t *) q, (__half *) d, nb);
 }
 
 GS_EXPORT int gs_rope_kv_append_at(const float *kv, void *cache_row0, int64_t pos0, int T, int d_row, int d_rope,
@@ -285,9 +348,7 @@ GS_EXPORT int gs_rope_kv_append_at(const float *kv, void *cache_row0, int64_t po
     P.d_row = d_row;
     P.d_rope = d_rope;
     fill_table(P.tab, d_rope, rope_base);
-    k_rope_append<<<dim3(T, 1), 128, 0, (cudaStream_t) stream>>>(P);
-    GS_TRY(cudaGetLastError());
-    return 0;
+    return launch_pdl(k_rope_append, dim3(T, 1), APPEND_NT, 0, (cudaStream_t) stream, P);
 }
 
 GS_EXPORT int gs_norm_rope_kv_append_at(const float *kv, const float *w, float eps, void *cache_row0, int64_t pos0, int T,
@@ -306,9 +367,7 @@ GS_EXPORT int gs_norm_rope_kv_append_at(const float *kv, const float *w, float e
     P.d_row = d_row;
     P.d_rope = d_rope;
     fill_table(P.tab, d_rope, rope_base);
-    k_norm_rope_append<<<T, 128, 0, (cudaStream_t) stream>>>(P, w, eps);
-    GS_TRY(cudaGetLastError());
-    return 0;
+    return launch_pdl(k_norm_rope_append, dim3(T), 128, 0, (cudaStream_t) stream, P, w, eps);
 }
 
 GS_EXPORT int gs_rope_kv_append(const float *kv, void *cache, const int32_t *pos0, const int32_t *seq_base,
@@ -331,9 +390,7 @@ GS_EXPORT int gs_rope_kv_append(const float *kv, void *cache, const int32_t *pos
     P.d_row = d_row;
     P.d_rope = d_rope;
     fill_table(P.tab, d_rope, rope_base);
-    k_rope_append<<<dim3(T, n_seq), 128, 0, (cudaStream_t) stream>>>(P);
-    GS_TRY(cudaGetLastError());
-    return 0;
+    return launch_pdl(k_rope_append, dim3(T, n_seq), APPEND_NT, 0, (cudaStream_t) stream, P);
 }
 
 GS_EXPORT int gs_rope_kv_append_checked(const float *kv, void *cache, int64_t cache_rows, const int32_t *pos0,
@@ -360,9 +417,7 @@ GS_EXPORT int gs_rope_kv_append_checked(const float *kv, void *cache, int64_t ca
     P.cache_rows = cache_rows;
     P.status = status;
     fill_table(P.tab, d_rope, rope_base);
-    k_rope_append<<<dim3(T, n_seq), 128, 0, (cudaStream_t) stream>>>(P);
-    GS_TRY(cudaGetLastError());
-    return 0;
+    return launch_pdl(k_rope_append, dim3(T, n_seq), APPEND_NT, 0, (cudaStream_t) stream, P);
 }
 
 GS_EXPORT int gs_rope_f16_inplace(void *x, int S, int H, int d, int d_rope, int64_t pos0, float rope_base,
@@ -372,11 +427,14 @@ GS_EXPORT int gs_rope_f16_inplace(void *x, int S, int H, int d, int d_rope, int6
     if (S <= 0 || H <= 0 || d_rope == 0) return 0;
     RopeTable tab;
     fill_table(tab, d_rope, rope_base);
-    const int64_t n_pairs = (int64_t) S * H * (d_rope / 2);
-    k_rope_f16<<<(unsigned) ((n_pairs + 255) / 256), 256, 0, (cudaStream_t) stream>>>((__half *) x, n_pairs, H, d, d_rope,
-                                                                                     pos0, tab);
-    GS_TRY(cudaGetLastError());
-    return 0;
+    // positions per block: enough for a few accesses per thread, fewer when the blocks would not fill the GPU
+    int n_pos = 8;
+    while (n_pos > 1 && (S + n_pos - 1) / n_pos < 296) n_pos >>= 1;
+    const dim3 grid((S + n_pos - 1) / n_pos);
+    const size_t smem = (size_t) n_pos * (d_rope / 2) * sizeof(float2);
+    if (d % 8 == 0 && d_rope % 8 == 0 && !(reinterpret_cast<uintptr_t>(x) & 15))
+        return launch_pdl(k_rope_f16<uint4>, grid, ROPE_NT, smem, (cudaStream_t) stream, (__half *) x, S, H, d, d_rope, pos0, n_pos, tab);
+    return launch_pdl(k_rope_f16<uint32_t>, grid, ROPE_NT, smem, (cudaStream_t) stream, (__half *) x, S, H, d, d_rope, pos0, n_pos, tab);
 }
 
 // ---- one decode step of a layer with host buffers ---------------------------------------------------
@@ -407,8 +465,7 @@ GS_EXPORT int gs_mla_layer_step_host(const gs_mla_layer_step *s, void *stream) {
     P.len_out = s->seq_len_dev;
     P.len_val = (int32_t) (s->pos0 + s->T);
     fill_table(P.tab, s->d_rope, s->rope_base);
-    k_rope_append<<<dim3(s->T, 1), 128, 0, st>>>(P);
-    GS_TRY(cudaGetLastError());
+    if (int e = launch_pdl(k_rope_append, dim3(s->T, 1), APPEND_NT, 0, st, P)) return e;
     gs_mla_decode_args a{};
     a.q = s->q_dev;
     a.cache = s->cache;
