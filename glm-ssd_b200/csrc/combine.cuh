@@ -238,30 +238,36 @@ __device__ __forceinline__ bool combine_item_compute(const CombinePlan &C, const
 
 // The records of the tcgen05 kernel ([segment][row][d_v]) fetched by ONE tiled 3-D TMA copy: what an item (output row,
 // 128 columns) needs is one 512-byte piece per segment, a whole record apart from the next - a box
-// {128, 1, n_ctas} of the tensor {d_v, rows, segments}.  The box always spans n_ctas segments (a sequence has at most
-// one per CTA); segments past the sequence's last one belong to other sequences or lie outside the tensor (zero-filled)
-// and get weight 0.
+// {128, 1, box} of the tensor {d_v, rows, segments}.  With one sequence the box spans n_ctas segments (a sequence has at
+// most one per CTA); with several a row has about n_ctas / n_seq + 1, a number only the device knows, and as many boxes of
+// 16 as it needs are fetched.  Segments past the sequence's last one belong to other sequences or lie outside the tensor
+// (zero-filled) and get weight 0.
 constexpr int32_t ST_COMBINE = 1 << 18;  // status bit: the copy of the records did not complete in time
 struct CombineBulk {
     CUtensorMap tm;
     CombinePlan c;
+    int box;   // segments per copy
+    int cap;   // segments the shared-memory tile holds, a multiple of box; a row with more takes several rounds
 };
 
-// All CB_NT threads call this with the same arguments.  `tile` is 128-byte aligned shared memory of n_ctas x 512 bytes,
-// `bar` an initialised mbarrier (count 1) in its first phase, *abort_flag zero.  Thread 0 issues the copy; meanwhile
-// thread i fetches (m, l) of segment i and the block forms M, the weights and L; after the copy has landed 8 segment
-// lanes x 32 column quads sum from shared memory.  Returns false when the copy did not complete in time (status bit
+// All CB_NT threads call this with the same arguments.  `tile` is 128-byte aligned shared memory of cap x 512 bytes,
+// `bar` an initialised mbarrier (count 1) in its first phase, *abort_flag zero.  Thread 0 issues the copies; meanwhile
+// thread i fetches (m, l) of segment i and the block forms M, the weights and L; after the copies have landed 8 segment
+// lanes x 32 column quads sum from shared memory.  Returns false when a copy did not complete in time (status bit
 // set, nothing may be written); else the threads of warp 0 hold the four merged (unnormalised) columns col0 + 4 lane
 // in `a`, and every thread M and L.
-__device__ __forceinline__ bool combine_item_fetch_tma(const CombinePlan &C, const CUtensorMap *tm, const SegRange &R, int col0,
-                                                       float4 *tile, uint64_t *bar, int *abort_flag, CombineSmem &S, float4 &a,
-                                                       float &M, float &L) {
+__device__ __forceinline__ bool combine_item_fetch_tma(const CombinePlan &C, const CUtensorMap *tm, int box, int cap, const SegRange &R, int col0,
+                                                       float4 *tile, uint64_t *bar, int *abort_flag, CombineSmem &S, float4 &a, float &M,
+                                                       float &L) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nseg = min(R.nseg, min(C.n_ctas, CB_NT));
-    if (tid == 0 && nseg > 0) {
-        sm100::mbar_arrive_expect_tx(bar, (uint32_t) C.n_ctas * CB_COLS * 4);  // the whole box, zero-filled rows included
-        sm100::tma_load_3d(tile, tm, bar, col0, R.row_in_seg, R.first);
-    }
+    auto fetch = [&](int s0) {  // the boxes that hold segments s0 .. of this round; whole boxes count, zero-filled rows included
+        const int n_box = (min(nseg - s0, cap) + box - 1) / box;
+        sm100::mbar_arrive_expect_tx(bar, (uint32_t) (n_box * box) * CB_COLS * 4);
+        for (int k = 0; k < n_box; k++)
+            sm100::tma_load_3d(tile + k * box * (CB_COLS / 4), tm, bar, col0, R.row_in_seg, R.first + s0 + k * box);
+    };
+    if (tid == 0 && nseg > 0) fetch(0);
     float2 ml = make_float2(-INFINITY, 0.f);
     if (tid < nseg) ml = __ldcg(reinterpret_cast<const float2 *>(combine_ml_ptr(C, R.first + tid, R.row_in_seg)));
     const float mx = warp_max(ml.x);
@@ -274,23 +280,27 @@ __device__ __forceinline__ bool combine_item_fetch_tma(const CombinePlan &C, con
     S.m[tid] = wgt;
     const float ls = warp_sum(ml.y * wgt);
     if (lane == 0) S.lred[warp] = ls;
-    if (nseg > 0 && !sm100::mbar_wait(bar, 0, abort_flag, const_cast<int32_t *>(C.status), ST_COMBINE)) *abort_flag = 1;
-    __syncthreads();
-    if (*abort_flag) return false;
+    a = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s0 = 0, round = 0; round == 0 || s0 < nseg; s0 += cap, round++) {
+        if (round > 0 && tid == 0) fetch(s0);
+        if (nseg > 0 && !sm100::mbar_wait(bar, round & 1, abort_flag, const_cast<int32_t *>(C.status), ST_COMBINE)) *abort_flag = 1;
+        __syncthreads();
+        if (*abort_flag) return false;
+        for (int s = s0 + warp; s < min(nseg, s0 + cap); s += CB_LANES) {
+            const float w = S.m[s];
+            if (w != 0.f) {  // an empty segment's accumulator never enters the sum
+                const float4 u = tile[(s - s0) * (CB_COLS / 4) + lane];
+                a.x = fmaf(u.x, w, a.x);
+                a.y = fmaf(u.y, w, a.y);
+                a.z = fmaf(u.z, w, a.z);
+                a.w = fmaf(u.w, w, a.w);
+            }
+        }
+        if (s0 + cap < nseg) __syncthreads();  // the tile is filled again
+    }
     L = 0.f;
 #pragma unroll
     for (int w = 0; w < CB_NT / 32; w++) L += S.lred[w];
-    a = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = warp; s < nseg; s += CB_LANES) {
-        const float w = S.m[s];
-        if (w != 0.f) {  // an empty segment's accumulator never enters the sum
-            const float4 u = tile[s * (CB_COLS / 4) + lane];
-            a.x = fmaf(u.x, w, a.x);
-            a.y = fmaf(u.y, w, a.y);
-            a.z = fmaf(u.z, w, a.z);
-            a.w = fmaf(u.w, w, a.w);
-        }
-    }
     S.part[warp][lane] = a;
     __syncthreads();
     if (warp == 0) {

@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(CB_NT) k_exchange_combine(const __grid_constan
         const SegRange R = combine_locate(C, row, S);
         bool holds;
         if (EL.tma) {  // the item's pieces of all local segments by one tiled TMA copy
-            if (!combine_item_fetch_tma(C, &EL.tm, R, chunk * CB_COLS, tile, &bar, &s_fetch_abort, S, a, M, L)) {
+            if (!combine_item_fetch_tma(C, &EL.tm, C.n_ctas, C.n_ctas, R, chunk * CB_COLS, tile, &bar, &s_fetch_abort, S, a, M, L)) {
                 exchange_block_done(X);
                 return;  // status bit 18 says why; nothing is sent, the other ranks' waits run out
             }
