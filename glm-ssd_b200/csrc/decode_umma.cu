@@ -114,6 +114,17 @@ constexpr int NGRP = (NBLK_MAX + GRP - 1) / GRP;
 constexpr int AHEAD = 2;                 // tiles of a CTA's range asked into L2 before the inputs are final (1-3 measured: 2 best)
 constexpr int N_MMA_WARPS = 3;           // MMA warp slots (warps 1-3); a kernel form issues from the first NI of them
 constexpr int NTHREADS = 32 * (1 + N_MMA_WARPS + 4);  // warp 0 producer, warps 1-3 MMA, warps 4-7 softmax group
+// Position lists: four producer warps more (8-11; warp 0 has no part).  Registers per thread of the three warpgroups after
+// the hand-over of setmaxnreg; their sum is what the block is launched with, 3 x 168.
+constexpr int LIST_NTHREADS = NTHREADS + 128;
+struct ListRegs {
+    int mma, softmax, producer;
+};
+__host__ __device__ constexpr ListRegs list_regs(int nq, bool q8) {
+    return q8 ? (nq > 48 ? ListRegs{112, 240, 152} : ListRegs{160, 208, 136}) : (nq > 48 ? ListRegs{128, 248, 128} : ListRegs{168, 208, 128});
+}
+constexpr bool list_regs_fit(int nq, bool q8) { return list_regs(nq, q8).mma + list_regs(nq, q8).softmax + list_regs(nq, q8).producer <= 3 * 168; }
+static_assert(list_regs_fit(32, false) && list_regs_fit(64, false) && list_regs_fit(32, true) && list_regs_fit(64, true), "registers of a block of 384 threads");
 constexpr int TMEM_COLS = 512;
 // TMEM columns (slots of NQ columns): S^T partials [2 buffers][NI issuers], then the 4 O^T tiles:
 // 10 x 48 = 480 of the 512 columns for NQ = 48 with three issuers, 8 x 64 = 512 for NQ = 64 with two
@@ -151,7 +162,8 @@ struct UmmaParams {
     const int32_t *sel;
     int sel_stride;
     const float *q_f32;            // list form: f32 queries [tokens][H_full][d_qk], rounded to f16 inside the kernel
-    int whole_seq;                 // list form: every sequence is attended by one CTA, which normalises and stores o itself
+    int whole_seq;                 // list form: every sequence is attended by one CTA (or one cluster), which normalises and stores o itself
+    int cluster;                   // whole_seq: CTAs that share a sequence (a thread-block cluster when > 1; then grid = n_seq * cluster)
     float *o;                      // whole_seq: output f32 [tokens][H_out][d_v]
     int H_out;
     int seg_cap;                   // segments the record arrays hold
@@ -162,32 +174,45 @@ struct UmmaParams {
 
 struct Barriers {
     uint64_t kv_full[STAGES][NGRP], kv_empty[STAGES];
-    uint64_t kv_raw[STAGES];  // Q8 list form: the int8 rows and scales of a tile have landed (not yet widened)
     uint64_t s_full[2], s_empty[2], p_full[2], p_empty[2];
     uint64_t q_full, q_empty, o_full, o_empty;
+    uint64_t x_ready, x_data; // cluster form: every CTA's stages are free; everything the other CTAs send has arrived
 };
 
 // NQ <= 48: stages and query rows sized for the widest row (576 columns), one layout for both row widths.  NQ = 64 (only
 // built for 512-column rows): sized by the row width, or two stages, the query rows and P would not fit.
-template <int NQ, int NBLK = NBLK_MAX, bool Q8 = false>
+constexpr int MAX_CLUSTER = 16;
+template <int NQ, int NBLK = NBLK_MAX>
 struct Smem {
-    static constexpr int SBLK = (NQ > 48 || Q8) ? NBLK : NBLK_MAX;   // 64-column blocks a stage and the query rows are sized for
+    static constexpr int SBLK = NQ > 48 ? NBLK : NBLK_MAX;   // 64-column blocks a stage and the query rows are sized for
     static constexpr int STAGE = SBLK * BLK_BYTES;
     static constexpr int Q_BYTES = SBLK * NQ * 128;
     static constexpr int P_BYTES = NQ * TILE * 2;
     static constexpr int OFF_Q = STAGES * STAGE;
     static constexpr int OFF_P = OFF_Q + Q_BYTES;
-    static constexpr int QS_BYTES = Q8 ? TILE * (NBLK * 2) * 2 : 0;  // Q8: the tile's scales, NBLK * 2 halves per row
-    static constexpr int OFF_QS = OFF_P + 2 * P_BYTES;
-    static constexpr int OFF_MISC = OFF_QS + STAGES * QS_BYTES;
+    static constexpr int OFF_MISC = OFF_P + 2 * P_BYTES;
+    // cluster form, over stages and query rows: all CTAs' accumulators of this CTA's columns, [source][query row][512 / cluster]
+    // f32, and behind them this CTA's own accumulators on their way out, X_ROWS query rows at a time
+    static constexpr int OFF_XOUT = 512 * NQ * 4;
+    static constexpr int X_ROWS = NQ > 48 ? NQ / 2 : NQ;
+    static_assert(OFF_XOUT + 512 * X_ROWS * 4 <= OFF_P, "the exchanged accumulators lie over the stages and the query rows");
     struct Misc {
         Barriers bar;
         uint32_t tmem_base;
         int abort_flag;
         int flag[2];
-        int cum[MAX_SEQ + 1];
-        int len[MAX_SEQ];
-        int base[MAX_SEQ];
+        union {
+            struct {
+                int cum[MAX_SEQ + 1];
+                int len[MAX_SEQ];
+                int base[MAX_SEQ];
+            };
+            struct {                       // cluster form (which needs none of them)
+                alignas(16) float2 x_ml[MAX_CLUSTER][NQ];   // (m in log2 units, l) of every CTA
+                alignas(16) float2 x_mine[NQ];              // this CTA's, on their way out
+                float x_w[MAX_CLUSTER][NQ];                 // weight of every CTA's accumulators in the normalised sum
+            };
+        };
         float smax[4][NQ];
         float sl[4][NQ];
         float mref[NQ];
@@ -197,6 +222,26 @@ struct Smem {
     static constexpr int TOTAL = OFF_MISC + (int) sizeof(Misc) + 1024;  // + slack for the 1024-byte alignment
     static_assert(TOTAL <= 232448, "shared memory of one CTA");
 };
+
+// The bounded wait.  A kernel that hands registers over (setmaxnreg) may not call functions: its slow path is inlined.
+template <bool INLINE>
+__device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int32_t *status, int32_t code) {
+    if (!INLINE) return mbar_wait(bar, parity, abort_flag, status, code);
+    if (mbar_try_wait(bar, parity)) return true;
+    const long long t0 = clock64();
+    int spins = 0;
+    while (!mbar_try_wait(bar, parity)) {
+        if ((++spins & 63) == 0) {
+            if (*abort_flag) return false;
+            if (clock64() - t0 > kWaitLimitCycles) {
+                *abort_flag = 1;
+                if (status) atomicOr(status, code);
+                return false;
+            }
+        }
+    }
+    return true;
+}
 
 struct Segment {
     int b, r0, r1, len, n_tiles, seg_id;
@@ -208,15 +253,30 @@ struct Sched {
     int total, chunk, start, end, b0;
     int len0, base0;  // single sequence: its (capped) length and first row
     bool single;
-    bool whole;       // sequences are not cut: CTA c attends sequences c, c + grid, ... from their first row to their last
+    bool whole;       // sequences are not dealt by rows: CTA c attends sequences c, c + grid, ... from their first row to their
+                      // last, or - share > 1 - every CTA of cluster b the rank-th part of sequence b
+    int share, rank;
 };
 
 // Walks the segments of this CTA's unit range [pos, end); `b` is a cursor over sequences.
 __device__ __forceinline__ bool next_segment(int &pos, int &b, int end, const int *cum, int unit_rows,
                                              const int *seq_lens, Segment &sg, const Sched &sc) {
     if (sc.whole) {
-        // `b` walks this CTA's sequences; empty ones yield no segment (their output rows are zeroed up front)
         int len = 0;
+        if (sc.share > 1) {  // an equal share of the sequence's rows, possibly none
+            if (b >= sc.total) return false;
+            len = sc.len0;
+            const int per = (len + sc.share - 1) / sc.share;
+            sg.b = b;
+            sg.len = len;
+            sg.r0 = min(len, sc.rank * per);
+            sg.r1 = min(len, sg.r0 + per);
+            sg.n_tiles = (sg.r1 - sg.r0 + TILE - 1) / TILE;
+            sg.seg_id = 0;
+            b = sc.total;
+            return true;
+        }
+        // `b` walks this CTA's sequences; empty ones yield no segment (their output rows are zeroed up front)
         while (b < sc.total && (len = sc.single ? sc.len0 : seq_lens[b]) <= 0) b += (int) gridDim.x;
         if (b >= sc.total) return false;
         sg.b = b;
@@ -276,9 +336,10 @@ __device__ __forceinline__ void issue_pv(uint32_t tmem, uint64_t d_vt, uint64_t 
 }
 
 template <int NQ, int NBLK, bool LIST, bool Q8 = false>
-__global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_constant__ UmmaParams P) {
+__global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_umma(const __grid_constant__ UmmaParams P) {
     static_assert(!Q8 || LIST, "the Q8 cache comes with position lists only");
-    using SM = Smem<NQ, NBLK, Q8>;
+    using SM = Smem<NQ, NBLK>;
+    constexpr int NTHR = LIST ? LIST_NTHREADS : NTHREADS;
     constexpr int NI = issuers_for(NQ);   // issuing MMA warps
     constexpr int O_SLOT0 = 2 * NI;       // first O^T slot in tensor memory
     constexpr int STAGE_BYTES = SM::STAGE;
@@ -288,7 +349,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
     uint8_t *kv_smem = smem;
     uint8_t *q_smem = smem + SM::OFF_Q;
     uint8_t *p_smem = smem + SM::OFF_P;
-    uint8_t *qs_smem = smem + SM::OFF_QS;
     typename SM::Misc &M = *reinterpret_cast<typename SM::Misc *>(smem + SM::OFF_MISC);
     Barriers &B = M.bar;
     volatile int *abort_flag = &M.abort_flag;
@@ -324,9 +384,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
         tma_prefetch_desc(&P.tm_kv16);
         tma_prefetch_desc(&P.tm_q);
         for (int s = 0; s < STAGES; s++) {
-            // list form: one arrival per producer lane; Q8 list form: one per softmax warp, after the widening
-            for (int g = 0; g < NGRP; g++) mbar_init(&B.kv_full[s][g], Q8 ? 4 : LIST ? 32 : 1);
-            mbar_init(&B.kv_raw[s], 32);
+            // list form: one arrival per producer lane (it follows the lane's copies) or, Q8, per producer warp
+            for (int g = 0; g < NGRP; g++) mbar_init(&B.kv_full[s][g], !LIST ? 1 : Q8 ? 4 : 128);
             mbar_init(&B.kv_empty[s], NI);
         }
         for (int s = 0; s < 2; s++) {
@@ -339,9 +398,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
         mbar_init(&B.q_empty, NI);
         mbar_init(&B.o_full, NI);
         mbar_init(&B.o_empty, 4);
+        if (LIST && P.cluster > 1) {
+            mbar_init(&B.x_ready, P.cluster);
+            mbar_init(&B.x_data, 1);
+        }
         M.abort_flag = 0;
         M.flag[0] = M.flag[1] = 0;
-        M.cum[0] = 0;
+        if (!(LIST && P.whole_seq)) M.cum[0] = 0;
         fence_barrier_init();
     }
     if (warp == 1) {
@@ -352,6 +415,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
     Sched sc;
     sc.single = P.n_seq == 1;
     sc.whole = LIST && P.whole_seq;
+    sc.share = LIST && P.whole_seq ? P.cluster : 1;
+    sc.rank = sc.share > 1 ? (int) blockIdx.x % sc.share : 0;
     sc.total = 0;
     sc.chunk = 1;
     sc.start = sc.end = sc.b0 = 0;
@@ -369,8 +434,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
             sc.len0 = (int) min((int64_t) max(ld_global_hint(P.seq_lens, pol_keep), 0), len_cap);
             sc.base0 = P.seq_base ? ld_global_hint(P.seq_base, pol_keep) : 0;
             sc.total = (sc.len0 + unit_rows - 1) / unit_rows;
+        } else if (LIST && sc.share > 1) {  // one sequence per cluster: every thread reads its length itself
+            sc.len0 = (int) min((int64_t) max(ld_global_hint(P.seq_lens + (int) blockIdx.x / sc.share / P.seq_div, pol_keep), 0), len_cap);
+        } else if (LIST && sc.whole) {  // no units to deal, only the lengths
+            for (int b = tid; b < P.n_seq; b += NTHR)
+                M.len[b] = (int) min((int64_t) max(ld_global_hint(P.seq_lens + b / P.seq_div, pol_keep), 0), len_cap);
+            __syncthreads();
         } else {
-            for (int b = tid; b < P.n_seq; b += NTHREADS) {
+            for (int b = tid; b < P.n_seq; b += NTHR) {
                 const int len = (int) min((int64_t) max(ld_global_hint(P.seq_lens + b / P.seq_div, pol_keep), 0), len_cap);
                 M.base[b] = P.seq_base ? ld_global_hint(P.seq_base + b / P.seq_div, pol_keep) : 0;
                 M.len[b] = len;
@@ -403,7 +474,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
         sc.b0 = 0;
         if (sc.whole) {  // sequences dealt round-robin; `total` counts sequences, the cursor starts at this CTA's first
             sc.total = P.n_seq;
-            sc.b0 = (int) blockIdx.x;
+            sc.b0 = (int) blockIdx.x / sc.share;
             return;
         }
         if (!sc.single) {
@@ -445,6 +516,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (LIST && sc.share > 1) cluster_sync();  // every CTA's barriers are initialised before another CTA arrives on them
     griddep_wait();
     if (tid == 0) GS_CTA_STAMP(1);
     build_schedule();
@@ -453,7 +525,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
         if (sc.single) {
             if (tid == 0) P.ws_desc[0] = sc.total > 0 ? make_int2(0, (sc.total - 1) / sc.chunk + 1) : make_int2(0, 0);
         } else {
-            for (int b = tid; b < P.n_seq; b += NTHREADS) {
+            for (int b = tid; b < P.n_seq; b += NTHR) {
                 const int u0 = M.cum[b], u1 = M.cum[b + 1];
                 int2 d = make_int2(0, 0);
                 if (u1 > u0) {
@@ -471,7 +543,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
     uint32_t it = 0, sgc = 0;  // running tile and segment counters (identical in every role)
     Segment sg;
 
-    if (warp == 0) {
+    // (The hand-over of registers in the list form: every warpgroup executes one instruction; the softmax group takes over
+    // what the others do not need.)
+    if (warp < 4) {
+    if constexpr (LIST && list_regs(NQ, Q8).mma < 168) setmaxnreg_dec<list_regs(NQ, Q8).mma>();
+    if (!LIST && warp == 0) {
         // =================================== TMA producer ==================================================
         // The whole warp runs the loop (uniform control flow); one elected lane issues each copy.
         bool ok = true;
@@ -480,71 +556,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
             const int64_t base_row = sc.single ? sc.base0 : M.base[sg.b];
             for (int j = 0; j < sg.n_tiles; j++, it++) {
                 const int s = it & 1;
-                ok = mbar_wait(&B.kv_empty[s], ((it >> 1) & 1) ^ 1, abort_flag, status_w, ST_PRODUCER);
+                ok = bar_wait<LIST>(&B.kv_empty[s], ((it >> 1) & 1) ^ 1, abort_flag, status_w, ST_PRODUCER);
                 if (!ok) break;
                 if (lane == 0) GS_STAMP(it, PF_LOAD_ISSUE);
                 if (lane == 0 && it == 0) GS_CTA_STAMP(7);
                 const int row = sg.r0 + j * TILE;
                 const int valid = min(TILE, sg.r1 - row);
                 uint8_t *dst = kv_smem + s * STAGE_BYTES;
-                if (LIST && Q8) {
-                    // Q8 cache: the listed rows arrive as they are - 512 bytes of int8 per row (one 16-byte copy per lane)
-                    // into the upper half of the stage, their scales (32 bytes per row) beside the stages - and the
-                    // softmax warps widen them to f16 in place before the MMAs see the stage (see there).
-                    const int32_t *lp = P.sel + (int64_t) (sg.b / P.seq_div) * P.sel_stride + row;
-                    const int ra = lane < valid ? max(lp[lane], 0) : 0, rb = lane + 32 < valid ? max(lp[lane + 32], 0) : 0;
-                    const char *qbase = reinterpret_cast<const char *>(P.list_cache);
-                    const char *sbase = reinterpret_cast<const char *>(P.list_scales);
-                    uint8_t *raw = dst + STAGE_BYTES / 2;
-                    uint8_t *qs = qs_smem + s * SM::QS_BYTES;
-#pragma unroll 4
-                    for (int r = 0; r < valid; r++) {
-                        const int grow = __shfl_sync(0xffffffffu, r < 32 ? ra : rb, r & 31);
-                        cp_async16_hint(raw + r * (NBLK * 64) + lane * 16, qbase + (int64_t) grow * (NBLK * 64) + lane * 16, pol_stream);
-                    }
-#pragma unroll
-                    for (int k = 0; k < TILE / 16; k++) {  // scales: two 16-byte halves per row, sixteen rows per instruction
-                        const int r = k * 16 + (lane >> 1);
-                        const int ga = __shfl_sync(0xffffffffu, ra, r & 31), gb = __shfl_sync(0xffffffffu, rb, r & 31);
-                        const int grow = r < 32 ? ga : gb;
-                        if (r < valid)
-                            cp_async16_hint(qs + r * (NBLK * 4) + (lane & 1) * 16, sbase + (int64_t) grow * (NBLK * 4) + (lane & 1) * 16, pol_stream);
-                    }
-                    cp_async_mbar_arrive(&B.kv_raw[s]);
-                    __syncwarp();
-                } else if (LIST) {
-                    // Rows named by the position list.  Lane l holds the cache rows of tile rows l and l + 32; every warp
-                    // instruction copies 512 contiguous bytes of one listed row (16 bytes per lane) to the place the tiled
-                    // copy of the dense form would have put them: 64-column block c / 8, 16-byte chunk (c % 8) xor (r % 8)
-                    // of row r.  Each lane's arrival on the stage's barrier follows its own copies.
-                    // (Measured per 64-row tile of 64 KB, rows already in L2: these copies 2.6 us, the same when four warps
-                    // share the issuing; TMA gather copies of four rows x 64 columns, 128 per tile, 5.9 us issued lane by
-                    // lane from one warp, 3.6 us with one copy per lane from four warps.  A listed row is 1 KB somewhere:
-                    // about 20-25 GB/s per SM whatever issues the requests, against 44 GB/s and more for the tiled copies
-                    // of consecutive rows.  Splitting a tile between the two paths does not add them up: with 16, 24 or 32
-                    // of the 64 rows on gather copies and the rest on these copies the T = 256 shape took 468, 549 and 589 us
-                    // against 343 us, and an evict-last hint on the listed rows 367 us.  Asking for the next tile's list
-                    // entries a tile ahead (346 us) or dropping the eviction hint (339 us) changes nothing either: for that
-                    // shape the profiler shows L2 at 7 %, DRAM at 4 % and the L1 fill path at 8 % of their peaks - the
-                    // copies are bound by what one SM keeps in flight, two 64 KB tiles against 3.2 us of latency each.)
-                    const int32_t *lp = P.sel + (int64_t) (sg.b / P.seq_div) * P.sel_stride + row;
-                    const int ra = lane < valid ? max(lp[lane], 0) : 0, rb = lane + 32 < valid ? max(lp[lane + 32], 0) : 0;
-                    constexpr int CPR = NBLK * 8;  // 16-byte chunks per row
-                    const char *cbase = reinterpret_cast<const char *>(P.list_cache);
-#pragma unroll 4
-                    for (int r = 0; r < valid; r++) {
-                        const int grow = __shfl_sync(0xffffffffu, r < 32 ? ra : rb, r & 31);
-                        const char *src = cbase + (int64_t) grow * (NBLK * 128);
-                        uint8_t *drow = dst + r * 128;
-#pragma unroll
-                        for (int c0 = 0; c0 < CPR; c0 += 32) {
-                            const int c = c0 + lane;
-                            if (c < CPR) cp_async16_hint(drow + (c >> 3) * BLK_BYTES + (((c & 7) ^ (r & 7)) << 4), src + c * 16, pol_stream);
-                        }
-                    }
-                    cp_async_mbar_arrive(&B.kv_full[s][0]);
-                    __syncwarp();
-                } else if (P.paged || valid == TILE) {
+                if (P.paged || valid == TILE) {
                     const int grow = P.paged ? P.page_table[(int64_t) (sg.b / P.seq_div) * P.page_table_stride +
                                                             min(max(row / TILE, 0), P.page_table_stride - 1)] * TILE
                                              : (int) (base_row + row);
@@ -576,8 +595,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
                         }
                     }
                 }
-                if (j == 0 && !(LIST && P.q_f32)) {  // the query rows of this sequence, after the first (larger, farther) cache tile
-                    ok = mbar_wait(&B.q_empty, (sgc & 1) ^ 1, abort_flag, status_w, ST_PRODUCER);
+                if (j == 0) {  // the query rows of this sequence, after the first (larger, farther) cache tile
+                    ok = bar_wait<LIST>(&B.q_empty, (sgc & 1) ^ 1, abort_flag, status_w, ST_PRODUCER);
                     if (!ok) break;
                     if (elect_one()) {
                         if (P.H_full == P.H) {  // the sequence's T*H query rows are contiguous: one box per block
@@ -600,7 +619,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
             }
             sgc++;
         }
-    } else if (warp <= NI) {
+    } else if (warp >= 1 && warp <= NI) {
         // =================================== MMA issuers ====================================================
         // Three warps issue concurrently: one issuer cannot keep the tensor pipe busy with MMAs this
         // small.  Each warp owns its accumulators: a third of the 16-column k-steps of S^T (partial sums,
@@ -617,17 +636,18 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
         const uint64_t d_kmaj = make_smem_desc(0, 16, 1024, kSwizzle128B);         // cache tile / Q, K-major
         const uint64_t d_vt = make_smem_desc(0, BLK_BYTES, 1024, kSwizzle128B);    // cache tile, MN-major
         const uint64_t d_pt = make_smem_desc(0, 128, 1024, kSwizzleNone);          // P^T, MN-major
-        const uint32_t q_lo = smem_u32(q_smem) >> 4, p_lo0 = smem_u32(p_smem) >> 4, kv_lo0 = smem_u32(kv_smem) >> 4;
+        const uint32_t q_lo = smem_desc_addr(q_smem), p_lo0 = smem_desc_addr(p_smem), kv_lo0 = smem_desc_addr(kv_smem);
         bool ok = true;
         while (ok && next_segment(pos, b_cur, end, M.cum, unit_rows, M.len, sg, sc)) {
-            ok = mbar_wait(&B.q_full, sgc & 1, abort_flag, status_w, ST_MMA);
+            if (LIST && sg.n_tiles == 0) continue;  // (cluster form: no share of the rows)
+            ok = bar_wait<LIST>(&B.q_full, sgc & 1, abort_flag, status_w, ST_MMA);
             // S of tile j+1 is issued ahead of P.V of tile j whenever its data has already landed, so it
             // runs on the tensor pipe while the softmax of tile j is computed.
             auto issue_s = [&](uint32_t i) {
                 const int s = i & 1;
                 const uint32_t kv_lo = kv_lo0 + s * (STAGE_BYTES >> 4);
                 tc_fence_after();
-                if (LIST) fence_proxy_async_smem();  // the stage was filled by ordinary asynchronous copies, not by the TMA
+                if (LIST && !Q8) fence_proxy_async_smem();  // the stage was filled by ordinary asynchronous copies, not by the TMA
                 if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < K_PER; k++) {
@@ -648,8 +668,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
                 const uint32_t ph = (it >> 1) & 1;
                 const uint32_t kv_lo = kv_lo0 + s * (STAGE_BYTES >> 4);
                 if (!s_ahead) {
-                    ok = mbar_wait(&B.s_empty[s], ph ^ 1, abort_flag, status_w, ST_MMA);
-                    for (int g = g_lo; ok && g <= g_hi; g++) ok = mbar_wait(&B.kv_full[s][g], ph, abort_flag, status_w, ST_MMA);
+                    ok = bar_wait<LIST>(&B.s_empty[s], ph ^ 1, abort_flag, status_w, ST_MMA);
+                    for (int g = g_lo; ok && g <= g_hi; g++) ok = bar_wait<LIST>(&B.kv_full[s][g], ph, abort_flag, status_w, ST_MMA);
                     if (!ok) break;
                     if (mw == 0 && lane == 0) GS_STAMP(it, PF_KV_FULL);
                     if (mw == 0 && lane == 0 && it == 0) GS_CTA_STAMP(2);
@@ -671,15 +691,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
                     }
                 }
                 // ---- O^T[my tiles] += V^T . P^T ----
-                ok = mbar_wait(&B.p_full[s], ph, abort_flag, status_w, ST_MMA);
+                ok = bar_wait<LIST>(&B.p_full[s], ph, abort_flag, status_w, ST_MMA);
                 // P.V reads every value block of the tile: all groups (they have landed: the scores the softmax
                 // just turned into P needed them; the waits return at once and make that landing visible here)
-                for (int g = 0; ok && g < g_all; g++) ok = mbar_wait(&B.kv_full[s][g], ph, abort_flag, status_w, ST_MMA);
-                if (ok && j == 0) ok = mbar_wait(&B.o_empty, (sgc & 1) ^ 1, abort_flag, status_w, ST_MMA);
+                for (int g = 0; ok && g < g_all; g++) ok = bar_wait<LIST>(&B.kv_full[s][g], ph, abort_flag, status_w, ST_MMA);
+                if (ok && j == 0) ok = bar_wait<LIST>(&B.o_empty, (sgc & 1) ^ 1, abort_flag, status_w, ST_MMA);
                 if (!ok) break;
                 if (mw == 0 && lane == 0) GS_STAMP(it, PF_P_FULL_SEEN);
                 tc_fence_after();
-                if (LIST) fence_proxy_async_smem();
                 const int valid = min(TILE, sg.r1 - (sg.r0 + j * TILE));
                 const int nk = (valid + 15) >> 4;
                 const uint32_t p_lo = p_lo0 + s * (SM::P_BYTES >> 4);
@@ -702,7 +721,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
             }
             sgc++;
         }
-    } else if (warp > N_MMA_WARPS) {  // (with two issuers warp 3 has no part)
+    }
+    } else if (warp < 8) {  // (with two issuers warp 3 has no part)
+        if constexpr (LIST) setmaxnreg_inc<list_regs(NQ, Q8).softmax>();
         // =================================== softmax / epilogue group ==========================================
         const int wg_tid = tid - 32 * (1 + N_MMA_WARPS);
         const int qt = warp & 3;                      // TMEM lane quarter this warp may touch
@@ -718,7 +739,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
         float l_part[HQ];                             // row sums of this thread's cache row, per query row
         float nm[HQ];                                 // minus the reference maximum (log2 units) per query row
         bool ok = true;
-        if (LIST && sc.whole) {
+        if (LIST && sc.whole && sc.share == 1) {
             // a query that attends nothing gets zeros (crates/cuda/kernels/ops.cu:535); such sequences yield no segment
             for (int b = (int) blockIdx.x; b < P.n_seq; b += (int) gridDim.x) {
                 if ((sc.single ? sc.len0 : M.len[b]) > 0) continue;
@@ -727,27 +748,37 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
             }
         }
         while (ok && next_segment(pos, b_cur, end, M.cum, unit_rows, M.len, sg, sc)) {
-            if (LIST && P.q_f32) {
+            if (LIST && sg.n_tiles > 0) {
                 // f32 queries: the four warps round this sequence's rows to f16 straight into the operand layout the
                 // TMA would have produced (64-column blocks of [NQ rows][128 bytes], 16-byte chunk j of row r at chunk
                 // position j ^ (r % 8)), once the MMAs of the previous sequence have finished with the old rows
-                (void) mbar_wait(&B.q_empty, (sgc & 1) ^ 1, abort_flag, status_w, ST_SOFTMAX);
+                (void) bar_wait<LIST>(&B.q_empty, (sgc & 1) ^ 1, abort_flag, status_w, ST_SOFTMAX);
                 const float *qsrc = P.q_f32 + ((int64_t) (sg.b / P.seq_div) * P.H_full + (int64_t) (sg.b % P.seq_div) * P.H) * (NBLK * 64);
                 constexpr int CPR = NBLK * 8;  // 16-byte chunks (8 columns) per row
-                for (int i = wg_tid; i < NQ * CPR; i += 128) {
-                    const int r = i / CPR, cc = i - r * CPR;
-                    uint4 v = make_uint4(0, 0, 0, 0);
-                    if (r < P.rows_q) {
-                        const float4 a = __ldg(reinterpret_cast<const float4 *>(qsrc + (int64_t) r * (NBLK * 64) + cc * 8));
-                        const float4 b4 = __ldg(reinterpret_cast<const float4 *>(qsrc + (int64_t) r * (NBLK * 64) + cc * 8 + 4));
-                        __half2 h;
-                        h = __floats2half2_rn(a.x, a.y); v.x = *reinterpret_cast<uint32_t *>(&h);
-                        h = __floats2half2_rn(a.z, a.w); v.y = *reinterpret_cast<uint32_t *>(&h);
-                        h = __floats2half2_rn(b4.x, b4.y); v.z = *reinterpret_cast<uint32_t *>(&h);
-                        h = __floats2half2_rn(b4.z, b4.w); v.w = *reinterpret_cast<uint32_t *>(&h);
+                constexpr int U = 4;           // chunks per thread requested together
+                static_assert(!LIST || NQ * CPR % (128 * U) == 0, "whole rounds");
+#pragma unroll 1
+                for (int i0 = wg_tid; i0 < NQ * CPR; i0 += 128 * U) {
+                    float4 a[U], b4[U];
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const int i = i0 + u * 128, r = min(i / CPR, P.rows_q - 1), cc = i % CPR;  // (rows past the last: zeros, below)
+                        a[u] = __ldcg(reinterpret_cast<const float4 *>(qsrc + (int64_t) r * (NBLK * 64) + cc * 8));
+                        b4[u] = __ldcg(reinterpret_cast<const float4 *>(qsrc + (int64_t) r * (NBLK * 64) + cc * 8 + 4));
                     }
-                    const int kb = cc >> 3, jj = cc & 7;
-                    *reinterpret_cast<uint4 *>(q_smem + kb * (NQ * 128) + r * 128 + ((jj ^ (r & 7)) << 4)) = v;
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const int i = i0 + u * 128, r = i / CPR, cc = i % CPR;
+                        uint4 v = make_uint4(0, 0, 0, 0);
+                        if (r < P.rows_q) {
+                            __half2 h;
+                            h = __floats2half2_rn(a[u].x, a[u].y); v.x = *reinterpret_cast<uint32_t *>(&h);
+                            h = __floats2half2_rn(a[u].z, a[u].w); v.y = *reinterpret_cast<uint32_t *>(&h);
+                            h = __floats2half2_rn(b4[u].x, b4[u].y); v.z = *reinterpret_cast<uint32_t *>(&h);
+                            h = __floats2half2_rn(b4[u].z, b4[u].w); v.w = *reinterpret_cast<uint32_t *>(&h);
+                        }
+                        *reinterpret_cast<uint4 *>(q_smem + (cc >> 3) * (NQ * 128) + r * 128 + (((cc & 7) ^ (r & 7)) << 4)) = v;
+                    }
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
@@ -768,67 +799,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
                 nm[i] = UNSET;
             }
             named_bar_sync(1, 128);
-            // Q8 cache: widen tile i (the jj-th of this segment): int8 rows (upper half of the stage) x f16 scales ->
-            // half_rn(scale * q) in the operand layout the f16 form's copies produce (crates/cuda/kernels/ops.cu:461-477 attends over
-            // these values).  Each of the four warps takes 16 rows into registers; only when every raw row is in
-            // registers are the f16 rows written, since they cover the raw area.  Rows past the segment's end become
-            // zeros.  Done for the segment's first tile before its scores are awaited and for every further tile right
-            // after the probabilities of the tile before are handed over, so that it runs beside that tile's P.V.
-            // (Measured on 2052-row lists, 64 heads, T = 1 / 2 / 256: 24.9 / 53.4 / 473 us this way; 26.7 / 66.7 / 684 us
-            // with the three issuing warps widening instead - fewer threads, two more barriers, and their MMAs late;
-            // 24.2 / 55.1 / 484 us with one f16 stage filled from a ring of three stand-alone raw buffers - the copies
-            // then never wait for a stage, but widening, scores, softmax and P.V of consecutive tiles no longer
-            // overlap: the chain of hand-overs per tile, not the copies, is what the time follows.)
-            auto widen_tile = [&](uint32_t i, int jj) {
-                const int s = i & 1;
-                (void) mbar_wait(&B.kv_raw[s], (i >> 1) & 1, abort_flag, status_w, ST_SOFTMAX);
-                const int valid_q = min(TILE, sg.r1 - (sg.r0 + jj * TILE));
-                uint8_t *stage = kv_smem + s * STAGE_BYTES;
-                const uint8_t *raw = stage + STAGE_BYTES / 2;
-                const uint8_t *qs = qs_smem + s * SM::QS_BYTES;
-                uint4 rv[16];
-#pragma unroll
-                for (int k = 0; k < 16; k++) rv[k] = *reinterpret_cast<const uint4 *>(raw + (qt * 16 + k) * (NBLK * 64) + lane * 16);
-                named_bar_sync(1, 128);
-#pragma unroll
-                for (int k = 0; k < 16; k++) {
-                    const int r = qt * 16 + k;
-                    // scale * q as an f16 product: q (|q| <= 127) is exact in f16 and the product of an 11-bit by a 7-bit
-                    // significand is exact before the one rounding, so this is half_rn(scale * q) bit for bit.  The bytes
-                    // become f16 through the 1024-offset trick: 0x6400 | (q + 128) is the f16 number 1152 + q.
-                    const __half sc = r < valid_q ? *reinterpret_cast<const __half *>(qs + r * (NBLK * 4) + (lane >> 1) * 2) : __ushort_as_half(0);
-                    const __half2 sc2 = __half2half2(sc), off2 = __half2half2(__ushort_as_half(0x6480));  // 1152
-                    auto widen4 = [&](uint32_t w, uint32_t &h01, uint32_t &h23) {
-                        const uint32_t u = w ^ 0x80808080u;
-                        uint32_t a = __byte_perm(u, 0x64646464u, 0x5140), b2 = __byte_perm(u, 0x64646464u, 0x7362);
-                        const __half2 x = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&a), off2), sc2);
-                        const __half2 y = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&b2), off2), sc2);
-                        h01 = *reinterpret_cast<const uint32_t *>(&x);
-                        h23 = *reinterpret_cast<const uint32_t *>(&y);
-                    };
-                    uint4 lo, hi;
-                    widen4(rv[k].x, lo.x, lo.y);
-                    widen4(rv[k].y, lo.z, lo.w);
-                    widen4(rv[k].z, hi.x, hi.y);
-                    widen4(rv[k].w, hi.z, hi.w);
-                    if (r >= valid_q) lo = hi = make_uint4(0, 0, 0, 0);  // (a stale byte times a zero scale is zero too; this says so)
-                    // 16-byte chunks 2 * lane and 2 * lane + 1 of the row.  Lanes of every other 64-column block store
-                    // their odd chunk first, so that one store instruction covers all eight chunk positions of the
-                    // 128-byte lines (four lanes each) instead of four positions (eight lanes each).
-                    const int flip = (lane >> 2) & 1;
-                    const int c0 = lane * 2 + flip, c1 = lane * 2 + 1 - flip;
-                    *reinterpret_cast<uint4 *>(stage + (c0 >> 3) * BLK_BYTES + r * 128 + (((c0 & 7) ^ (r & 7)) << 4)) = flip ? hi : lo;
-                    *reinterpret_cast<uint4 *>(stage + (c1 >> 3) * BLK_BYTES + r * 128 + (((c1 & 7) ^ (r & 7)) << 4)) = flip ? lo : hi;
-                }
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&B.kv_full[s][0]);
-            };
             for (int j = 0; j < sg.n_tiles; j++, it++) {
                 const int s = it & 1;
                 const uint32_t ph = (it >> 1) & 1;
-                if (Q8 && j == 0) widen_tile(it, 0);
-                (void) mbar_wait(&B.s_full[s], ph, abort_flag, status_w, ST_SOFTMAX);
+                (void) bar_wait<LIST>(&B.s_full[s], ph, abort_flag, status_w, ST_SOFTMAX);
                 GS_STAMP(it, PF_S_FULL);
                 tc_fence_after();
                 const int row0 = sg.r0 + j * TILE;
@@ -914,7 +888,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
                         nm[i] = mr == -INFINITY ? UNSET : -mr;
                     }
                 }
-                (void) mbar_wait(&B.p_empty[s], ph ^ 1, abort_flag, status_w, ST_SOFTMAX);
+                (void) bar_wait<LIST>(&B.p_empty[s], ph ^ 1, abort_flag, status_w, ST_SOFTMAX);
                 // probabilities: row sums in registers; P^T as f16, 8 query rows per 16-byte store, in the
                 // MN-major operand layout [q/8][row/8][row%8][q%8].  A masked score is -inf and gives 0; an
                 // unset column holds only masked scores.
@@ -937,7 +911,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
                 }
                 if (rescale) {
                     // S of this tile may have been issued ahead of P.V of the previous one: wait for that P.V
-                    (void) mbar_wait(&B.p_empty[s ^ 1], ((it - 1) >> 1) & 1, abort_flag, status_w, ST_SOFTMAX);
+                    (void) bar_wait<LIST>(&B.p_empty[s ^ 1], ((it - 1) >> 1) & 1, abort_flag, status_w, ST_SOFTMAX);
                     tc_fence_after();
 #pragma unroll 1
                     for (int mt = 0; mt < NVT; mt++) {
@@ -956,7 +930,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
                 }
                 // rows of the last 16-row group past the segment's end must not feed NaNs into P.V
                 const int valid = min(TILE, sg.r1 - row0);
-                if (valid & 15) {
+                if (!LIST && (valid & 15)) {  // (the producers of the list form store zeros there)
                     const int r_lo = valid, r_hi = (valid + 15) & ~15;
                     const int n_vec = (r_hi - r_lo) * NBLK * 8;  // 16-byte vectors
                     uint8_t *stage = kv_smem + s * STAGE_BYTES;
@@ -971,11 +945,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&B.p_full[s]);
                 GS_STAMP(it, PF_P_WRITTEN);
-                if (Q8 && j + 1 < sg.n_tiles) widen_tile(it + 1, j + 1);
             }
             if (!ok) break;
             // ---- end of segment: drain the accumulators into this segment's partial record ----------------
-            (void) mbar_wait(&B.o_full, sgc & 1, abort_flag, status_w, ST_SOFTMAX);
+            if (!LIST || sg.n_tiles > 0) (void) bar_wait<LIST>(&B.o_full, sgc & 1, abort_flag, status_w, ST_SOFTMAX);
             named_bar_sync(2, 128);
             if (*abort_flag) { ok = false; break; }
             tc_fence_after();
@@ -991,6 +964,100 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
                 if ((lane & 15) == 0) M.sl[qt][col0 + i] = v;
             }
             named_bar_sync(1, 128);
+            if (LIST && sc.share > 1) {
+                // ---- the CTAs of the cluster merge their parts through distributed shared memory -----------------------
+                // Every CTA tells all others that its MMAs are done with its stages, stages its accumulators column block
+                // by column block, and sends each CTA its 512 / cluster columns (and everybody its (m, l)) by bulk copies;
+                // then it adds up the columns it was sent, each source weighted by e^(m - M) / L (the arithmetic of
+                // ops.cu:552-574), and stores them.
+                // (About 5 us for 16 CTAs x 64 KB, half of it the copies at 27 GB/s per SM.  With 4-byte stores to the other CTAs instead of bulk copies 6.4 us, with
+                // 16-byte stores a row apart 9 us, and 3.3 us more for exchanging the maxima first.)
+                const int share = sc.share, cols = 512 / share;
+                float *const x_acc = reinterpret_cast<float *>(kv_smem), *const x_out = reinterpret_cast<float *>(smem + SM::OFF_XOUT);
+                // "ready" of a round: this CTA takes the copies of the round and has everything of the round before, so that the
+                // others may fill their staging area again (one round up to 48 query rows, two for 64)
+                auto ready = [&](int nq, bool first) {
+                    if (wg_tid == 0) mbar_arrive_expect_tx(&B.x_data, (uint32_t) (nq * 512 * 4 + (first ? share * P.rows_q * 8 : 0)));
+                    __syncwarp();
+                    if (wg_tid < share) mbar_arrive_cluster(mapa(smem_u32(&B.x_ready), wg_tid));
+                };
+                ready(min(SM::X_ROWS, P.rows_q), true);
+                if (wg_tid < NQ) M.x_mine[wg_tid] = make_float2(M.mref[wg_tid], (M.sl[0][wg_tid] + M.sl[1][wg_tid]) + (M.sl[2][wg_tid] + M.sl[3][wg_tid]));
+                bool xok = true;
+#pragma unroll 1
+                for (int q0 = 0; q0 < P.rows_q; q0 += SM::X_ROWS) {
+                    const int nq = min(SM::X_ROWS, P.rows_q - q0);
+                    if (q0 > 0) {
+                        xok = xok && mbar_wait_cluster(&B.x_data, 0, abort_flag, status_w, ST_SOFTMAX);
+                        ready(nq, false);
+                        xok = xok && mbar_wait_cluster(&B.x_ready, 1, abort_flag, status_w, ST_SOFTMAX);
+                    }
+#pragma unroll 1
+                    for (int mt = 0; mt < NVT; mt++) {
+                        const int c0 = mt * 128 + qt * 32;
+                        float *const dst = x_out + c0 / cols * nq * cols + c0 % cols + lane;
+#pragma unroll
+                        for (int c = 0; c < SM::X_ROWS / 16; c++) {
+                            uint32_t r[16];
+                            if (sg.n_tiles > 0) {
+                                tmem_ld16(tmem + lane_base + (O_SLOT0 + mt) * NQ + q0 + c * 16, r);
+                                tmem_wait_ld();
+                            }
+#pragma unroll
+                            for (int i = 0; i < 16; i++)
+                                if (c * 16 + i < nq) dst[(c * 16 + i) * cols] = sg.n_tiles > 0 ? __uint_as_float(r[i]) : 0.f;
+                        }
+                    }
+                    fence_proxy_async_smem();
+                    named_bar_sync(1, 128);
+                    if (wg_tid < share) {  // thread i: what CTA i of the cluster gets
+                        if (q0 == 0) xok = mbar_wait_cluster(&B.x_ready, 0, abort_flag, status_w, ST_SOFTMAX);
+                        if (xok) {
+                            const uint32_t bar = mapa(smem_u32(&B.x_data), wg_tid);
+                            bulk_copy_cluster(mapa(smem_u32(x_acc + (sc.rank * P.rows_q + q0) * cols), wg_tid), x_out + wg_tid * nq * cols, (uint32_t) (nq * cols * 4), bar);
+                            if (q0 == 0) bulk_copy_cluster(mapa(smem_u32(&M.x_ml[sc.rank][0]), wg_tid), M.x_mine, (uint32_t) (P.rows_q * 8), bar);
+                        }
+                    }
+                }
+                tc_fence_before();
+                if (xok) xok = mbar_wait_cluster(&B.x_data, P.rows_q > SM::X_ROWS, abort_flag, status_w, ST_SOFTMAX);
+                if (group_any(2, 128, !xok || *abort_flag)) { ok = false; break; }  // (one decision for the group)
+                if (wg_tid < P.rows_q) {
+                    float mx = -INFINITY;
+                    for (int r = 0; r < share; r++) mx = fmaxf(mx, M.x_ml[r][wg_tid].x);
+                    float l = 0.f;
+                    for (int r = 0; r < share; r++) {
+                        const float2 v = M.x_ml[r][wg_tid];
+                        const float w = v.x == -INFINITY ? 0.f : exp2f(v.x - mx);
+                        l = fmaf(v.y, w, l);
+                        M.x_w[r][wg_tid] = w;
+                    }
+                    M.f[wg_tid] = l > 0.f ? 1.f / l : 0.f;
+                }
+                named_bar_sync(1, 128);
+                float *dst = P.o + ((int64_t) (sg.b / P.seq_div) * P.H_out + (sg.b % P.seq_div) * P.H) * P.d_v + sc.rank * cols;
+                const int cq = cols / 4, stride = P.rows_q * cols;
+                for (int i = wg_tid; i < cq * P.rows_q; i += 128) {
+                    const int q = i / cq, c = (i - q * cq) * 4;
+                    const float *src = x_acc + q * cols + c;
+                    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+                    for (int r = 0; r < share; r++) {
+                        const float w = M.x_w[r][q];
+                        const float4 u = *reinterpret_cast<const float4 *>(src + r * stride);
+                        if (w != 0.f) {  // an empty part's accumulator never enters the sum
+                            a.x = fmaf(u.x, w, a.x);
+                            a.y = fmaf(u.y, w, a.y);
+                            a.z = fmaf(u.z, w, a.z);
+                            a.w = fmaf(u.w, w, a.w);
+                        }
+                    }
+                    const float inv = M.f[q];
+                    *reinterpret_cast<float4 *>(dst + (int64_t) q * P.d_v + c) = make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv);
+                }
+                sgc++;
+                continue;
+            }
             if (LIST && sc.whole) {
                 // the whole sequence was attended here: no record, no merge - normalise and store (ops.cu:531-538)
                 if (wg_tid < NQ) {
@@ -1028,7 +1095,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
             float *acc = P.ws_acc + (int64_t) sg.seg_id * P.rows_q * P.d_v + qt * 32 + lane;
             // one value tile (NQ columns of this lane's row) per step; the loads of the next tile are in flight
             // while the current one is stored
-            constexpr int NB = NQ > 48 ? 1 : 2;  // (64 columns twice over would not leave the registers for the rest)
+            constexpr int NB = LIST || NQ > 48 ? 1 : 2;  // (64 columns twice over would not leave the registers for the rest)
             uint32_t rbuf[NB][NQ];
             if (NB == 2) {
 #pragma unroll
@@ -1061,11 +1128,118 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
             if (wg_tid == 0) GS_CTA_STAMP(4);
             sgc++;
         }
+    } else if (LIST) {
+        if constexpr (list_regs(NQ, Q8).producer < 168) setmaxnreg_dec<list_regs(NQ, Q8).producer>();
+        if constexpr (list_regs(NQ, Q8).producer > 168) setmaxnreg_inc<list_regs(NQ, Q8).producer>();
+        // =================================== producers of the list form ========================================
+        // Rows named by the position list.  Warp w of the four takes tile rows w, w + 4, ...; a row goes to the place the
+        // tiled copy of the dense form would have put it: 64-column block c / 8, 16-byte chunk (c % 8) xor (r % 8) of row r.
+        // f16 rows: asynchronous 16-byte copies, 512 contiguous bytes of a row per instruction; each lane's arrival on the
+        // stage's barrier follows its own copies.  Q8 rows: 16 rows per warp requested together into registers (one 16-byte
+        // load and a scale per lane and row) while the stage is still in use, widened on the way into it.
+        // (What a tile takes alone, 64 KB of rows in L2, all SMs at once: one warp of asynchronous copies 1.8 us, two 1.1,
+        // four 0.8; four warps through registers 1.1; TMA boxes of 4 rows x 64 columns 3.9 us from one warp, 1.2 from four;
+        // TMA tiles of consecutive rows 0.54.  In the kernel, 256-token chunk of 2052-row lists, 64 heads: one warp 190 us,
+        // two 183, four 166 us, four through registers 228 us.)
+        const int pw = warp - 8;
+        bool ok = true;
+        while (ok && next_segment(pos, b_cur, end, M.cum, unit_rows, M.len, sg, sc)) {
+            const int32_t *lp = P.sel + (int64_t) (sg.b / P.seq_div) * P.sel_stride + sg.r0;
+            const int n_rows = sg.r1 - sg.r0;
+            int n_left = n_rows;
+            // lane l holds the cache rows of tile rows l and l + 32, of this tile and of the next (requested a tile ahead)
+            auto entry = [&](int i) { return i < n_rows ? max(__ldcg(lp + i), 0) : 0; };
+            int ra = entry(lane), rb = entry(lane + 32), na = entry(TILE + lane), nb = entry(TILE + lane + 32);
+            for (int j = 0; j < sg.n_tiles; j++, it++, n_left -= TILE) {
+                const int s = it & 1;
+                uint8_t *dst = kv_smem + s * STAGE_BYTES;
+                auto row_of = [&](int r) { return (int64_t) __shfl_sync(0xffffffffu, r < 32 ? ra : rb, r & 31); };
+                auto next_rows = [&]() {
+                    ra = na;
+                    rb = nb;
+                    na = entry((j + 2) * TILE + lane);
+                    nb = entry((j + 2) * TILE + lane + 32);
+                };
+                constexpr int RPW = TILE / 4;
+                if (Q8) {
+                    // int8 rows and their f16 scales, widened to half_rn(scale * q), the values crates/cuda/kernels/ops.cu:461-477
+                    // attends over
+                    const char *qbase = reinterpret_cast<const char *>(P.list_cache) + lane * 16;
+                    const __half *sbase = P.list_scales + (lane >> 1);
+                    uint4 v[RPW];
+                    __half sc_row[RPW];
+#pragma unroll
+                    for (int k = 0; k < RPW; k++) {
+                        const int r = k * 4 + pw;
+                        const int64_t g = row_of(r);
+                        v[k] = make_uint4(0, 0, 0, 0);
+                        sc_row[k] = __ushort_as_half(0);  // rows past the segment's end become zeros
+                        if (r < n_left) {
+                            v[k] = ld_global_stream(qbase + g * (NBLK * 64));
+                            sc_row[k] = __ldcg(sbase + g * (NBLK * 2));
+                        }
+                    }
+                    next_rows();
+                    ok = bar_wait<LIST>(&B.kv_empty[s], ((it >> 1) & 1) ^ 1, abort_flag, status_w, ST_PRODUCER);
+                    if (!ok) break;
+                    // lanes of every other 64-column block store their odd chunk first, so that one store instruction covers
+                    // all eight chunk positions of the 128-byte lines (four lanes each) instead of four (eight lanes each)
+                    const int flip = (lane >> 2) & 1;
+                    const int c0 = lane * 2 + flip, c1 = lane * 2 + 1 - flip;
+#pragma unroll
+                    for (int k = 0; k < RPW; k++) {
+                        const int r = k * 4 + pw;
+                        // scale * q as an f16 product: q (|q| <= 127) is exact in f16 and the product of an 11-bit by a 7-bit
+                        // significand is exact before the one rounding, so this is half_rn(scale * q) bit for bit.  The bytes
+                        // become f16 through the 1024-offset trick: 0x6400 | (q + 128) is the f16 number 1152 + q.
+                        const __half2 sc2 = __half2half2(sc_row[k]), off2 = __half2half2(__ushort_as_half(0x6480));  // 1152
+                        auto widen4 = [&](uint32_t w, uint32_t &h01, uint32_t &h23) {
+                            const uint32_t u = w ^ 0x80808080u;
+                            uint32_t a = __byte_perm(u, 0x64646464u, 0x5140), b2 = __byte_perm(u, 0x64646464u, 0x7362);
+                            const __half2 x = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&a), off2), sc2);
+                            const __half2 y = __hmul2(__hsub2(*reinterpret_cast<const __half2 *>(&b2), off2), sc2);
+                            h01 = *reinterpret_cast<const uint32_t *>(&x);
+                            h23 = *reinterpret_cast<const uint32_t *>(&y);
+                        };
+                        uint4 lo, hi;
+                        widen4(v[k].x, lo.x, lo.y);
+                        widen4(v[k].y, lo.z, lo.w);
+                        widen4(v[k].z, hi.x, hi.y);
+                        widen4(v[k].w, hi.z, hi.w);
+                        *reinterpret_cast<uint4 *>(dst + (c0 >> 3) * BLK_BYTES + r * 128 + (((c0 & 7) ^ (r & 7)) << 4)) = flip ? hi : lo;
+                        *reinterpret_cast<uint4 *>(dst + (c1 >> 3) * BLK_BYTES + r * 128 + (((c1 & 7) ^ (r & 7)) << 4)) = flip ? lo : hi;
+                    }
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&B.kv_full[s][0]);
+                } else {
+                    ok = bar_wait<LIST>(&B.kv_empty[s], ((it >> 1) & 1) ^ 1, abort_flag, status_w, ST_PRODUCER);
+                    if (!ok) break;
+                    if (pw == 0 && lane == 0) GS_STAMP(it, PF_LOAD_ISSUE);
+                    const char *cbase = reinterpret_cast<const char *>(P.list_cache) + lane * 16;
+#pragma unroll
+                    for (int k = 0; k < RPW; k++) {
+                        const int r = k * 4 + pw;
+                        const char *src = cbase + row_of(r) * (NBLK * 128);
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            const int c = h * 32 + lane;
+                            uint8_t *d = dst + (c >> 3) * BLK_BYTES + r * 128 + (((c & 7) ^ (r & 7)) << 4);
+                            if (r < n_left) cp_async16(d, src + h * 512);
+                            else *reinterpret_cast<uint4 *>(d) = make_uint4(0, 0, 0, 0);  // rows past the segment's end become zeros
+                        }
+                    }
+                    cp_async_mbar_arrive(&B.kv_full[s][0]);
+                    next_rows();
+                }
+            }
+        }
     }
 
     // ---- common exit -----------------------------------------------------------------------------------------
     tc_fence_before();
     __syncthreads();
+    if (LIST && sc.share > 1) cluster_sync();  // no CTA leaves while another may still write to its shared memory
     if (*abort_flag && tid == 0) {
         // loads that were issued but never consumed may still be landing in this CTA's shared memory
         const long long t0 = clock64();
@@ -1085,20 +1259,27 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_decode_umma(const __grid_consta
 
 template <int NQ, int NBLK, bool LIST = false, bool Q8 = false>
 int launch_cfg(const UmmaParams &P, int grid, cudaStream_t st) {
-    const int smem = Smem<NQ, NBLK, Q8>::TOTAL;
+    const int smem = Smem<NQ, NBLK>::TOTAL;
     // attributes are set on every call: a cached flag would go stale across a device reset
     GS_TRY(cudaFuncSetAttribute(k_decode_umma<NQ, NBLK, LIST, Q8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(NTHREADS);
+    cfg.blockDim = dim3(LIST ? LIST_NTHREADS : NTHREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     // programmatic dependent launch: the CTA-local set-up may overlap the tail of the preceding kernel
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    if (LIST && P.cluster > 1) {
+        if (P.cluster > 8) GS_TRY(cudaFuncSetAttribute(k_decode_umma<NQ, NBLK, LIST, Q8>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = P.cluster;
+        attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+        cfg.numAttrs = 2;
+    }
     GS_TRY(cudaLaunchKernelEx(&cfg, k_decode_umma<NQ, NBLK, LIST, Q8>, P));
     return 0;
 }
@@ -1110,68 +1291,79 @@ int read_list_status(int32_t *out) {
     return 0;
 }
 
-// Position lists on the tensor cores.  Head groups of at most 48 heads (a multiple of 8 each): 0 = not cut that way.
-// (49..64 heads may also run as one group of 64 query columns, see launch_decode_umma_list.)
+// Head counts the list form takes: those that can be cut into equal groups of at most 48 heads (a multiple of 8 each).
 static int list_head_groups(int H) {
     const int n = (H + 47) / 48;
     return (n > 0 && H % n == 0 && (H / n) % 8 == 0) ? n : 0;
 }
 
-// Returns 0 when launched, -1 when the shape is not taken by the tcgen05 kernel (the caller then runs the CUDA-core
-// kernel), or a cudaError_t.  Every (token, head group) is a kernel sequence over the token's list.  With one split, or
-// when the caller's `part` cannot hold enough records, every sequence is attended by one CTA that stores o itself;
-// otherwise the rows are dealt to CTAs as in the dense form and the records live in `part`
-// (T*H*splits*(R+2) floats, crates/cuda/kernels/ops.cu:578): accumulators [segment][row][R], then (m, l) [segment][row][2], then
-// the per-sequence descriptors.
-// What a cut into n_groups head groups gives: the grid, whether every (token, group) is attended whole by one CTA, and
-// the longest run of tiles one CTA walks (what the call's time follows).
+// How a call is cut: head groups, and who attends a (token, head group) - a kernel sequence.
 struct ListPlan {
-    int n_groups, grid, grid_rec, grid_whole;
-    bool whole;
-    int64_t depth;
+    int n_groups, grid, cluster;
+    bool whole;   // one CTA or one cluster per kernel sequence stores o itself; else records in the caller's `part`
+    float cost;   // estimated time, microseconds
 };
-static ListPlan list_plan(int n_groups, int T, int H, int R, int sel_stride, int splits, const float *part, int grid_max) {
-    ListPlan L{};
-    L.n_groups = n_groups;
-    const int Hg = H / n_groups;
-    const int64_t n_seq_k = (int64_t) T * n_groups;
-    const int64_t tiles_seq = (sel_stride + TILE - 1) / TILE;
-    // records that fit the caller's buffer
-    if (splits > 1 && part && !(reinterpret_cast<uintptr_t>(part) & 15)) {
-        const int64_t part_floats = (int64_t) T * H * splits * (R + 2);
-        const int64_t desc_floats = (n_seq_k * 2 + 3) / 4 * 4;
-        const int64_t segs = (part_floats - desc_floats) / ((int64_t) Hg * (R + 2));
-        const int64_t tiles = n_seq_k * tiles_seq;
-        int64_t g = segs - n_seq_k;
-        if (g > grid_max) g = grid_max;
-        if (g > tiles) g = tiles;
-        L.grid_rec = (int) (g > 0 ? g : 0);
+// Three ways, all with the same results:
+//  * one CTA per sequence, in rounds when there are more sequences than SMs;
+//  * a cluster of 2 to 16 CTAs per sequence, which merge through distributed shared memory - when all clusters run at once;
+//  * the rows of all sequences dealt to CTAs as in the dense form, records in `part` (as many segments as its
+//    T*H*splits*(R+2) floats hold), a combine launch - long lists with a large `part`.
+// The estimate: a CTA's longest run of 64-row tiles times the time of a tile, plus what the merge costs.  Measured over 2052-row
+// lists, 1 to 256 tokens, 16 to 64 heads, every cut (f16 / Q8 cache): a tile 2.2 / 3.0 us with up to 32 query columns and
+// 2.85 / 3.4 with 64, 2.5 and 3.1 in a cluster; a cluster's start and merge 7.5 / 9.5 us, 17 with 64 columns (two rounds of the
+// exchange), 2.5 more with 16 CTAs and a little for every CTA that fetches; records and their combine 11 us, 7 when there is one sequence (its schedule needs no
+// scan).  The choice it makes is within about 6 % of the best cut measured.
+static ListPlan list_plan(int T, int H, int R, int sel_stride, int splits, const float *part, bool q8, int grid_max) {
+    ListPlan best{0, 0, 1, true, 1e30f};
+    auto offer = [&](int n, int64_t grid, int cluster, bool whole, float cost) {
+        if (cost < best.cost) best = ListPlan{n, (int) grid, cluster, whole, cost};
+    };
+    for (int n = 1; n <= 8; n++) {
+        if (H % n || (H / n) % 8 || H / n > 64) continue;
+        const int Hg = H / n;
+        const int64_t n_seq_k = (int64_t) T * n, tiles_seq = (sel_stride + TILE - 1) / TILE;
+        if (n_seq_k > MAX_SEQ) break;
+        const float t_one = (Hg <= 32 ? 2.2f : Hg <= 48 ? 2.5f : 2.85f) + (q8 ? (Hg <= 48 ? 0.8f : 0.55f) : 0.f);
+        const float t_cl = (Hg <= 32 ? 2.5f : Hg <= 48 ? 2.8f : 3.1f) + (q8 ? 0.2f : 0.f);
+        const int64_t grid = n_seq_k < grid_max ? n_seq_k : grid_max;
+        offer(n, grid, 1, true, (float) ((n_seq_k + grid - 1) / grid * tiles_seq) * t_one + 2.f);
+        for (int c = 2; c <= MAX_CLUSTER; c *= 2) {
+            // CTAs of clusters of c that run at once on 148 SMs, one per SM
+            const int resident = c == 2 ? 148 : c == 4 ? 132 : c == 8 ? 120 : 112;
+            if (n_seq_k * c > (resident < grid_max ? resident : grid_max)) break;
+            const int64_t per = (sel_stride + c - 1) / c;
+            offer(n, n_seq_k * c, c, true, (float) ((per + TILE - 1) / TILE) * t_cl + (Hg <= 48 ? 6.5f + 0.03f * (float) Hg : 17.f) +
+                                               (c == 16 ? 2.5f : 0.f) + (q8 ? 2.f : 0.f) + 0.03f * (float) (n_seq_k * c));
+        }
+        if (splits > 1 && part && !(reinterpret_cast<uintptr_t>(part) & 15)) {
+            // records that fit the caller's buffer
+            const int64_t part_floats = (int64_t) T * H * splits * (R + 2);
+            const int64_t desc_floats = (n_seq_k * 2 + 3) / 4 * 4;
+            const int64_t segs = (part_floats - desc_floats) / ((int64_t) Hg * (R + 2));
+            const int64_t tiles = n_seq_k * tiles_seq;
+            int64_t g = segs - n_seq_k;
+            if (g > grid_max) g = grid_max;
+            if (g > tiles) g = tiles;
+            if (g > 0) offer(n, g, 1, false, (float) ((tiles + g - 1) / g) * t_cl + (n_seq_k == 1 ? 7.f : 11.f) + (q8 ? 2.f : 0.f));
+        }
     }
-    L.grid_whole = (int) (n_seq_k < grid_max ? n_seq_k : grid_max);
-    L.whole = L.grid_rec <= L.grid_whole;
-    L.grid = L.whole ? L.grid_whole : L.grid_rec;
-    L.depth = L.whole ? (n_seq_k + L.grid - 1) / L.grid * tiles_seq : (n_seq_k * tiles_seq + L.grid - 1) / L.grid;
-    return L;
+    return best;
 }
 
+// Position lists on the tensor cores.  Returns 0 when launched, -1 when the shape is not taken by the tcgen05 kernel (the
+// caller then runs the CUDA-core kernel), or a cudaError_t.  Every (token, head group) is a kernel sequence over the token's
+// list.  Records, when the plan has any, live in `part` (T*H*splits*(R+2) floats, crates/cuda/kernels/ops.cu:578):
+// accumulators [segment][row][R], then (m, l) [segment][row][2], then the per-sequence descriptors.
 int launch_decode_umma_list(const float *q, const void *C, const __half *C_scales, const int32_t *sel, int sel_stride, const int32_t *cnt,
                             float scale, float *o, float *part, int T, int H, int R, int splits, int sm_count, cudaStream_t st) {
-    const int g48 = list_head_groups(H);
-    if (R != 512 || g48 == 0 || sel_stride <= 0 || !(scale > 0.f)) return -1;
+    if (R != 512 || list_head_groups(H) == 0 || sel_stride <= 0 || !(scale > 0.f)) return -1;
     if ((reinterpret_cast<uintptr_t>(C) & 15) || (reinterpret_cast<uintptr_t>(q) & 15) || (reinterpret_cast<uintptr_t>(C_scales) & 15)) return -1;
     int grid_max = sm_count < kMaxCtas ? sm_count : kMaxCtas;
     if (grid_max < 1) grid_max = 1;
-    // 49..64 heads: two groups of at most 32 heads (the listed rows are copied once per group), or all heads in one
-    // pass with 64 query columns and two issuing warps.  Listed rows arrive at a latency-bound rate per SM, so the
-    // cut with the shorter longest run of tiles wins; the two-group form on a tie.
-    ListPlan L = list_plan(g48, T, H, R, sel_stride, splits, part, grid_max);
-    if (H > 48 && H <= 64 && !C_scales) {  // (the 64-column form is built for the f16 cache only)
-        const ListPlan L1 = list_plan(1, T, H, R, sel_stride, splits, part, grid_max);
-        if (L1.depth < L.depth) L = L1;
-    }
+    const ListPlan L = list_plan(T, H, R, sel_stride, splits, part, C_scales != nullptr, grid_max);
+    if (L.n_groups == 0) return -1;
     const int n_groups = L.n_groups;
     const int64_t n_seq_k = (int64_t) T * n_groups;
-    if (n_seq_k > MAX_SEQ) return -1;
     const int Hg = H / n_groups;
     UmmaParams P;
     memset(&P, 0, sizeof(P));
@@ -1205,6 +1397,7 @@ int launch_decode_umma_list(const float *q, const void *C, const __half *C_scale
     const bool whole = L.whole;
     const int grid = L.grid;
     P.whole_seq = whole ? 1 : 0;
+    P.cluster = L.cluster;
     CombinePlan c{};
     if (!whole) {
         P.seg_cap = grid + (int) n_seq_k;
@@ -1232,10 +1425,10 @@ int launch_decode_umma_list(const float *q, const void *C, const __half *C_scale
         c.bulk = true;
     }
     int e;
-    if (C_scales) e = Hg <= 32 ? launch_cfg<32, 8, true, true>(P, grid, st) : launch_cfg<48, 8, true, true>(P, grid, st);
-    else if (Hg <= 32) e = launch_cfg<32, 8, true>(P, grid, st);
-    else if (Hg <= 48) e = launch_cfg<48, 8, true>(P, grid, st);
-    else e = launch_cfg<64, 8, true>(P, grid, st);
+    if (C_scales)
+        e = Hg <= 32 ? launch_cfg<32, 8, true, true>(P, grid, st) : Hg <= 48 ? launch_cfg<48, 8, true, true>(P, grid, st) : launch_cfg<64, 8, true, true>(P, grid, st);
+    else
+        e = Hg <= 32 ? launch_cfg<32, 8, true>(P, grid, st) : Hg <= 48 ? launch_cfg<48, 8, true>(P, grid, st) : launch_cfg<64, 8, true>(P, grid, st);
     if (e) return e;
     if (!whole) return launch_combine(c, st);
     return 0;

@@ -127,9 +127,6 @@ __device__ __forceinline__ void bulk_load(void *smem_dst, const void *gsrc, uint
 }
 // 16 bytes global -> shared by the asynchronous copy unit (bypassing L1), and the arrival that lets an mbarrier track
 // all copies the executing thread has issued so far (the arrival counts against the barrier's expected count).
-__device__ __forceinline__ void cp_async16_hint(void *smem_dst, const void *gsrc, uint64_t policy) {
-    asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)), "l"(gsrc), "l"(policy) : "memory");
-}
 __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
 }
@@ -225,6 +222,9 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t 
     return (uint64_t) ((smem_addr >> 4) & 0x3FFF) | ((uint64_t) ((lbo_bytes >> 4) & 0x3FFF) << 16) |
            ((uint64_t) ((sbo_bytes >> 4) & 0x3FFF) << 32) | (1ull << 46) | (swizzle << 61);
 }
+// The address field to add to a descriptor made with address 0.  (In a thread-block cluster the upper bits of a shared-memory
+// address hold the CTA's rank; they must not run into the fields above.)
+__device__ __forceinline__ uint32_t smem_desc_addr(const void *p) { return (smem_u32(p) & 0x3ffff) >> 4; }
 // Instruction descriptor for kind::f16 with f16 operands and f32 accumulation.
 // a_mn / b_mn: 1 when the operand is MN-major (its M or N index is the contiguous one), 0 for K-major.
 __host__ __device__ constexpr uint32_t make_idesc_f16(int m, int n, int a_mn, int b_mn) {
@@ -292,6 +292,67 @@ __device__ __forceinline__ bool group_any(int id, int n_threads, bool pred) {
         : "r"((uint32_t) pred), "r"(id), "r"(n_threads)
         : "memory");
     return out != 0;
+}
+
+// ---- thread-block clusters and distributed shared memory ---------------------------------------------------
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The address of shared-memory location `addr` of this CTA in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t mapa(uint32_t addr, int rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+// Bulk copy of this CTA's shared memory into another CTA's (address and barrier from mapa; 16-byte aligned, a multiple of 16
+// bytes), completion counted in bytes on that CTA's barrier.
+__device__ __forceinline__ void bulk_copy_cluster(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "r"(smem_u32(src)),
+                 "r"(bytes), "r"(bar)
+                 : "memory");
+}
+// Arrival on a barrier of another CTA (address from mapa).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+// Bounded wait on one of this CTA's barriers that other CTAs arrive on.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int32_t *status, int32_t code) {
+    const long long t0 = clock64();
+    for (int spins = 0;; spins++) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t"
+            ".reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t"
+            "}\n"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+        if (ok) return true;
+        if ((spins & 63) == 63) {
+            if (*abort_flag) return false;
+            if (clock64() - t0 > kWaitLimitCycles) {
+                *abort_flag = 1;
+                if (status) atomicOr(status, code);
+                return false;
+            }
+        }
+    }
+}
+
+// ---- register hand-over between the warpgroups of a block (executed by all four warps of one) ----------------
+template <int N>
+__device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void setmaxnreg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// 16 bytes of data that is not read again by this SM: past L1.
+__device__ __forceinline__ uint4 ld_global_stream(const void *p) {
+    uint4 v;
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
 }
 
 }  // namespace sm100

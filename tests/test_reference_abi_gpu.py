@@ -279,6 +279,41 @@ def test_gs_mla_attn_tensor_kernel_vs_oracle_and_cuda_core_kernel(pkg, cuda, ora
         check_not_degenerate(fast[-1], "tcgen05 kernel")
 
 
+@pytest.mark.parametrize("q8", [False, True])
+@pytest.mark.parametrize("T,H,cnts,stride", [
+    (1, 16, [2052], 2052),               # one sequence
+    (2, 64, [2052, 2049], 2052),         # head groups in clusters of 16: a third tile of one row
+    (3, 32, [0, 1, 300], 2052),          # nothing attended; CTAs of a cluster without a row
+    (4, 64, [2052, 17, 1025, 0], 2052),  # clusters of 8
+    (16, 64, [2052 - 100 * i for i in range(16)], 2052),  # clusters of 4
+    (32, 64, [65 * i for i in range(32)], 2052),          # 64 query columns in a cluster: two rounds of the exchange
+    (33, 48, [63 + i for i in range(33)], 130),           # 48 columns, clusters of 4 with less than a tile each
+    (60, 64, [900 + i for i in range(60)], 960),          # clusters of 2
+])
+def test_gs_mla_attn_list_cuts(pkg, cuda, oracle, q8, T, H, cnts, stride):
+    """One call per way of dealing (token, head group) lists to CTAs and clusters, single split: no part buffer at all."""
+    torch = cuda
+    rng = np.random.default_rng(T * 100 + H)
+    ctx = 4000
+    q = rng.standard_normal((T, H, 512), dtype=np.float32)
+    Cc = (rng.standard_normal((ctx, 512), dtype=np.float32) * np.float32(0.5)).astype(np.float16)
+    sel = rng.integers(0, ctx, size=(T, stride)).astype(np.int32)
+    cnt = np.array(cnts, np.int32)
+    cq, cs = oracle.quant_q8_rows(Cc.astype(np.float32)) if q8 else (Cc, None)
+    qd, cd, sd, nd = to_dev(torch, q), to_dev(torch, cq), to_dev(torch, sel), to_dev(torch, cnt)
+    scd = None if cs is None else to_dev(torch, cs)
+    o = torch.full((T, H, 512), 7.0, dtype=torch.float32, device="cuda")
+    L = pkg._lib.load()
+    with _Impl(L, 2):
+        for _ in range(2):  # the second call overlaps the first one's end
+            assert L.gs_mla_attn(qd.data_ptr(), cd.data_ptr(), None if scd is None else scd.data_ptr(), sd.data_ptr(), stride, nd.data_ptr(),
+                                 1 / 16, o.data_ptr(), None, T, H, 512, 1, None) == 0
+    st = C.c_int32(-1)
+    assert L.gs_mla_attn_status(C.byref(st), None) == 0 and st.value == 0
+    want = oracle.mla_attn_ref(q, oracle.dequant_q8(cq, cs) if q8 else Cc, sel, cnt, 1 / 16)
+    check_close(o.cpu().numpy(), want, "gs_mla_attn, list cut")
+
+
 def test_gs_mla_attn_lists_with_scattered_unsorted_and_repeated_rows(pkg, cuda, oracle):
     """Position lists are arbitrary: unsorted, with repeats, not in groups of four, different lengths per token."""
     rng = np.random.default_rng(5)
