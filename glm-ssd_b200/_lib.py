@@ -5,6 +5,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 
 from . import build as _build
 
@@ -38,7 +39,12 @@ class DecodeArgs(C.Structure):
     ]
 
 
-# name -> (restype, argtypes); every symbol include/glmssd_attn.h declares
+# The bytes of a DecodeArgs from its fields in order (native alignment), in one call.
+_decode_struct = struct.Struct("@PPqPPPiifiPPPqiiiiiiiPiP")
+assert _decode_struct.size == C.sizeof(DecodeArgs)
+pack_decode_args = _decode_struct.pack
+
+
 class FusedArgs(C.Structure):
     """gs_mla_fused_args of include/glmssd_attn.h."""
     _fields_ = [("q", vp), ("k_b", vp), ("v_b", vp), ("cache", vp), ("cache_rows", i64), ("seq_len", vp), ("scale", f32),
@@ -46,6 +52,7 @@ class FusedArgs(C.Structure):
                 ("d_out", i32)]
 
 
+# name -> (restype, argtypes); every symbol include/glmssd_attn.h declares
 SIGNATURES = {
     "gs_mla_attn": (i32, [vp, vp, vp, vp, i32, vp, f32, vp, vp, i32, i32, i32, i32, vp]),
     "gs_f32_to_f16": (i32, [vp, vp, i64, vp]),
@@ -108,6 +115,19 @@ def load() -> C.CDLL:
         fn.argtypes = args
     _lib = L
     return L
+
+
+_packed = {}
+
+
+def load_packed(name: str):
+    """The entry point taking its argument struct as packed bytes."""
+    fn = _packed.get(name)
+    if fn is None:
+        fn = load()[name]  # a function object of its own, beside the one with the declared signature
+        fn.restype, fn.argtypes = i32, [C.c_char_p, vp]
+        _packed[name] = fn
+    return fn
 
 
 class GsError(RuntimeError):

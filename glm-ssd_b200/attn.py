@@ -18,7 +18,16 @@ from . import _lib
 SCALE_256 = 1.0 / math.sqrt(256.0)  # 1/sqrt(mla_head_k), forward.rs:904
 
 
+# A decode step is about ten microseconds of device time, so what a call costs on the host shows (measured per call:
+# torch.cuda.current_stream() 3.2 us, the raw handle 0.1; twenty attribute assignments of an argument struct 1.5 us, packing
+# them 0.7).
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_raw_device = getattr(torch._C, "_cuda_getDevice", None)
+
+
 def _stream() -> int:
+    if _raw_stream is not None and _raw_device is not None and torch.cuda.is_initialized():
+        return _raw_stream(_raw_device())
     return torch.cuda.current_stream().cuda_stream
 
 
@@ -40,9 +49,10 @@ def _need(t: torch.Tensor, dtype, name: str) -> torch.Tensor:
 
 def mla_attn(q, C_latent, C_scales, sel, sel_stride, cnt, scale, o, part, T, H, R, splits):
     """``gs_mla_attn`` with the reference's argument list (crates/cuda/src/lib.rs:97-100)."""
-    L = _lib.load()
-    _lib.check(L.gs_mla_attn(_ptr(q), _ptr(C_latent), _ptr(C_scales), _ptr(sel), sel_stride, _ptr(cnt), scale,
-                             _ptr(o), _ptr(part), T, H, R, splits, _stream()), "gs_mla_attn")
+    rc = _lib.load().gs_mla_attn(q.data_ptr(), C_latent.data_ptr(), _ptr(C_scales), sel.data_ptr(), sel_stride, cnt.data_ptr(), scale,
+                                 o.data_ptr(), _ptr(part), T, H, R, splits, _stream())
+    if rc:
+        _lib.check(rc, "gs_mla_attn")
 
 
 def mla_attn_impl(impl: int) -> None:
@@ -84,7 +94,6 @@ def mla_decode(q, cache, seq_lens, *, scale=SCALE_256, d_v=512, seq_base=None, p
                ev_after_main=None, no_combine=False, static_scratch=False, exchange=None):
     """Absorbed-MLA decode.  q f16 [n_seq,T,H,d_qk]; cache f16 [rows,d_qk]; seq_lens i32 [n_seq] (device).
     Returns ``out`` (f32 [n_seq,T,H,d_v]) or, with ``want_out=False``, ``part_out``."""
-    L = _lib.load()
     _need(q, torch.float16, "q")
     _need(cache, torch.float16, "cache")
     _need(seq_lens, torch.int32, "seq_lens")
@@ -95,30 +104,24 @@ def mla_decode(q, cache, seq_lens, *, scale=SCALE_256, d_v=512, seq_base=None, p
         workspace = new_workspace(n_seq, T, H, d_v, q.device)
     if want_out and out is None:
         out = torch.empty((n_seq, T, H, d_v), dtype=torch.float32, device=q.device)
-    a = _lib.DecodeArgs()
-    a.q, a.cache, a.cache_rows = q.data_ptr(), cache.data_ptr(), cache.shape[0]
-    a.seq_lens, a.seq_base = seq_lens.data_ptr(), _ptr(seq_base)
-    a.page_table = _ptr(page_table)
-    a.page_table_stride = 0 if page_table is None else page_table.shape[1]
-    a.page_rows = page_rows
-    a.scale = scale
-    a.tail_causal = 1 if tail_causal else 0
-    a.o = _ptr(out) if want_out else None
-    a.part_out = _ptr(part_out)
-    if not static_scratch:
-        a.workspace, a.workspace_bytes = workspace.data_ptr(), workspace.numel()
-    a.n_seq, a.T, a.H, a.d_qk, a.d_v = n_seq, T, H, d_qk, d_v
-    a.max_seq_len = max_seq_len
-    a.impl = impl
-    a.ev_after_main = ev_after_main  # raw cudaEvent_t handle (int) or None
-    a.flags = 1 if no_combine else 0
-    if exchange is not None:  # a _lib.ShardExchange kept alive by the caller (see sharded.PeerExchange)
-        a.exchange = C.pointer(exchange)
+    a = _lib.pack_decode_args(
+        q.data_ptr(), cache.data_ptr(), cache.shape[0], seq_lens.data_ptr(), 0 if seq_base is None else seq_base.data_ptr(),
+        0 if page_table is None else page_table.data_ptr(), 0 if page_table is None else page_table.shape[1], page_rows, scale,
+        1 if tail_causal else 0, out.data_ptr() if want_out else 0, 0 if part_out is None else part_out.data_ptr(),
+        0 if static_scratch else workspace.data_ptr(), 0 if static_scratch else workspace.numel(),
+        n_seq, T, H, d_qk, d_v, max_seq_len, impl,
+        ev_after_main or 0,  # raw cudaEvent_t handle (int) or None
+        1 if no_combine else 0,
+        0 if exchange is None else C.addressof(exchange))  # a _lib.ShardExchange kept alive by the caller (see sharded.PeerExchange)
     if static_scratch:
         # the library's built-in scratch array instead of a workspace: nothing is allocated for the call
-        _lib.check(L.gs_mla_decode_static(C.byref(a), _stream()), "gs_mla_decode_static")
+        rc = _lib.load_packed("gs_mla_decode_static")(a, _stream())
+        if rc:
+            _lib.check(rc, "gs_mla_decode_static")
     else:
-        _lib.check(L.gs_mla_decode(C.byref(a), _stream()), "gs_mla_decode")
+        rc = _lib.load_packed("gs_mla_decode")(a, _stream())
+        if rc:
+            _lib.check(rc, "gs_mla_decode")
     return out if want_out else part_out
 
 
@@ -194,10 +197,11 @@ def rope_kv_append(kv, cache, pos0, *, seq_base=None, page_table=None, page_rows
     _need(cache, torch.float16, "cache")
     _need(pos0, torch.int32, "pos0")
     n_seq, T, d_row = kv.shape
-    _lib.check(_lib.load().gs_rope_kv_append(kv.data_ptr(), cache.data_ptr(), pos0.data_ptr(), _ptr(seq_base),
-                                             _ptr(page_table), 0 if page_table is None else page_table.shape[1],
-                                             page_rows, n_seq, T, d_row, d_rope, rope_base, _stream()),
-               "gs_rope_kv_append")
+    rc = _lib.load().gs_rope_kv_append(kv.data_ptr(), cache.data_ptr(), pos0.data_ptr(), _ptr(seq_base), _ptr(page_table),
+                                       0 if page_table is None else page_table.shape[1], page_rows, n_seq, T, d_row, d_rope,
+                                       rope_base, _stream())
+    if rc:
+        _lib.check(rc, "gs_rope_kv_append")
 
 
 def rope_f16_inplace(x, *, d_rope=64, pos0=0, rope_base=10000.0):
