@@ -63,11 +63,21 @@ constexpr int PF_THREADS = 288;
 constexpr int S_COLS = 64, O_COL = 256;
 constexpr float PF_RESCALE = 8.0f;
 
+// Split form: the keys of one (query block, head) item dealt to the CTAs of a cluster.  When they are done, the accumulators
+// are exchanged over the memory of Q and the K / V stages, 128 columns at a time: the own ones on their way out, and two
+// buffers to receive in; rows are padded by 16 bytes so that a warp's 16-byte accesses (a row per lane) hit all banks.
+constexpr int PX_PITCH = 128 * 4 + 16;
+constexpr int PX_BYTES = BM * PX_PITCH;
+constexpr int PF_MAX_CLUSTER = 16;
+
 struct PrefillParams {
     CUtensorMap tm_q, tm_k, tm_v;
     void *o;
     int o_f16;
     int S, H, p0;
+    int n_blocks;      // 128-query blocks of the chunk
+    int item0;         // first (head, block) item of this launch; items are counted head by head, heavier (later) blocks first
+    int cluster;       // split form: CTAs per item
     float scale_log2;
     int32_t *status;  // may be nullptr
 };
@@ -77,7 +87,7 @@ struct PrefillParams {
 __device__ long long g_pf_prof[32 * 8];
 #define PF_STAMP(j, slot)                                                                                  \
     do {                                                                                                   \
-        if (blockIdx.x == 0 && blockIdx.y == 0 && (j) >= 8 && (j) < 40) g_pf_prof[((j) - 8) * 8 + (slot)] = clock64(); \
+        if (blockIdx.x == 0 && (j) >= 8 && (j) < 40) g_pf_prof[((j) - 8) * 8 + (slot)] = clock64(); \
     } while (0)
 #else
 #define PF_STAMP(j, slot) do { } while (0)
@@ -89,6 +99,7 @@ struct PfBarriers {
     // would test for the phase after one that has not completed - which reads as complete.
     uint64_t q_full, k_full[2 * K_STAGES], k_empty[K_STAGES], v_full[V_STAGES], v_empty[V_STAGES];
     uint64_t s_full[S_BUFS], p_full[S_BUFS], p_free[S_BUFS];  // p_free[b]: P.V has read the probabilities in buffer b
+    uint64_t x_ready, x_data;  // split form: every CTA takes this round's copies; everything sent to this CTA has arrived
 };
 
 struct PfSmemMisc {
@@ -96,8 +107,15 @@ struct PfSmemMisc {
     uint32_t tmem_base;
     int abort_flag;
 };
+struct PfExchange {              // split form, behind the accumulators
+    float2 x_mine[BM];           // (m in log2 units, l) of this CTA's rows, on their way out
+    float2 x_ml[BM];             // [source][row of this CTA's 128 / cluster]
+    float x_w[BM];               // weight of every source in the normalised sum, same index
+};
+static_assert(PX_BYTES % 16 == 0 && 3 * PX_BYTES + (int) sizeof(PfExchange) <= Q_BYTES + (K_STAGES + V_STAGES) * KV_BYTES, "the exchange lies over Q and the stages");
 constexpr int PF_SMEM = Q_BYTES + (K_STAGES + V_STAGES) * KV_BYTES + (int) sizeof(PfSmemMisc) + 1024;
 
+template <bool SPLIT>
 __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_constant__ PrefillParams P) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t) 1023);
@@ -106,11 +124,14 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
     PfBarriers &B = M.bar;
     volatile int *abort_flag = &M.abort_flag;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // heavier (later) query blocks first
-    const int qb = gridDim.x - 1 - blockIdx.x, h = blockIdx.y;
+    const int share = SPLIT ? P.cluster : 1, rank = SPLIT ? (int) blockIdx.x % share : 0;
+    const int item = P.item0 + (SPLIT ? (int) blockIdx.x / share : (int) blockIdx.x);
+    const int h = item / P.n_blocks, qb = P.n_blocks - 1 - item % P.n_blocks;
     const int q0 = qb * BM;
     const int k_end = min(P.p0 + P.S, P.p0 + q0 + BM);  // keys any row of this block attends
-    const int n_tiles = (k_end + BN - 1) / BN;
+    const int all_tiles = (k_end + BN - 1) / BN;
+    const int t0 = SPLIT ? (int) ((int64_t) all_tiles * rank / share) : 0;                       // this CTA's key tiles
+    const int n_tiles = (SPLIT ? (int) ((int64_t) all_tiles * (rank + 1) / share) : all_tiles) - t0;
     const int col0 = h * HD;
 
     if (tid == 0) {
@@ -129,6 +150,10 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
             mbar_init(&B.p_full[i], 4);
             mbar_init(&B.p_free[i], 1);
         }
+        if (SPLIT) {
+            mbar_init(&B.x_ready, share);
+            mbar_init(&B.x_data, 1);
+        }
         M.abort_flag = 0;
         fence_barrier_init();
     }
@@ -140,12 +165,15 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = M.tmem_base;
-    griddep_wait();  // q, k and v may come from the kernel in front (RoPE)
+    if (SPLIT) cluster_sync();  // every CTA's barriers are initialised before another CTA arrives on them
+    // q, k and v may come from the kernel in front (RoPE).  A launch behind the whole items of the same call (item0 > 0) was
+    // started after all of those had passed this wait, so its inputs are final; it waits for that launch itself before it ends.
+    if (!SPLIT || P.item0 == 0) griddep_wait();
     griddep_launch_dependents();
 
     if (warp == 0) {
         // ---- Q once, then the K tiles -------------------------------------------------------------------
-        if (elect_one()) {
+        if (n_tiles > 0 && elect_one()) {
             mbar_arrive_expect_tx(&B.q_full, Q_BYTES);
 #pragma unroll
             for (int b = 0; b < NDB; b++) tma_load_2d(q_smem + b * QBLK, &P.tm_q, &B.q_full, col0 + b * 64, q0);
@@ -159,7 +187,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
                 mbar_arrive_expect_tx(full, KV_BYTES);
 #pragma unroll
                 for (int b = 0; b < NDB; b++)
-                    tma_load_2d(k_smem + st * KV_BYTES + b * KBLK, &P.tm_k, full, col0 + b * 64, j * BN);
+                    tma_load_2d(k_smem + st * KV_BYTES + b * KBLK, &P.tm_k, full, col0 + b * 64, (t0 + j) * BN);
             }
             __syncwarp();
         }
@@ -172,7 +200,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
                 mbar_arrive_expect_tx(&B.v_full[st], KV_BYTES);
 #pragma unroll
                 for (int b = 0; b < NDB; b++)
-                    tma_load_2d(v_smem + st * KV_BYTES + b * KBLK, &P.tm_v, &B.v_full[st], col0 + b * 64, j * BN);
+                    tma_load_2d(v_smem + st * KV_BYTES + b * KBLK, &P.tm_v, &B.v_full[st], col0 + b * 64, (t0 + j) * BN);
             }
             __syncwarp();
         }
@@ -182,8 +210,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
         // 4 P.V MMAs: three issuing warps keep the pipe's queue filled.
         constexpr uint32_t idesc_s = make_idesc_f16(BM, BN, 0, 0);
         const uint64_t d_kmaj = make_smem_desc(0, 16, 1024, kSwizzle128B);
-        const uint32_t q_lo = smem_u32(q_smem) >> 4, k_lo = smem_u32(k_smem) >> 4;
-        bool ok = mbar_wait(&B.q_full, 0, abort_flag, P.status, 2);
+        const uint32_t q_lo = smem_desc_addr(q_smem), k_lo = smem_desc_addr(k_smem);
+        bool ok = n_tiles == 0 || mbar_wait(&B.q_full, 0, abort_flag, P.status, 2);
         // Scores run up to three tiles ahead of the softmax: S(j) goes into tensor-memory buffer j & 3, where
         // P(j-4) lives until P.V(j-4) has read it.  Two MMAs are only ordered with respect to each other on the
         // same accumulator, so that P.V is awaited explicitly.
@@ -210,7 +238,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
         // ---- P.V MMA issuer: O += P . V ----------------------------------------------------------------------------
         constexpr uint32_t idesc_pv = make_idesc_f16(BM, HD, 0, 1);  // A = P from tensor memory, B = V MN-major
         const uint64_t d_v = make_smem_desc(0, KBLK, 1024, kSwizzle128B);
-        const uint32_t v_lo = smem_u32(v_smem) >> 4;
+        const uint32_t v_lo = smem_desc_addr(v_smem);
         bool ok = true;
         for (int j = 0; ok && j < n_tiles; j++) {
             const int sb = j & (S_BUFS - 1);
@@ -246,7 +274,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
                 if (!ok) break;
                 tc_fence_after();
                 if (warp == 2 && lane == 0) PF_STAMP(j, 3);
-                const int k0 = j * BN;
+                const int k0 = (t0 + j) * BN;
                 const bool need_mask = k0 + BN - 1 > P.p0 + q0;  // some row of the block must not see some key
                 // the whole score row of this thread (128 keys) is read once and kept in registers: one
                 // tensor-memory round trip per tile instead of eight
@@ -298,7 +326,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
                 }
                 // probabilities, row sum, P as packed f16 pairs (keys 2i, 2i+1 -> column i of this S buffer)
                 if (warp == 2 && lane == 0) PF_STAMP(j, 5);
-                const float nm = -m_run;
+                const float nm = SPLIT && m_run == -INFINITY ? 0.f : -m_run;  // (split: a row may attend none of this CTA's keys)
                 float l4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int i = 0; i < BN / 2; i++) {
@@ -321,8 +349,96 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
             // ---- epilogue: O / l -> global ------------------------------------------------------------------------
             // The P.V MMAs come from one thread and share one accumulator, so they complete in order: the last one
             // done means all done.  Its barrier's previous phase, P.V(n-5), was over before S(n-1) was issued.
-            if (ok) ok = mbar_wait(&B.p_free[(n_tiles - 1) & (S_BUFS - 1)], ((n_tiles - 1) / S_BUFS) & 1, abort_flag, P.status, 4);
-            if (ok) {
+            if (ok && n_tiles > 0) ok = mbar_wait(&B.p_free[(n_tiles - 1) & (S_BUFS - 1)], ((n_tiles - 1) / S_BUFS) & 1, abort_flag, P.status, 4);
+            if (SPLIT) {
+                // Every CTA of the cluster sends each other one that one's 128 / cluster rows of its accumulators, in two
+                // rounds of 128 columns, and their (m, l); the owner adds the parts up, each weighted by 2^(m - M) / L, and
+                // stores them.  (The bulk copies move about 27 GB/s per SM: 128 KB, 5 us.)
+                const int rows = BM / share, st = tid - 64;  // st: thread of the four softmax warps, which also names a row
+                uint8_t *const x_out = smem;
+                PfExchange &X = *reinterpret_cast<PfExchange *>(smem + 3 * PX_BYTES);
+                X.x_mine[row] = make_float2(m_run, l_run);
+                auto ready = [&](bool first) {  // "this CTA takes the copies of the round and has everything of the round before"
+                    if (st == 0) mbar_arrive_expect_tx(&B.x_data, (uint32_t) (PX_BYTES + (first ? BM * 8 : 0)));
+                    __syncwarp();
+                    if (st >= 0 && st < share) mbar_arrive_cluster(mapa(smem_u32(&B.x_ready), st));
+                };
+                if (group_any(1, 128, !ok || *abort_flag)) ok = false;  // (also: every warp is done with Q, K, V and the accumulator)
+                tc_fence_after();
+                if (ok) ready(true);
+#pragma unroll 1
+                for (int half = 0; ok && half < 2; half++) {
+                    uint8_t *const x_in = smem + (1 + half) * PX_BYTES;
+                    if (half == 1) ok = mbar_wait_cluster(&B.x_ready, 1, abort_flag, P.status, 4);
+                    uint8_t *const mine = x_out + row * PX_PITCH;
+#pragma unroll 1
+                    for (int c = 0; c < 8; c++) {
+                        uint32_t r[16];
+                        if (n_tiles > 0) {
+                            tmem_ld16(tmem + lane_base + O_COL + half * 128 + c * 16, r);
+                            tmem_wait_ld();
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 16; i++) r[i] = 0;
+                        }
+#pragma unroll
+                        for (int i = 0; i < 4; i++) *reinterpret_cast<uint4 *>(mine + c * 64 + i * 16) = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+                    }
+                    fence_proxy_async_smem();
+                    named_bar_sync(2, 128);
+                    bool xok = ok;
+                    if (st < share) {  // thread i: what CTA i of the cluster gets
+                        if (half == 0) xok = mbar_wait_cluster(&B.x_ready, 0, abort_flag, P.status, 4);
+                        if (xok) {
+                            const uint32_t bar = mapa(smem_u32(&B.x_data), st);
+                            bulk_copy_cluster(mapa(smem_u32(x_in + rank * rows * PX_PITCH), st), x_out + st * rows * PX_PITCH, (uint32_t) (rows * PX_PITCH), bar);
+                            if (half == 0) bulk_copy_cluster(mapa(smem_u32(&X.x_ml[rank * rows]), st), &X.x_mine[st * rows], (uint32_t) (rows * 8), bar);
+                        }
+                    }
+                    xok = xok && mbar_wait_cluster(&B.x_data, half, abort_flag, P.status, 4);
+                    if (group_any(1, 128, !xok || *abort_flag)) ok = false;  // (one decision for the four warps)
+                    if (!ok) break;
+                    if (half == 0) {
+                        ready(false);
+                        if (st < rows) {
+                            float mx = -INFINITY, l = 0.f;
+                            for (int r = 0; r < share; r++) mx = fmaxf(mx, X.x_ml[r * rows + st].x);
+                            for (int r = 0; r < share; r++) {
+                                const float2 v = X.x_ml[r * rows + st];
+                                l = fmaf(v.y, v.x == -INFINITY ? 0.f : exp2f(v.x - mx), l);
+                            }
+                            for (int r = 0; r < share; r++) {
+                                const float2 v = X.x_ml[r * rows + st];
+                                X.x_w[r * rows + st] = v.x == -INFINITY || !(l > 0.f) ? 0.f : exp2f(v.x - mx) / l;
+                            }
+                        }
+                        named_bar_sync(2, 128);
+                    }
+                    for (int i = st; i < rows * 32; i += 128) {
+                        const int rr = i >> 5, c4 = i & 31, qr = q0 + rank * rows + rr;
+                        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+                        for (int r = 0; r < share; r++) {
+                            const float w = X.x_w[r * rows + rr];
+                            const float4 u = *reinterpret_cast<const float4 *>(x_in + (r * rows + rr) * PX_PITCH + c4 * 16);
+                            a.x = fmaf(u.x, w, a.x);
+                            a.y = fmaf(u.y, w, a.y);
+                            a.z = fmaf(u.z, w, a.z);
+                            a.w = fmaf(u.w, w, a.w);
+                        }
+                        if (qr < P.S) {
+                            const int64_t off = ((int64_t) qr * P.H + h) * HD + half * 128 + c4 * 4;
+                            if (P.o_f16) {
+                                const __half2 lo = __floats2half2_rn(a.x, a.y), hi = __floats2half2_rn(a.z, a.w);
+                                *reinterpret_cast<uint2 *>(reinterpret_cast<__half *>(P.o) + off) =
+                                    make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+                            } else {
+                                *reinterpret_cast<float4 *>(reinterpret_cast<float *>(P.o) + off) = a;
+                            }
+                        }
+                    }
+                }
+            } else if (ok) {
                 tc_fence_after();
                 const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
                 const int64_t off = ((int64_t) qi * P.H + h) * HD;
@@ -357,6 +473,10 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
     // ---- common exit ---------------------------------------------------------------------------------------------
     tc_fence_before();
     __syncthreads();
+    if (SPLIT) {
+        cluster_sync();  // no CTA leaves while another may still write to its shared memory or read from it
+        if (P.item0 > 0) griddep_wait();  // what follows this launch in the stream also follows the launch in front of it
+    }
     if (*abort_flag && tid == 0) {
         const long long t0 = clock64();
         while (clock64() - t0 < 2000000LL) {
@@ -370,6 +490,73 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
 }
 
 }  // namespace
+
+// How the (head, query block) items of a call are run: the first `whole` of them one per CTA, the rest in clusters.
+struct PrefillPlan {
+    int whole, cluster;
+};
+// A CTA takes an item from its first key tile to its last, and with one CTA per SM the items run in rounds of 148: a chunk
+// of 1000 tokens behind 7168 (160 items of 113 to 128 tiles) left 136 SMs idle for half its time, one of 128 tokens 128 of
+// them for all of it.  So when the items do not fill whole rounds, the last ones are split.  Estimated in key tiles (0.65 us);
+// a split item costs 18 tiles and more besides its share (its own start, the exchange and the sum; measured 11 us from 2 to 4
+// CTAs, 15 with 8, over 20 with 16).  Measured, whole / chosen: 1000 tokens behind 7168 188 / 135 us, 32 behind 4096 51 / 32 us,
+// 128 behind 32000 352 / 130 us (5 TB/s of keys and values), 900 behind 20000 482 / 332 us.
+constexpr int split_cost(int c) { return c <= 4 ? 18 : c == 8 ? 24 : 34; }
+static PrefillPlan prefill_plan(int S, int H, int p0) {
+    constexpr int SMS = 148;
+    const int nb = (S + BM - 1) / BM;
+    const int64_t items = (int64_t) nb * H;
+    // From five rounds on the last round is at most a few per cent.
+    if (items > 5 * SMS) return PrefillPlan{(int) items, 1};
+    auto tiles_of = [&](int64_t i) {
+        const int qb = nb - 1 - (int) (i % nb);
+        const int end = p0 + (S < (qb + 1) * BM ? S : (qb + 1) * BM);
+        return (end + BN - 1) / BN;
+    };
+    // when the SM that is free first has finished, items handed out in order: a heap of 148 finishing times
+    int busy[SMS] = {0};
+    auto give = [&](int t) {
+        int i = 0;
+        const int v = busy[0] + t;
+        for (;;) {
+            int c = 2 * i + 1;
+            if (c >= SMS) break;
+            if (c + 1 < SMS && busy[c + 1] < busy[c]) c++;
+            if (busy[c] >= v) break;
+            busy[i] = busy[c];
+            i = c;
+        }
+        busy[i] = v;
+    };
+    auto latest = [&]() {
+        int m = 0;
+        for (int i = 0; i < SMS; i++) m = busy[i] > m ? busy[i] : m;
+        return m;
+    };
+    PrefillPlan best{(int) items, 1};
+    const int64_t rounds = items / SMS;
+    int64_t at = 0;
+    for (; at < rounds * SMS; at++) give(tiles_of(at));
+    const int done = latest();          // the full rounds
+    int most = 0;
+    for (int64_t i = at; i < items; i++) {
+        const int t = tiles_of(i);
+        most = t > most ? t : most;
+        give(t);
+    }
+    int cost = latest();
+    const int64_t rest = items - at;
+    for (int c = 2; rest > 0 && c <= PF_MAX_CLUSTER; c *= 2) {
+        const int resident = c == 2 ? 74 : c == 4 ? 33 : c == 8 ? 15 : 7;  // clusters that run at once, one CTA per SM
+        const int64_t turns = (rest + resident - 1) / resident;
+        const int64_t t = done + turns * ((most + c - 1) / c + split_cost(c));
+        if (t < cost) {
+            cost = (int) t;
+            best = PrefillPlan{(int) at, c};
+        }
+    }
+    return best;
+}
 
 bool prefill_umma_supported(int S, int H, int d, int p0, const char **why) {
     if (d != HD) { *why = "head width other than 256"; return false; }
@@ -398,9 +585,33 @@ int launch_prefill_umma(const __half *q, const __half *k, const __half *v, void 
     P.p0 = p0;
     P.scale_log2 = scale * 1.4426950408889634f;
     P.status = status;  // may be nullptr: a wait that gives up is then not reported
-    GS_TRY(cudaFuncSetAttribute(k_prefill_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
-    dim3 grid((S + BM - 1) / BM, H);
-    return launch_pdl(k_prefill_umma, grid, PF_THREADS, PF_SMEM, st, P);
+    P.n_blocks = (S + BM - 1) / BM;
+    const PrefillPlan plan = prefill_plan(S, H, p0);
+    if (plan.whole > 0) {
+        GS_TRY(cudaFuncSetAttribute(k_prefill_umma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
+        if (int e = launch_pdl(k_prefill_umma<false>, dim3(plan.whole), PF_THREADS, PF_SMEM, st, P)) return e;
+    }
+    const int64_t items = (int64_t) P.n_blocks * H;
+    if (plan.whole == items) return 0;
+    P.item0 = plan.whole;
+    P.cluster = plan.cluster;
+    GS_TRY(cudaFuncSetAttribute(k_prefill_umma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
+    if (plan.cluster > 8) GS_TRY(cudaFuncSetAttribute(k_prefill_umma<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned) ((items - plan.whole) * plan.cluster));
+    cfg.blockDim = dim3(PF_THREADS);
+    cfg.dynamicSmemBytes = PF_SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = plan.cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    GS_TRY(cudaLaunchKernelEx(&cfg, k_prefill_umma<true>, P));
+    return 0;
 }
 
 }  // namespace gs

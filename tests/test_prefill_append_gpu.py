@@ -26,6 +26,32 @@ def test_prefill_vs_oracle(pkg, cuda, oracle, impl, S, H, p0):
         check_not_degenerate(got.cpu().numpy())
 
 
+@pytest.mark.parametrize("S,H,p0,f16", [
+    (32, 4, 3000, False),    # four items in clusters of 16
+    (64, 10, 2000, True),    # clusters of 8, fewer rows than a block
+    (200, 9, 2500, False),   # clusters of 4; a ragged second block whose last tiles only some rows attend
+    (129, 30, 1960, True),   # clusters of 2; one row in the second block
+    (640, 30, 2100, False),  # 150 items: 148 whole, two split
+])
+def test_prefill_split_items_vs_oracle(pkg, cuda, oracle, S, H, p0, f16):
+    """Items dealt over clusters along the keys; the row subset keeps the oracle short."""
+    Q, K, V = _qkv(S + H, S, H, 256, p0)
+    Qd, Kd, Vd = to_dev(cuda, Q), to_dev(cuda, K), to_dev(cuda, V)
+    status = cuda.zeros(1, dtype=cuda.int32, device="cuda")
+    o = cuda.empty((S, H, 256), dtype=cuda.float16 if f16 else cuda.float32, device="cuda")
+    for _ in range(3):  # launches that overlap
+        assert pkg._lib.load().gs_prefill_attn_checked(Qd.data_ptr(), Kd.data_ptr(), Vd.data_ptr(), o.data_ptr(), int(f16), S, H, 256, p0,
+                                                       1 / 16, 0, status.data_ptr(), None) == 0
+    cuda.cuda.synchronize()
+    assert int(status) == 0
+    rows = np.unique(np.concatenate([np.arange(min(S, 8)), np.arange(max(0, S - 8), S), np.arange(120, min(S, 136))])).astype(np.int32)
+    want = oracle.prefill(Q, K, V, 1 / 16, p0=p0, rows=rows)
+    check_close(o.float().cpu().numpy()[rows], want, "split prefill", *((3e-3, 4e-4) if f16 else ()))
+    whole = pkg.prefill_attn(Qd, Kd, Vd, p0=p0, impl=1)  # every row against the CUDA-core kernel
+    cuda.cuda.synchronize()
+    check_close(o.float().cpu().numpy(), whole.cpu().numpy(), "split prefill, all rows", *((3e-3, 4e-4) if f16 else ()))
+
+
 def test_config4_prefill_8192_with_rope(pkg, cuda, oracle):
     # 8192-token chunk, 20 heads, d = 256 (192 nope + 64 rope), RoPE base 10000 on the last 64 dims
     S, H, d = 8192, 20, 256
