@@ -110,7 +110,7 @@ __device__ __forceinline__ SegRange combine_locate(const CombinePlan &C, int row
     const int after = (int) min(before64 + mine, (long long) kUnitCap);  // saturated running sums, as the kernel holds them
     const int before = (int) min(before64, (long long) kUnitCap);
     const int total = (int) min(total64, (long long) kUnitCap);
-    const int chunk = max(1, (total + C.n_ctas - 1) / C.n_ctas);
+    const int chunk = decode_chunk(total, C.n_ctas, C.n_seq == 1, C.unit_rows);
     r.first = b;
     r.nseg = 0;
     if (after > before) {
@@ -238,9 +238,8 @@ __device__ __forceinline__ bool combine_item_compute(const CombinePlan &C, const
 
 // The records of the tcgen05 kernel ([segment][row][d_v]) fetched by ONE tiled 3-D TMA copy: what an item (output row,
 // 128 columns) needs is one 512-byte piece per segment, a whole record apart from the next - a box
-// {128, 1, box} of the tensor {d_v, rows, segments}.  With one sequence the box spans n_ctas segments (a sequence has at
-// most one per CTA); with several a row has about n_ctas / n_seq + 1, a number only the device knows, and as many boxes of
-// 16 as it needs are fetched.  Segments past the sequence's last one belong to other sequences or lie outside the tensor
+// {128, 1, box} of the tensor {d_v, rows, segments}.  How many segments a row has only the device knows (at most n_ctas with
+// one sequence, about n_ctas / n_seq + 1 with several): as many boxes as it needs are fetched.  Segments past the sequence's last one belong to other sequences or lie outside the tensor
 // (zero-filled) and get weight 0.
 constexpr int32_t ST_COMBINE = 1 << 18;  // status bit: the copy of the records did not complete in time
 struct CombineBulk {

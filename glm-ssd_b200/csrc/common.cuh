@@ -55,6 +55,26 @@ inline int64_t decode_segments_bound(int n_seq, int T) {
     return umma > simt ? umma : simt;
 }
 
+// Units (of unit_rows rows) one CTA of the tcgen05 decode kernel takes; the combine kernel recomputes the schedule with it.
+// Several sequences: an equal share.  One sequence: whole 64-row tiles, since the last tile of a CTA costs what a full one
+// does - 32768 rows are 128 runs of 4 tiles (18.5 us with two query tokens), not 147 of 3.5 (18.9 us) - and a record less to
+// write and to merge for every CTA left out; for the same reason from 75 tiles on at least two tiles, which the two stages hold
+// at once anyway (4096 rows: 64 runs 9.4 us, 128 half tiles 10.9 us; 8192 rows: 64 runs of two 10.2 us, 128 of one 11.1 us).
+__host__ __device__ inline int decode_chunk(int total_units, int n_ctas, bool one_sequence, int unit_rows) {
+    const int even = (total_units + n_ctas - 1) / n_ctas;
+    if (!one_sequence) return even > 1 ? even : 1;
+    const int shift = unit_rows == 16 ? 2 : 0, tiles = (total_units + (1 << shift) - 1) >> shift;
+    int t = (tiles + n_ctas - 1) / n_ctas;
+    if (t < 2) t = tiles > 74 ? 2 : 1;
+    return t << shift;
+}
+// CTAs that rule can use for any length up to max_rows (148 from 296 tiles on): no more need to be launched.
+inline int decode_grid(int64_t max_rows, int sm_count) {
+    const int64_t tiles = (max_rows + 63) / 64;
+    const int64_t n = tiles <= 74 ? tiles : tiles <= 148 ? 74 : (tiles + 1) / 2;
+    return (int) (n < 1 ? 1 : n < sm_count ? n : sm_count);
+}
+
 // Row addressing shared by the kernels: explicit list, paged or dense.
 struct RowMap {
     const int32_t *list;   // explicit positions (legacy `sel` row) or nullptr

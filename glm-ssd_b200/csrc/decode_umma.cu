@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
             tc_fence_after();
             sc.total = M.cum[P.n_seq];
         }
-        sc.chunk = max(1, (sc.total + (int) gridDim.x - 1) / (int) gridDim.x);
+        sc.chunk = decode_chunk(sc.total, (int) gridDim.x, sc.single, unit_rows);
         sc.start = min(sc.total, (int) blockIdx.x * sc.chunk);
         sc.end = min(sc.total, sc.start + sc.chunk);
         sc.b0 = 0;
@@ -1501,6 +1501,10 @@ int launch_decode_umma(const DecodeProblem &p, cudaStream_t st) {
     P.d_v = p.d_v;
     P.cache_rows = p.cache_rows;
     int grid = p.sm_count < kMaxCtas ? p.sm_count : kMaxCtas;
+    if (n_seq_k == 1) {  // (a length beyond max_seq_len would still be attended, in longer runs)
+        const int64_t most = p.page_table ? (int64_t) p.page_table_stride * TILE : p.cache_rows;
+        grid = decode_grid(p.max_seq_len > 0 && p.max_seq_len < most ? p.max_seq_len : most, grid);
+    }
     if (p.max_ctas > 0 && grid > p.max_ctas) grid = p.max_ctas;
     if (grid < 1) grid = 1;
     // every CTA and every sequence can add one segment, each with the query rows of one launch

@@ -197,3 +197,17 @@ def test_length_beyond_the_cache_is_taken_as_the_cache_size(pkg, cuda, oracle, T
     want = oracle.mla_decode(q, cache, np.array([1500, 0, 400], np.int32), 1 / 16, seq_base=base)
     check_close(got, want, "clamped lengths")
     assert (got[1] == 0).all()
+
+
+@pytest.mark.parametrize("T", [1, 2])
+@pytest.mark.parametrize("n", [74 * 64, 74 * 64 + 1, 75 * 64, 148 * 64, 148 * 64 + 1, 149 * 64 + 15, 296 * 64, 297 * 64 + 63])
+def test_one_sequence_runs_of_whole_tiles(pkg, cuda, oracle, T, n):
+    """Lengths around which the run of tiles per CTA, or the number of CTAs launched, changes; the bound exact, loose and unset."""
+    q, cache = make_decode_inputs(n, 1, T, 20, n + 5)
+    cache[n:] = np.float16(np.nan)
+    want = oracle.mla_decode(q, cache, [n], 1 / 16)
+    qd, cd, ld = to_dev(cuda, q), to_dev(cuda, cache), to_dev(cuda, np.array([n], np.int32))
+    for bound in (n, n + 5, 0, 64):  # (a length beyond the bound is attended all the same)
+        got = pkg.mla_decode(qd, cd, ld, max_seq_len=bound)
+        cuda.cuda.synchronize()
+        check_close(got.cpu().numpy(), want, f"n={n} T={T} bound={bound}")
