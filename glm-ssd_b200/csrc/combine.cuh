@@ -280,26 +280,43 @@ __device__ __forceinline__ bool combine_item_fetch_tma(const CombinePlan &C, con
     const float ls = warp_sum(ml.y * wgt);
     if (lane == 0) S.lred[warp] = ls;
     a = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s0 = 0, round = 0; round == 0 || s0 < nseg; s0 += cap, round++) {
-        if (round > 0 && tid == 0) fetch(s0);
-        if (nseg > 0 && !sm100::mbar_wait(bar, round & 1, abort_flag, const_cast<int32_t *>(C.status), ST_COMBINE)) *abort_flag = 1;
-        __syncthreads();
-        if (*abort_flag) return false;
-        for (int s = s0 + warp; s < min(nseg, s0 + cap); s += CB_LANES) {
-            const float w = S.m[s];
-            if (w != 0.f) {  // an empty segment's accumulator never enters the sum
-                const float4 u = tile[(s - s0) * (CB_COLS / 4) + lane];
-                a.x = fmaf(u.x, w, a.x);
-                a.y = fmaf(u.y, w, a.y);
-                a.z = fmaf(u.z, w, a.z);
-                a.w = fmaf(u.w, w, a.w);
+    // four segments of this segment lane at a time; an empty segment's accumulator (weight 0) never enters the sum
+    auto add = [&](int s0, int end) {
+        const float4 *src = tile + warp * (CB_COLS / 4) + lane;
+        for (int s = s0 + warp; s < end; s += 4 * CB_LANES, src += 4 * CB_LANES * (CB_COLS / 4)) {
+            float w[4];
+            float4 u[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                w[k] = s + k * CB_LANES < end ? S.m[s + k * CB_LANES] : 0.f;
+                u[k] = s + k * CB_LANES < end ? src[k * CB_LANES * (CB_COLS / 4)] : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (w[k] != 0.f) {
+                    a.x = fmaf(u[k].x, w[k], a.x);
+                    a.y = fmaf(u[k].y, w[k], a.y);
+                    a.z = fmaf(u[k].z, w[k], a.z);
+                    a.w = fmaf(u[k].w, w[k], a.w);
+                }
             }
         }
-        if (s0 + cap < nseg) __syncthreads();  // the tile is filled again
-    }
+    };
+    if (nseg > 0 && !sm100::mbar_wait(bar, 0, abort_flag, const_cast<int32_t *>(C.status), ST_COMBINE)) *abort_flag = 1;
+    __syncthreads();
+    if (*abort_flag) return false;
     L = 0.f;
 #pragma unroll
     for (int w = 0; w < CB_NT / 32; w++) L += S.lred[w];
+    add(0, min(nseg, cap));
+    for (int s0 = cap, round = 1; s0 < nseg; s0 += cap, round++) {  // (several sequences, one with more segments than the tile holds)
+        __syncthreads();
+        if (tid == 0) fetch(s0);
+        if (!sm100::mbar_wait(bar, round & 1, abort_flag, const_cast<int32_t *>(C.status), ST_COMBINE)) *abort_flag = 1;
+        __syncthreads();
+        if (*abort_flag) return false;
+        add(s0, min(nseg, s0 + cap));
+    }
     S.part[warp][lane] = a;
     __syncthreads();
     if (warp == 0) {
