@@ -6,8 +6,9 @@
 // the combine kernel merges (ops.cu:539-574).  How it computes it is specific to sm_100a:
 //
 //  * One persistent CTA per SM.  The 16-row units (64-row pages when paged) of all sequences are
-//    cut into equal contiguous chunks, one per CTA; the part of a sequence inside a chunk is a
-//    "segment" and yields one partial record.  The cache is read from HBM exactly once.
+//    cut into equal contiguous chunks, one per CTA (whole tiles with one sequence, see decode_chunk); the part of a
+//    sequence inside a chunk is a "segment" and yields one partial record.  The cache is read from HBM exactly once.
+//    Position lists may instead be attended by one CTA or one thread-block cluster each (see list_plan).
 //  * A producer warp streams 64-row cache tiles into a two-stage shared-memory ring with TMA
 //    (128-byte swizzle, one 64x64 box per 64-column block); the ragged last tile of a segment is
 //    fetched in 16-row boxes so no row outside the segment is read.
@@ -156,7 +157,7 @@ struct UmmaParams {
     int n_seq, T, H, rows_q, d_v;  // H: heads handled by this launch (a group of the H_full heads of q)
     int H_full, h0;                // q holds H_full heads per token; this launch takes heads h0 .. h0+H-1
     // position-list form (the reference's sel / cnt): kernel sequence b attends rows sel[(b / seq_div) * sel_stride + i],
-    // i < seq_lens[b / seq_div]; the rows are fetched by the producer warp with 16-byte asynchronous copies
+    // i < seq_lens[b / seq_div]; the rows are fetched by four producer warps (16-byte asynchronous copies; Q8 through registers)
     const void *list_cache;        // the cache as a plain pointer (rows of d_qk f16, or of d_qk int8 when list_scales is set)
     const __half *list_scales;     // Q8 cache (crates/cuda/kernels/ops.cu:427): one f16 scale per 32 values, [rows][d_qk / 32]
     const int32_t *sel;

@@ -42,19 +42,19 @@ int gs_mla_attn(const float *q, const void *C, const void *C_scales, const int *
                 float scale, float *o, float *part, int T, int H, int R, int splits, void *stream);
 
 /* Which kernel gs_mla_attn runs (no counterpart in the reference).  The call runs on the tcgen05 decode kernel whenever
- * that kernel takes the shape: the rows a list names are fetched straight from the cache by the kernel's producer warp
- * (f16 rows, or the int8 rows and scales of a Q8 cache, which the kernel widens to half_rn(scale * q) in shared
- * memory), the f32 queries are rounded to f16 inside the kernel (the precision
+ * that kernel takes the shape: the rows a list names are fetched straight from the cache by the kernel's producer warps
+ * (f16 rows, or the int8 rows and scales of a Q8 cache, which they widen to half_rn(scale * q)), the f32 queries are rounded to f16 inside the kernel (the precision
  * of the f16-query entry points; outputs stay within max-abs 2e-3 of the f32-query result), and nothing beyond the
- * reference's own arguments is needed: with splits > 1 the split records live in `part` (as many segments as fit its
- * T*H*splits*(R+2) floats), with splits == 1 every (token, head group) is attended by one CTA that stores o itself.
+ * reference's own arguments is needed: a (token, head group) is attended by one CTA or by a thread-block cluster that
+ * merges inside the chip and stores o, or - with splits > 1, where that is faster - by CTAs whose split records live in
+ * `part` (as many segments as fit its T*H*splits*(R+2) floats).  With splits == 1 `part` is not touched.
  * Head counts that cannot be cut into groups of 8..48 heads and misaligned q / C / C_scales run on the CUDA-core
  * kernel, which keeps the queries in f32.
  *   gs_mla_attn_set_impl(impl): 0 = automatic (default), 1 = always the CUDA-core kernel, 2 = the tcgen05 kernel or
  *     cudaErrorInvalidValue.  A process-wide setting; it changes no result beyond the rounding described above.
  *   gs_mla_attn_status(status_out, stream): synchronises `stream` and reads the sticky status word of the tcgen05
  *     path (the reference's argument list has no workspace that could carry one): 0 = ok, else a bounded wait inside
- *     the kernel gave up and cudaErrorLaunchTimeout is returned. */
+ *     the kernel gave up and cudaErrorLaunchTimeout is returned (bits 8 and up: inside the tcgen05 form of gs_idx_score). */
 int gs_mla_attn_set_impl(int impl);
 int gs_mla_attn_status(int32_t *status_out /* host, may be NULL */, void *stream);
 
