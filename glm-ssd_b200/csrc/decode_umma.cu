@@ -756,7 +756,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                 (void) bar_wait<LIST>(&B.q_empty, (sgc & 1) ^ 1, abort_flag, status_w, ST_SOFTMAX);
                 const float *qsrc = P.q_f32 + ((int64_t) (sg.b / P.seq_div) * P.H_full + (int64_t) (sg.b % P.seq_div) * P.H) * (NBLK * 64);
                 constexpr int CPR = NBLK * 8;  // 16-byte chunks (8 columns) per row
-                constexpr int U = 4;           // chunks per thread requested together
+                constexpr int U = NQ > 48 ? 8 : 4;  // chunks per thread requested together
                 static_assert(!LIST || NQ * CPR % (128 * U) == 0, "whole rounds");
 #pragma unroll 1
                 for (int i0 = wg_tid; i0 < NQ * CPR; i0 += 128 * U) {
