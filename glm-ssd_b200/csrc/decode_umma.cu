@@ -682,13 +682,30 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                     const uint32_t i1 = it + 1;
                     const uint32_t ph1 = (i1 >> 1) & 1;
                     // uniform over the warp: every lane polls the same barriers
-                    bool landed = mbar_test(&B.s_empty[i1 & 1], ph1 ^ 1);
-                    for (int g = g_lo; g <= g_hi; g++) landed = landed && mbar_test(&B.kv_full[i1 & 1][g], ph1);
-                    if (__all_sync(0xffffffffu, landed)) {
+                    auto landed = [&]() {
+                        bool l = mbar_test(&B.s_empty[i1 & 1], ph1 ^ 1);
+                        for (int g = g_lo; g <= g_hi; g++) l = l && mbar_test(&B.kv_full[i1 & 1][g], ph1);
+                        return __all_sync(0xffffffffu, l);
+                    };
+                    s_ahead = landed();
+                    // Where the next load does not wait for this stage (the last two tiles of a segment; long lists, whose
+                    // rows come from L2) go on asking while the softmax is at work: asked only once, a tile that landed a
+                    // little later had its scores behind P.V.  In a stream from HBM the release of the stage comes first.
+                    // (us, once -> this: 256-token chunk of lists 173 -> 159; 32K rows, two tokens, 20.6 -> 20.2; 64 heads
+                    // 21.9 -> 21.1.  Asking on in every tile costs 64K rows, one token, 23.1 -> 23.7; never issuing ahead
+                    // costs 16K rows 12.7 -> 13.6.)
+                    if (!s_ahead && (LIST ? sg.n_tiles > 4 : j + 2 >= sg.n_tiles)) {
+                        for (int spins = 1; !__all_sync(0xffffffffu, mbar_test(&B.p_full[s], ph)); spins++) {
+                            s_ahead = landed();
+                            if (s_ahead) break;
+                            // (bounded: the wait for P below has the limit that reports)
+                            if ((spins & 63) == 0 && __any_sync(0xffffffffu, spins > (1 << 25) || *abort_flag)) break;
+                        }
+                    }
+                    if (s_ahead) {
                         if (mw == 0 && lane == 0) GS_STAMP(i1, PF_KV_FULL);
                         issue_s(i1);
                         if (mw == 0 && lane == 0) GS_STAMP(i1, PF_S_ISSUED);
-                        s_ahead = true;
                     }
                 }
                 // ---- O^T[my tiles] += V^T . P^T ----
