@@ -314,6 +314,12 @@ def test_gs_mla_attn_list_cuts(pkg, cuda, oracle, q8, T, H, cnts, stride):
     check_close(o.cpu().numpy(), want, "gs_mla_attn, list cut")
 
 
+@pytest.mark.parametrize("T,H", [(160, 64), (160, 32)])
+def test_gs_mla_attn_lists_around_four_tiles(pkg, cuda, oracle, T, H):
+    """Lists of four tiles and of one row more or less, two per CTA: the issuing warps ask on for the next tile above four."""
+    test_gs_mla_attn_list_cuts(pkg, cuda, oracle, False, T, H, [(255, 256, 257, 319, 321, 64, 0)[i % 7] for i in range(T)], 336)
+
+
 def test_gs_mla_attn_lists_with_scattered_unsorted_and_repeated_rows(pkg, cuda, oracle):
     """Position lists are arbitrary: unsorted, with repeats, not in groups of four, different lengths per token."""
     rng = np.random.default_rng(5)
