@@ -302,7 +302,7 @@ __device__ __forceinline__ bool combine_item_fetch_tma(const CombinePlan &C, con
             }
         }
     };
-    if (nseg > 0 && !sm100::mbar_wait(bar, 0, abort_flag, const_cast<int32_t *>(C.status), ST_COMBINE)) *abort_flag = 1;
+    if (nseg > 0 && !sm100::mbar_wait_lane(bar, 0, abort_flag, const_cast<int32_t *>(C.status), ST_COMBINE)) *abort_flag = 1;
     __syncthreads();
     if (*abort_flag) return false;
     L = 0.f;
@@ -312,7 +312,7 @@ __device__ __forceinline__ bool combine_item_fetch_tma(const CombinePlan &C, con
     for (int s0 = cap, round = 1; s0 < nseg; s0 += cap, round++) {  // (several sequences, one with more segments than the tile holds)
         __syncthreads();
         if (tid == 0) fetch(s0);
-        if (!sm100::mbar_wait(bar, round & 1, abort_flag, const_cast<int32_t *>(C.status), ST_COMBINE)) *abort_flag = 1;
+        if (!sm100::mbar_wait_lane(bar, round & 1, abort_flag, const_cast<int32_t *>(C.status), ST_COMBINE)) *abort_flag = 1;
         __syncthreads();
         if (*abort_flag) return false;
         add(s0, min(nseg, s0 + cap));

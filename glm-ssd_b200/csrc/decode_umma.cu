@@ -227,7 +227,7 @@ struct Smem {
 // The bounded wait.  A kernel that hands registers over (setmaxnreg) may not call functions: its slow path is inlined.
 template <bool INLINE>
 __device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int32_t *status, int32_t code) {
-    if (!INLINE) return mbar_wait(bar, parity, abort_flag, status, code);
+    if (!INLINE) return mbar_wait_lane(bar, parity, abort_flag, status, code);
     if (mbar_try_wait(bar, parity)) return true;
     const long long t0 = clock64();
     int spins = 0;
@@ -243,7 +243,6 @@ __device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity, volatil
     }
     return true;
 }
-
 struct Segment {
     int b, r0, r1, len, n_tiles, seg_id;
 };
@@ -543,6 +542,9 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
     const int end = sc.end;
     uint32_t it = 0, sgc = 0;  // running tile and segment counters (identical in every role)
     Segment sg;
+    // What a lane votes with: whether one of its waits gave up, or - list form, which has no register to spare for the answers of
+    // its waits (256-token chunk 160 -> 170 us with them) - the flag that such a wait sets.
+    auto gave_up = [&](bool lane_ok) { return LIST ? *abort_flag != 0 : !lane_ok; };
 
     // (The hand-over of registers in the list form: every warpgroup executes one instruction; the softmax group takes over
     // what the others do not need.)
@@ -551,14 +553,13 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
     if (!LIST && warp == 0) {
         // =================================== TMA producer ==================================================
         // The whole warp runs the loop (uniform control flow); one elected lane issues each copy.
-        bool ok = true;
+        bool ok = true, lane_ok = true;  // (of the warp; of this lane's waits)
         const uint64_t pol_stream = l2_policy_evict_first();  // every cache row is read once per step
         while (ok && next_segment(pos, b_cur, end, M.cum, unit_rows, M.len, sg, sc)) {
             const int64_t base_row = sc.single ? sc.base0 : M.base[sg.b];
-            for (int j = 0; j < sg.n_tiles; j++, it++) {
+            for (int j = 0; ok && j < sg.n_tiles; j++, it++) {
                 const int s = it & 1;
-                ok = bar_wait<LIST>(&B.kv_empty[s], ((it >> 1) & 1) ^ 1, abort_flag, status_w, ST_PRODUCER);
-                if (!ok) break;
+                lane_ok &= bar_wait<LIST>(&B.kv_empty[s], ((it >> 1) & 1) ^ 1, abort_flag, status_w, ST_PRODUCER);
                 if (lane == 0) GS_STAMP(it, PF_LOAD_ISSUE);
                 if (lane == 0 && it == 0) GS_CTA_STAMP(7);
                 const int row = sg.r0 + j * TILE;
@@ -597,8 +598,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                     }
                 }
                 if (j == 0) {  // the query rows of this sequence, after the first (larger, farther) cache tile
-                    ok = bar_wait<LIST>(&B.q_empty, (sgc & 1) ^ 1, abort_flag, status_w, ST_PRODUCER);
-                    if (!ok) break;
+                    lane_ok &= bar_wait<LIST>(&B.q_empty, (sgc & 1) ^ 1, abort_flag, status_w, ST_PRODUCER);
                     if (elect_one()) {
                         if (P.H_full == P.H) {  // the sequence's T*H query rows are contiguous: one box per block
                             mbar_arrive_expect_tx(&B.q_full, (uint32_t) (NBLK * NQ * 128));
@@ -616,7 +616,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                         }
                     }
                 }
-                __syncwarp();
+                ok = __all_sync(0xffffffffu, !gave_up(lane_ok));
             }
             sgc++;
         }
@@ -638,10 +638,10 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
         const uint64_t d_vt = make_smem_desc(0, BLK_BYTES, 1024, kSwizzle128B);    // cache tile, MN-major
         const uint64_t d_pt = make_smem_desc(0, 128, 1024, kSwizzleNone);          // P^T, MN-major
         const uint32_t q_lo = smem_desc_addr(q_smem), p_lo0 = smem_desc_addr(p_smem), kv_lo0 = smem_desc_addr(kv_smem);
-        bool ok = true;
+        bool ok = true, lane_ok = true;  // (of the warp; of this lane's waits)
         while (ok && next_segment(pos, b_cur, end, M.cum, unit_rows, M.len, sg, sc)) {
             if (LIST && sg.n_tiles == 0) continue;  // (cluster form: no share of the rows)
-            ok = bar_wait<LIST>(&B.q_full, sgc & 1, abort_flag, status_w, ST_MMA);
+            lane_ok &= bar_wait<LIST>(&B.q_full, sgc & 1, abort_flag, status_w, ST_MMA);
             // S of tile j+1 is issued ahead of P.V of tile j whenever its data has already landed, so it
             // runs on the tensor pipe while the softmax of tile j is computed.
             auto issue_s = [&](uint32_t i) {
@@ -669,9 +669,8 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                 const uint32_t ph = (it >> 1) & 1;
                 const uint32_t kv_lo = kv_lo0 + s * (STAGE_BYTES >> 4);
                 if (!s_ahead) {
-                    ok = bar_wait<LIST>(&B.s_empty[s], ph ^ 1, abort_flag, status_w, ST_MMA);
-                    for (int g = g_lo; ok && g <= g_hi; g++) ok = bar_wait<LIST>(&B.kv_full[s][g], ph, abort_flag, status_w, ST_MMA);
-                    if (!ok) break;
+                    lane_ok &= bar_wait<LIST>(&B.s_empty[s], ph ^ 1, abort_flag, status_w, ST_MMA);
+                    for (int g = g_lo; g <= g_hi; g++) lane_ok &= bar_wait<LIST>(&B.kv_full[s][g], ph, abort_flag, status_w, ST_MMA);
                     if (mw == 0 && lane == 0) GS_STAMP(it, PF_KV_FULL);
                     if (mw == 0 && lane == 0 && it == 0) GS_CTA_STAMP(2);
                     issue_s(it);
@@ -709,12 +708,11 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                     }
                 }
                 // ---- O^T[my tiles] += V^T . P^T ----
-                ok = bar_wait<LIST>(&B.p_full[s], ph, abort_flag, status_w, ST_MMA);
+                lane_ok &= bar_wait<LIST>(&B.p_full[s], ph, abort_flag, status_w, ST_MMA);
                 // P.V reads every value block of the tile: all groups (they have landed: the scores the softmax
                 // just turned into P needed them; the waits return at once and make that landing visible here)
-                for (int g = 0; ok && g < g_all; g++) ok = bar_wait<LIST>(&B.kv_full[s][g], ph, abort_flag, status_w, ST_MMA);
-                if (ok && j == 0) ok = bar_wait<LIST>(&B.o_empty, (sgc & 1) ^ 1, abort_flag, status_w, ST_MMA);
-                if (!ok) break;
+                for (int g = 0; g < g_all; g++) lane_ok &= bar_wait<LIST>(&B.kv_full[s][g], ph, abort_flag, status_w, ST_MMA);
+                if (j == 0) lane_ok &= bar_wait<LIST>(&B.o_empty, (sgc & 1) ^ 1, abort_flag, status_w, ST_MMA);
                 if (mw == 0 && lane == 0) GS_STAMP(it, PF_P_FULL_SEEN);
                 tc_fence_after();
                 const int valid = min(TILE, sg.r1 - (sg.r0 + j * TILE));
@@ -734,7 +732,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                         umma_commit(&B.q_empty);
                     }
                 }
-                __syncwarp();
+                ok = __all_sync(0xffffffffu, !gave_up(lane_ok));
                 if (mw == 0 && lane == 0) GS_STAMP(it, PF_PV_ISSUED);
             }
             sgc++;
@@ -756,7 +754,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
         const uint64_t pol_keep = l2_policy_evict_last();  // the partial records are read next, by the combine kernel
         float l_part[HQ];                             // row sums of this thread's cache row, per query row
         float nm[HQ];                                 // minus the reference maximum (log2 units) per query row
-        bool ok = true;
+        bool ok = true, lane_ok = true;               // (of the group; of this lane's waits)
         if (LIST && sc.whole && sc.share == 1) {
             // a query that attends nothing gets zeros (crates/cuda/kernels/ops.cu:535); such sequences yield no segment
             for (int b = (int) blockIdx.x; b < P.n_seq; b += (int) gridDim.x) {
@@ -820,7 +818,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
             for (int j = 0; j < sg.n_tiles; j++, it++) {
                 const int s = it & 1;
                 const uint32_t ph = (it >> 1) & 1;
-                (void) bar_wait<LIST>(&B.s_full[s], ph, abort_flag, status_w, ST_SOFTMAX);
+                lane_ok &= bar_wait<LIST>(&B.s_full[s], ph, abort_flag, status_w, ST_SOFTMAX);
                 GS_STAMP(it, PF_S_FULL);
                 tc_fence_after();
                 const int row0 = sg.r0 + j * TILE;
@@ -862,9 +860,9 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                 bool exceed = false;
 #pragma unroll
                 for (int i = 0; i < HQ; i++) exceed |= fmaf(sv[i], P.scale_log2, nm[i]) > RESCALE_LOG2;
-                // one barrier per tile: combines the vote and orders the group; on abort every thread leaves together
-                const bool slow = group_any(2, 128, exceed);
-                if (*abort_flag) { ok = false; break; }
+                // one barrier per tile: combines the vote and orders the group.  A thread whose wait gave up (a wait of any
+                // other role does, too, once the flag is set) votes for the slow path, where the group decides whether to leave.
+                const bool slow = group_any(2, 128, exceed || gave_up(lane_ok));
                 GS_STAMP(it, PF_VOTED);
                 bool rescale = false;
                 if (slow) {
@@ -879,7 +877,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
                         if ((lane & 15) == 0) M.smax[qt][col0 + i] = mx;
                     }
-                    named_bar_sync(1, 128);
+                    if (group_any(1, 128, *abort_flag != 0)) { ok = false; break; }
                     if (wg_tid < NQ) {
                         const int q = wg_tid;
                         const float mt = fmaxf(fmaxf(M.smax[0][q], M.smax[1][q]), fmaxf(M.smax[2][q], M.smax[3][q]));
@@ -906,7 +904,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                         nm[i] = mr == -INFINITY ? UNSET : -mr;
                     }
                 }
-                (void) bar_wait<LIST>(&B.p_empty[s], ph ^ 1, abort_flag, status_w, ST_SOFTMAX);
+                lane_ok &= bar_wait<LIST>(&B.p_empty[s], ph ^ 1, abort_flag, status_w, ST_SOFTMAX);
                 // probabilities: row sums in registers; P^T as f16, 8 query rows per 16-byte store, in the
                 // MN-major operand layout [q/8][row/8][row%8][q%8].  A masked score is -inf and gives 0; an
                 // unset column holds only masked scores.
@@ -929,7 +927,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                 }
                 if (rescale) {
                     // S of this tile may have been issued ahead of P.V of the previous one: wait for that P.V
-                    (void) bar_wait<LIST>(&B.p_empty[s ^ 1], ((it - 1) >> 1) & 1, abort_flag, status_w, ST_SOFTMAX);
+                    lane_ok &= bar_wait<LIST>(&B.p_empty[s ^ 1], ((it - 1) >> 1) & 1, abort_flag, status_w, ST_SOFTMAX);
                     tc_fence_after();
 #pragma unroll 1
                     for (int mt = 0; mt < NVT; mt++) {
@@ -967,8 +965,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
             if (!ok) break;
             // ---- end of segment: drain the accumulators into this segment's partial record ----------------
             if (!LIST || sg.n_tiles > 0) (void) bar_wait<LIST>(&B.o_full, sgc & 1, abort_flag, status_w, ST_SOFTMAX);
-            named_bar_sync(2, 128);
-            if (*abort_flag) { ok = false; break; }
+            if (group_any(2, 128, *abort_flag != 0)) { ok = false; break; }
             tc_fence_after();
             if (wg_tid == 0) GS_STAMP(kProfTiles - 1, 2);
             if (wg_tid == 0) GS_CTA_STAMP(3);
@@ -1160,7 +1157,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
         // TMA tiles of consecutive rows 0.54.  In the kernel, 256-token chunk of 2052-row lists, 64 heads: one warp 190 us,
         // two 183, four 166 us, four through registers 228 us.)
         const int pw = warp - 8;
-        bool ok = true;
+        bool ok = true, lane_ok = true;  // (of the warp; of this lane's waits)
         while (ok && next_segment(pos, b_cur, end, M.cum, unit_rows, M.len, sg, sc)) {
             const int32_t *lp = P.sel + (int64_t) (sg.b / P.seq_div) * P.sel_stride + sg.r0;
             const int n_rows = sg.r1 - sg.r0;
@@ -1168,7 +1165,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
             // lane l holds the cache rows of tile rows l and l + 32, of this tile and of the next (requested a tile ahead)
             auto entry = [&](int i) { return i < n_rows ? max(__ldcg(lp + i), 0) : 0; };
             int ra = entry(lane), rb = entry(lane + 32), na = entry(TILE + lane), nb = entry(TILE + lane + 32);
-            for (int j = 0; j < sg.n_tiles; j++, it++, n_left -= TILE) {
+            for (int j = 0; ok && j < sg.n_tiles; j++, it++, n_left -= TILE) {
                 const int s = it & 1;
                 uint8_t *dst = kv_smem + s * STAGE_BYTES;
                 auto row_of = [&](int r) { return (int64_t) __shfl_sync(0xffffffffu, r < 32 ? ra : rb, r & 31); };
@@ -1198,8 +1195,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                         }
                     }
                     next_rows();
-                    ok = bar_wait<LIST>(&B.kv_empty[s], ((it >> 1) & 1) ^ 1, abort_flag, status_w, ST_PRODUCER);
-                    if (!ok) break;
+                    lane_ok &= bar_wait<LIST>(&B.kv_empty[s], ((it >> 1) & 1) ^ 1, abort_flag, status_w, ST_PRODUCER);
                     // lanes of every other 64-column block store their odd chunk first, so that one store instruction covers
                     // all eight chunk positions of the 128-byte lines (four lanes each) instead of four (eight lanes each)
                     const int flip = (lane >> 2) & 1;
@@ -1231,8 +1227,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&B.kv_full[s][0]);
                 } else {
-                    ok = bar_wait<LIST>(&B.kv_empty[s], ((it >> 1) & 1) ^ 1, abort_flag, status_w, ST_PRODUCER);
-                    if (!ok) break;
+                    lane_ok &= bar_wait<LIST>(&B.kv_empty[s], ((it >> 1) & 1) ^ 1, abort_flag, status_w, ST_PRODUCER);
                     if (pw == 0 && lane == 0) GS_STAMP(it, PF_LOAD_ISSUE);
                     const char *cbase = reinterpret_cast<const char *>(P.list_cache) + lane * 16;
 #pragma unroll
@@ -1250,6 +1245,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                     cp_async_mbar_arrive(&B.kv_full[s][0]);
                     next_rows();
                 }
+                ok = __all_sync(0xffffffffu, !gave_up(lane_ok));
             }
         }
     }
@@ -1257,14 +1253,15 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
     // ---- common exit -----------------------------------------------------------------------------------------
     tc_fence_before();
     __syncthreads();
-    if (LIST && sc.share > 1) cluster_sync();  // no CTA leaves while another may still write to its shared memory
     if (*abort_flag && tid == 0) {
-        // loads that were issued but never consumed may still be landing in this CTA's shared memory
+        // loads that were issued but never consumed may still be landing in this CTA's shared memory, and copies it sent in
+        // another CTA's
         const long long t0 = clock64();
         while (clock64() - t0 < 2000000LL) {
         }
     }
     __syncthreads();
+    if (LIST && sc.share > 1) cluster_sync();  // no CTA leaves while another may still write to its shared memory
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, TMEM_COLS);

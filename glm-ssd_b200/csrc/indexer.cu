@@ -372,8 +372,9 @@ __global__ void __launch_bounds__(st_threads(KB), 1) k_idx_score_umma(const Scor
                 n_a++;
             }
             left--;
-            ok = ok && mbar_wait(&M.d_empty[un & 1], ((un >> 1) & 1) ^ 1, abort_flag, status, 2) &&
-                 mbar_wait(&M.b_full[st], st_ph, abort_flag, status, 2);
+            bool lane_ok = mbar_wait_lane(&M.d_empty[un & 1], ((un >> 1) & 1) ^ 1, abort_flag, status, 2);
+            lane_ok &= mbar_wait_lane(&M.b_full[st], st_ph, abort_flag, status, 2);
+            ok = __all_sync(0xffffffffu, ok && lane_ok);
             if (!ok) break;
             const uint32_t d = tmem + (un & 1) * 2 * ST_N + kb * ST_N;
             const uint64_t bd = d_kmaj + (b_lo + st * (ST_STAGE >> 4));

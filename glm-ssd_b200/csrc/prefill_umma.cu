@@ -211,15 +211,14 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
         constexpr uint32_t idesc_s = make_idesc_f16(BM, BN, 0, 0);
         const uint64_t d_kmaj = make_smem_desc(0, 16, 1024, kSwizzle128B);
         const uint32_t q_lo = smem_desc_addr(q_smem), k_lo = smem_desc_addr(k_smem);
-        bool ok = n_tiles == 0 || mbar_wait(&B.q_full, 0, abort_flag, P.status, 2);
+        bool ok = n_tiles == 0 || mbar_wait(&B.q_full, 0, abort_flag, P.status, 2), lane_ok = true;  // (of the warp; of this lane's waits)
         // Scores run up to three tiles ahead of the softmax: S(j) goes into tensor-memory buffer j & 3, where
         // P(j-4) lives until P.V(j-4) has read it.  Two MMAs are only ordered with respect to each other on the
         // same accumulator, so that P.V is awaited explicitly.
         for (int j = warp == 1 ? 0 : 1; ok && j < n_tiles; j += 2) {
             const int st = j % K_STAGES, sb = j & (S_BUFS - 1);
-            ok = mbar_wait(&B.k_full[j % (2 * K_STAGES)], (j / (2 * K_STAGES)) & 1, abort_flag, P.status, 2) &&
-                 mbar_wait(&B.p_free[sb], ((j / S_BUFS) & 1) ^ 1, abort_flag, P.status, 2);
-            if (!ok) break;
+            lane_ok &= mbar_wait_lane(&B.k_full[j % (2 * K_STAGES)], (j / (2 * K_STAGES)) & 1, abort_flag, P.status, 2);
+            lane_ok &= mbar_wait_lane(&B.p_free[sb], ((j / S_BUFS) & 1) ^ 1, abort_flag, P.status, 2);
             tc_fence_after();
             if (lane == 0) PF_STAMP(j, 0);
             if (elect_one()) {
@@ -232,19 +231,18 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
                 umma_commit(&B.s_full[sb]);
                 umma_commit(&B.k_empty[st]);
             }
-            __syncwarp();
+            ok = __all_sync(0xffffffffu, lane_ok);
         }
     } else if (warp == 8) {
         // ---- P.V MMA issuer: O += P . V ----------------------------------------------------------------------------
         constexpr uint32_t idesc_pv = make_idesc_f16(BM, HD, 0, 1);  // A = P from tensor memory, B = V MN-major
         const uint64_t d_v = make_smem_desc(0, KBLK, 1024, kSwizzle128B);
         const uint32_t v_lo = smem_desc_addr(v_smem);
-        bool ok = true;
+        bool ok = true, lane_ok = true;
         for (int j = 0; ok && j < n_tiles; j++) {
             const int sb = j & (S_BUFS - 1);
-            ok = mbar_wait(&B.p_full[sb], (j / S_BUFS) & 1, abort_flag, P.status, 2) &&
-                 mbar_wait(&B.v_full[j & 1], (j >> 1) & 1, abort_flag, P.status, 2);
-            if (!ok) break;
+            lane_ok &= mbar_wait_lane(&B.p_full[sb], (j / S_BUFS) & 1, abort_flag, P.status, 2);
+            lane_ok &= mbar_wait_lane(&B.v_full[j & 1], (j >> 1) & 1, abort_flag, P.status, 2);
             tc_fence_after();
             if (lane == 0) PF_STAMP(j, 1);
             if (elect_one()) {
@@ -255,7 +253,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
                 umma_commit(&B.v_empty[j & 1]);
                 umma_commit(&B.p_free[sb]);
             }
-            __syncwarp();
+            ok = __all_sync(0xffffffffu, lane_ok);
         }
     } else {
         // ---- softmax / correction / epilogue: one query row per thread ------------------------------------------
@@ -270,8 +268,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
             for (int j = 0; j < n_tiles; j++) {
                 const int sb = j & (S_BUFS - 1);
                 const uint32_t s_addr = tmem + lane_base + sb * S_COLS;
-                ok = mbar_wait(&B.s_full[sb], (j / S_BUFS) & 1, abort_flag, P.status, 4);
-                if (!ok) break;
+                const bool lane_ok = mbar_wait_lane(&B.s_full[sb], (j / S_BUFS) & 1, abort_flag, P.status, 4);
                 tc_fence_after();
                 if (warp == 2 && lane == 0) PF_STAMP(j, 3);
                 const int k0 = (t0 + j) * BN;
@@ -345,6 +342,8 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&B.p_full[sb]);
                 if (warp == 2 && lane == 0) PF_STAMP(j, 7);
+                ok = __all_sync(0xffffffffu, lane_ok);
+                if (!ok) break;
             }
             // ---- epilogue: O / l -> global ------------------------------------------------------------------------
             // The P.V MMAs come from one thread and share one accumulator, so they complete in order: the last one
@@ -473,16 +472,16 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
     // ---- common exit ---------------------------------------------------------------------------------------------
     tc_fence_before();
     __syncthreads();
-    if (SPLIT) {
-        cluster_sync();  // no CTA leaves while another may still write to its shared memory or read from it
-        if (P.item0 > 0) griddep_wait();  // what follows this launch in the stream also follows the launch in front of it
-    }
-    if (*abort_flag && tid == 0) {
+    if (*abort_flag && tid == 0) {  // loads, and copies to other CTAs of the cluster, may still be in flight
         const long long t0 = clock64();
         while (clock64() - t0 < 2000000LL) {
         }
     }
     __syncthreads();
+    if (SPLIT) {
+        cluster_sync();  // no CTA leaves while another may still write to its shared memory or read from it
+        if (P.item0 > 0) griddep_wait();  // what follows this launch in the stream also follows the launch in front of it
+    }
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, 512);

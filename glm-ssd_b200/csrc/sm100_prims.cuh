@@ -82,6 +82,13 @@ __device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
 // another thread of the CTA has flagged an abort) the wait gives up, records where in the device
 // status word and returns false; the caller then leaves through the kernel's common exit, which
 // releases tensor memory.  A healthy run never comes near the limit (about a second).
+// Who leaves is decided once for all threads that go on to meet again: the lanes of a warp see a barrier and the abort flag
+// at different times, and a lane that left alone would keep the others waiting for ever at the next warp-wide instruction.
+// mbar_wait() votes at once.  Where the wait is on the critical path, callers collect the answers of mbar_wait_lane() and
+// vote once per iteration, when the work of the iteration is issued (a vote behind every wait costs a decode step of 128K rows
+// 0.9 of 35.8 us): a lane that gave up goes through the rest of its iteration with the others, over data that may not have
+// landed, which harms nobody - the result is invalid either way and every later wait ends as well.  group_any() decides
+// for warps that share a named barrier.
 constexpr long long kWaitLimitCycles = 2000000000LL;
 
 // The slow path is kept out of line: the kernels are latency-sensitive to their code size.
@@ -101,10 +108,15 @@ static __device__ __noinline__ bool mbar_wait_slow(uint64_t *bar, uint32_t parit
     }
     return true;
 }
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int32_t *status,
-                                          int32_t code) {
+__device__ __forceinline__ bool mbar_wait_lane(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int32_t *status,
+                                               int32_t code) {
     if (mbar_try_wait(bar, parity)) return true;
     return mbar_wait_slow(bar, parity, abort_flag, status, code);
+}
+// Executed by whole warps.
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int32_t *status,
+                                          int32_t code) {
+    return __all_sync(0xffffffffu, mbar_wait_lane(bar, parity, abort_flag, status, code));
 }
 
 // ---- TMA ----------------------------------------------------------------------------------------------
