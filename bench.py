@@ -51,6 +51,20 @@ SCALE = 1.0 / 16.0
 L2_BYTES = 126 * 1024 * 1024
 
 
+class GaveUp(RuntimeError):
+    """A bounded wait inside a kernel gave up: what was timed is not the work, and every further launch may cost a second."""
+
+
+def must_be_ok(what: str, status: int) -> None:
+    if status != 0:
+        raise GaveUp(f"{what}: a bounded wait inside a kernel gave up (status 0x{status:x})")
+
+
+def note(text: str) -> None:
+    """Progress on stderr: a run that does not come back says where it was."""
+    print(f"bench: {text}", file=sys.stderr, flush=True)
+
+
 def algorithmic_bytes(n_rows: int, T: int, n_seq: int = 1) -> int:
     """Cache rows read once + queries + f32 outputs (the per-call figure of the measurement plan)."""
     return n_rows * D_QK * 2 + n_seq * T * H * D_QK * 2 + n_seq * T * H * D_V * 4
@@ -335,11 +349,12 @@ def _sparse_list_shape(torch, dev, fn, label, profile=False, q8=False):
     """The engine's own decode shape: 64 heads, f32 queries, a sparse list of 2052 positions per query token
     out of a 32768-row cache (forward.rs:461, :873), through the reference's entry point gs_mla_attn."""
     res = {}
+    ours = label != "reference_kernel"
+    pkg = importlib.import_module("glm-ssd_b200") if ours else None
     ctx, n, Hh = 32768, 2052, 64
     caches = [(torch.randn((ctx, 512), device=dev) * 0.5).half() for _ in range(6)]
     scales = [None] * 6
     if q8:  # the reference's Q8 cache (ops.cu:599-610): int8 rows and one f16 scale per 32 values, quantised on the device
-        pkg = importlib.import_module("glm-ssd_b200")
         q8c, q8s = [], []
         for c in caches:
             qq = torch.empty((ctx, 512), dtype=torch.int8, device=dev)
@@ -357,6 +372,8 @@ def _sparse_list_shape(torch, dev, fn, label, profile=False, q8=False):
         o = torch.empty((T, Hh, 512), dtype=torch.float32, device=dev)
         part = torch.empty(T * Hh * splits * 514, dtype=torch.float32, device=dev)  # the reference's size (ops.cu:578)
 
+        note(f"lists, {label}, T = {T}")
+
         def call(i):
             rc = fn(q.data_ptr(), caches[i % 6].data_ptr(), None if scales[i % 6] is None else scales[i % 6].data_ptr(), sel.data_ptr(), n,
                     cnt.data_ptr(), SCALE, o.data_ptr(),
@@ -366,6 +383,8 @@ def _sparse_list_shape(torch, dev, fn, label, profile=False, q8=False):
         for i in range(3):
             call(i)
         torch.cuda.synchronize()
+        if ours:
+            must_be_ok(f"lists, {label}, T = {T}", pkg.mla_attn_status())
         if profile:  # a few eager launches per shape are all a profiler needs
             continue
         # one pass over the cache copies captured in a CUDA graph and replayed: the device's time, not the caller's launch rate
@@ -442,17 +461,21 @@ def run_ours(args) -> None:
             flat[i:i + n] = (torch.randn(n, generator=gen, device=dev, dtype=torch.float32) * sigma).to(torch.float16)
         return out
 
-    def time_loop(fn, steps, warmup, period=1, use_graph=True, repeats=1, spread=None):
+    def time_loop(fn, steps, warmup, period=1, use_graph=True, repeats=1, spread=None, what="", status=None):
         """Device time of `steps` calls of fn(i) after `warmup` calls: barrier + sync on both sides,
         CUDA events on the launching stream, max over ranks.  Returns seconds per step.  With
         `repeats` > 1 the timed region (the same `steps` calls, bracketed the same way) is run that many
         times and the median is returned; `spread` receives min / median / max and the region's length.
+        `status()` reads the status word of the calls' workspace: after the first eager calls and once everything is timed.
 
         `period` consecutive calls (one pass over the rotating buffers) are captured once into a CUDA
         graph and replayed, so the figure is the device's, not the Python caller's launch rate."""
+        note(what)
         for i in range(min(warmup, 3)):
             fn(i)
         torch.cuda.synchronize()
+        if status is not None:
+            must_be_ok(what, status())
         graph = rem_graph = None
         rem = steps % period if steps >= period else 0
         if steps < period:
@@ -509,6 +532,8 @@ def run_ours(args) -> None:
             e1.record()
             barrier()
             per_step.append(max_over_ranks(e0.elapsed_time(e1) * 1e-3) / n_steps)
+        if status is not None:
+            must_be_ok(what, status())
         med = statistics.median(per_step)
         if spread is not None:
             spread.update({"repeats": len(per_step), "steps_per_repeat": n_steps, "us_min": min(per_step) * 1e6,
@@ -533,14 +558,16 @@ def run_ours(args) -> None:
 
     sampler.start()
     spread = {}
-    sec = time_loop(step, args.steps, args.warmup, period=n_copies, repeats=args.repeats, spread=spread)
+    sec = time_loop(step, args.steps, args.warmup, period=n_copies, repeats=args.repeats, spread=spread, what="headline",
+                    status=lambda: pkg.decode_status(ws))
     value = world * bytes_step / sec / 1e9
 
     # ---- roofline pass: the attention kernel alone (combine skipped), same rotation, same graph replay ----
     def step_kernel_only(i):
         pkg.mla_decode(q, caches[i % n_copies], seq_len, out=out, workspace=ws, max_seq_len=n_rows, no_combine=True)
 
-    kern_sec = time_loop(step_kernel_only, min(args.steps, 2000), args.warmup, period=n_copies, repeats=args.repeats)
+    kern_sec = time_loop(step_kernel_only, min(args.steps, 2000), args.warmup, period=n_copies, repeats=args.repeats,
+                         what="attention kernel alone", status=lambda: pkg.decode_status(ws))
     achieved = bytes_step / kern_sec / 1e9
     traffic = None
     tpath = os.path.join(ROOT, "profiles", "traffic.json")
@@ -555,6 +582,7 @@ def run_ours(args) -> None:
                 "kernel_us": kern_sec * 1e6, "algorithmic_bytes_per_launch": bytes_step}
 
     # ---- e2e: host buffers through the call-site mirror ---------------------------------------------
+    note("end to end")
     n_layers = n_copies
     layers = []
     for j in range(n_layers):
@@ -577,6 +605,8 @@ def run_ours(args) -> None:
     # every layer records its graph on its first step: all of that happens here, before anything is timed
     for i in range(max(2 * n_layers, min(args.warmup, 20))):
         e2e_step(i)
+        if i < n_layers:
+            must_be_ok("first step of a layer", pkg.decode_status(layers[i].workspace))
     e2e_runs = []
     for _ in range(max(1, args.repeats)):
         barrier()
@@ -602,6 +632,7 @@ def run_ours(args) -> None:
     # the same step without the wait: the graphs of all layers enqueued back to back on their streams, drained once.
     # What remains of a step then is the device's share (three kernels, one PCIe round trip for the host's rows); the
     # difference to the timed step is launch and completion latency that a step handing its result to the host exposes.
+    note("end to end, enqueued without waiting")
     hs = [lay._graphs[(q_host.data_ptr(), kv_host.data_ptr(), T)] for lay in layers]
     raw_step = layers[0]._graph_step
     torch.cuda.synchronize()
@@ -611,6 +642,8 @@ def run_ours(args) -> None:
         raw_step(hs[j], n_rows - T, layers[j]._graph_stream_handle, 0)
     torch.cuda.synchronize()
     e2e_nowait_us = max_over_ranks((time.perf_counter() - t0)) / e2e_steps * 1e6
+    for lay in layers:
+        must_be_ok("layer steps", pkg.decode_status(lay.workspace))
     clocks = sampler.stop()
     e2e = {"value": world * bytes_step / e2e_sec / 1e9, "unit": "GB/s", "h2d_bytes_per_step": h2d,
            "d2h_bytes_per_step": d2h, "us_per_step": e2e_sec * 1e6, "steps": e2e_steps, "repeats": len(e2e_runs),
@@ -624,6 +657,8 @@ def run_ours(args) -> None:
     if not args.no_others:
         try:
             others = run_others(pkg, torch, dist, dev, world, rank, randn_f16, time_loop, hbm_peak, (tf_peak, tf_sustained), args)
+        except GaveUp:
+            raise
         except Exception as exc:  # keep the headline line even if an extra fails
             others = {"error": f"{type(exc).__name__}: {exc}"}
 
@@ -684,7 +719,8 @@ def run_others(pkg, torch, dist, dev, world, rank, randn_f16, time_loop, hbm_pea
     if world == 1:
         o1 = torch.empty((1, 1, H, D_V), dtype=torch.float32, device=dev)
         sec = time_loop(lambda i: pkg.mla_decode(q1, shards[i % n_copies], lens, out=o1, workspace=ws,
-                                                 max_seq_len=rows_local), steps, warm, period=n_copies)
+                                                 max_seq_len=rows_local), steps, warm, period=n_copies, what="128K rows",
+                        status=lambda: pkg.decode_status(ws))
         exchange = "none"
     else:
         o1 = torch.empty((1, 1, H, D_V), dtype=torch.float32, device=dev)
@@ -794,7 +830,7 @@ def run_others(pkg, torch, dist, dev, world, rank, randn_f16, time_loop, hbm_pea
                                       max_seq_len=int(my_lens.max()))
     else:
         fn = lambda i: None
-    sec = time_loop(fn, min(steps, 50), min(warm, 5))
+    sec = time_loop(fn, min(steps, 50), min(warm, 5), what="paged batch", status=(lambda: pkg.decode_status(wsb)) if len(mine) else None)
     tot = int(lens_all.sum()) * D_QK * 2 + 64 * H * (D_QK * 2 + D_V * 4)
     res["paged64"] = {"metric": "aggregate GB/s", "value": tot / sec / 1e9, "us_per_step": sec * 1e6,
                       "frac_of_hbm_per_gpu": tot / sec / 1e9 / world / hbm_peak, "scaling": "strong",
@@ -817,7 +853,7 @@ def run_others(pkg, torch, dist, dev, world, rank, randn_f16, time_loop, hbm_pea
         ot = torch.empty((1, T, Ht, 512), dtype=torch.float32, device=dev)
         wt = pkg.new_workspace(1, T, Ht, 512, dev)
         sec = time_loop(lambda i: pkg.mla_decode(qt, cs[i % nc], lt, out=ot, workspace=wt, max_seq_len=n), steps, warm,
-                        period=nc)
+                        period=nc, what=f"twin shape {name}", status=lambda: pkg.decode_status(wt))
         twin[name] = {"us_per_call": sec * 1e6, "GB/s": n * 1024 / sec / 1e9}
         del cs
         torch.cuda.empty_cache()
@@ -841,7 +877,10 @@ def run_others(pkg, torch, dist, dev, world, rank, randn_f16, time_loop, hbm_pea
             pkg.mla_attn_impl(0)
         torch.cuda.synchronize()
         sp["tensor_path_status"] = pkg.mla_attn_status()
+        must_be_ok("lists", sp["tensor_path_status"])
         res["gs_mla_attn_sparse"] = sp
+    except GaveUp:
+        raise
     except Exception as exc:
         res["gs_mla_attn_sparse"] = {"error": f"{type(exc).__name__}: {exc}"}
     torch.cuda.empty_cache()
@@ -852,7 +891,8 @@ def run_others(pkg, torch, dist, dev, world, rank, randn_f16, time_loop, hbm_pea
     pkg.rope_f16_inplace(Q)
     pkg.rope_f16_inplace(K)
     O = torch.empty((S, H, d), dtype=torch.float32, device=dev)
-    sec = time_loop(lambda i: pkg.prefill_attn(Q, K, V, out=O), min(steps, 20), 3)
+    pst = torch.zeros(1, dtype=torch.int32, device=dev)
+    sec = time_loop(lambda i: pkg.prefill_attn(Q, K, V, out=O, status=pst), min(steps, 20), 3, what="prefill", status=lambda: int(pst))
     flops = H * S * (S + 1) / 2 * (2 * d + 2 * d)
     # one launch after an idle pause (the board is below its power cap), then the clock during half a second of launches
     single = []
@@ -861,7 +901,7 @@ def run_others(pkg, torch, dist, dev, world, rank, randn_f16, time_loop, hbm_pea
         time.sleep(0.05)
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record()
-        pkg.prefill_attn(Q, K, V, out=O)
+        pkg.prefill_attn(Q, K, V, out=O, status=pst)
         e1.record()
         torch.cuda.synchronize()
         single.append(e0.elapsed_time(e1))
@@ -870,8 +910,9 @@ def run_others(pkg, torch, dist, dev, world, rank, randn_f16, time_loop, hbm_pea
     t_end = time.perf_counter() + 0.5
     while time.perf_counter() < t_end:
         for _ in range(20):
-            pkg.prefill_attn(Q, K, V, out=O)
+            pkg.prefill_attn(Q, K, V, out=O, status=pst)
         torch.cuda.synchronize()
+        must_be_ok("prefill under load", int(pst))
     load_clocks = load.stop()
     res["prefill8k"] = {"metric": "TFLOP/s (causal FLOPs)", "value": flops / sec / 1e12, "ms_per_step": sec * 1e3,
                         "frac_of_tensor_peak": flops / sec / 1e12 / tf_peak[0],
@@ -950,7 +991,11 @@ def main() -> None:
     elif args.impl == "reference":
         run_reference(args)
     else:
-        run_ours(args)
+        try:
+            run_ours(args)
+        except GaveUp as exc:
+            print(json.dumps({"error": str(exc)}), flush=True)
+            raise SystemExit(1)
 
 
 if __name__ == "__main__":

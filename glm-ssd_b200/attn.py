@@ -149,8 +149,10 @@ def combine_parts(parts, n_parts, rows, d_v=512, out=None, part_stride=None):
     return out
 
 
-def prefill_attn(q, k, v, *, p0=0, scale=SCALE_256, out=None, out_f16=False, impl=0):
-    """Causal prefill attention.  q f16 [S,H,d]; k, v f16 [p0+S,H,d] -> f32 or f16 [S,H,d]."""
+def prefill_attn(q, k, v, *, p0=0, scale=SCALE_256, out=None, out_f16=False, impl=0, status=None):
+    """Causal prefill attention.  q f16 [S,H,d]; k, v f16 [p0+S,H,d] -> f32 or f16 [S,H,d].  ``status``: optional int32
+    tensor of one element on the device, zeroed once; becomes non-zero when a bounded wait inside the kernel gave up (the
+    output of that call is then not valid).  ``decode_status`` reads it."""
     for t, n in ((q, "q"), (k, "k"), (v, "v")):
         _need(t, torch.float16, n)
     S, H, d = q.shape
@@ -158,9 +160,12 @@ def prefill_attn(q, k, v, *, p0=0, scale=SCALE_256, out=None, out_f16=False, imp
         raise ValueError("k and v must be [p0+S, H, d]")
     if out is None:
         out = torch.empty((S, H, d), dtype=torch.float16 if out_f16 else torch.float32, device=q.device)
-    _lib.check(_lib.load().gs_prefill_attn(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
-                                           1 if out.dtype == torch.float16 else 0, S, H, d, p0, scale, impl,
-                                           _stream()), "gs_prefill_attn")
+    args = (q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), 1 if out.dtype == torch.float16 else 0, S, H, d, p0, scale, impl)
+    if status is None:
+        _lib.check(_lib.load().gs_prefill_attn(*args, _stream()), "gs_prefill_attn")
+    else:
+        _need(status, torch.int32, "status")
+        _lib.check(_lib.load().gs_prefill_attn_checked(*args, status.data_ptr(), _stream()), "gs_prefill_attn_checked")
     return out
 
 

@@ -109,6 +109,20 @@ def test_prefill_many_launches_no_wait_gives_up(pkg, cuda):
         assert torch.equal(o, w)
 
 
+def test_prefill_status_word(pkg, cuda):
+    """The word a caller passes stays zero in a healthy call and is not cleared by one."""
+    torch = cuda
+    q, k, v = (to_dev(cuda, a) for a in _qkv(6, 200, 4, 256))
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    got = pkg.prefill_attn(q, k, v, status=status)
+    assert pkg.decode_status(status) == 0 and torch.equal(got, pkg.prefill_attn(q, k, v))
+    status.fill_(4)
+    pkg.prefill_attn(q, k, v, status=status)
+    assert pkg.decode_status(status) == 4
+    with pytest.raises(ValueError):
+        pkg.prefill_attn(q, k, v, status=torch.zeros(1, device="cuda"))
+
+
 def test_prefill_f16_output(pkg, cuda, oracle):
     Q, K, V = _qkv(5, 200, 4, 256)
     got = pkg.prefill_attn(to_dev(cuda, Q), to_dev(cuda, K), to_dev(cuda, V), out_f16=True)
