@@ -1237,9 +1237,8 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
 #pragma unroll
                         for (int h = 0; h < 2; h++) {
                             const int c = h * 32 + lane;
-                            uint8_t *d = dst + (c >> 3) * BLK_BYTES + r * 128 + (((c & 7) ^ (r & 7)) << 4);
-                            if (r < n_left) cp_async16(d, src + h * 512);
-                            else *reinterpret_cast<uint4 *>(d) = make_uint4(0, 0, 0, 0);  // rows past the segment's end become zeros
+                            // (rows past the segment's end become zeros; their entries name row 0, which is not read)
+                            cp_async16_or_zero(dst + (c >> 3) * BLK_BYTES + r * 128 + (((c & 7) ^ (r & 7)) << 4), src + h * 512, r < n_left);
                         }
                     }
                     cp_async_mbar_arrive(&B.kv_full[s][0]);

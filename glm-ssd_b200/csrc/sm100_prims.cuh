@@ -142,6 +142,11 @@ __device__ __forceinline__ void bulk_load(void *smem_dst, const void *gsrc, uint
 __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
 }
+// The same with zeros in the place of the data when `valid` is false (nothing is read then): unlike an ordinary store, the
+// zeros are covered by the arrival below.
+__device__ __forceinline__ void cp_async16_or_zero(void *smem_dst, const void *gsrc, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)), "l"(gsrc), "r"(valid ? 16 : 0) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_mbar_arrive(uint64_t *bar) {

@@ -320,6 +320,37 @@ def test_gs_mla_attn_lists_around_four_tiles(pkg, cuda, oracle, T, H):
     test_gs_mla_attn_list_cuts(pkg, cuda, oracle, False, T, H, [(255, 256, 257, 319, 321, 64, 0)[i % 7] for i in range(T)], 336)
 
 
+@pytest.mark.parametrize("q8", [False, True])
+def test_gs_mla_attn_ragged_tail_behind_rows_that_are_not_finite(pkg, cuda, oracle, q8):
+    """The rows past a list's end count as zeros, whatever an earlier list of the same CTA left in shared memory: 160 lists of
+    whole tiles over NaN and infinite rows first, lists that end inside a 16-row group behind them."""
+    torch = cuda
+    T, H, ctx, stride, n_sms = 300, 64, 2000, 256, torch.cuda.get_device_properties(0).multi_processor_count
+    rng = np.random.default_rng(17)
+    q = rng.standard_normal((T, H, 512), dtype=np.float32)
+    Cc = (rng.standard_normal((ctx, 512), dtype=np.float32) * np.float32(0.5)).astype(np.float16)
+    cq, cs = oracle.quant_q8_rows(Cc.astype(np.float32)) if q8 else (Cc, None)
+    bad = rng.permutation(ctx)[:200]
+    good = np.setdiff1d(np.arange(ctx), bad)
+    if q8:
+        cs[bad] = np.float16(np.nan)
+    else:
+        cq[bad[:100]], cq[bad[100:]] = np.float16(np.nan), np.float16(np.inf)
+    sel = np.zeros((T, stride), np.int32)
+    cnt = np.full(T, 128, np.int32)
+    sel[:n_sms] = rng.choice(bad, size=(n_sms, stride))
+    sel[n_sms:] = rng.choice(good, size=(T - n_sms, stride))
+    cnt[n_sms:] = [(1, 15, 17, 63, 65, 129, 191, 250)[i % 8] for i in range(T - n_sms)]
+    o = torch.empty((T, H, 512), dtype=torch.float32, device="cuda")
+    pkg.mla_attn(to_dev(torch, q), to_dev(torch, cq), None if cs is None else to_dev(torch, cs), to_dev(torch, sel), stride, to_dev(torch, cnt),
+                 1 / 16, o, None, T, H, 512, 1)
+    assert pkg.mla_attn_status() == 0
+    got = o.cpu().numpy()
+    assert np.isnan(got[0]).all()
+    want = oracle.mla_attn_ref(q[n_sms:], oracle.dequant_q8(cq, cs) if q8 else cq, sel[n_sms:], cnt[n_sms:], 1 / 16)
+    check_close(got[n_sms:], want, "lists behind rows that are not finite")
+
+
 def test_gs_mla_attn_lists_with_scattered_unsorted_and_repeated_rows(pkg, cuda, oracle):
     """Position lists are arbitrary: unsorted, with repeats, not in groups of four, different lengths per token."""
     rng = np.random.default_rng(5)
