@@ -1327,7 +1327,9 @@ struct ListPlan {
 // 2.85 / 3.4 with 64, 2.5 and 3.1 in a cluster; a cluster's start and merge 7.5 / 9.5 us, 17 with 64 columns (two rounds of the
 // exchange), 2.5 more with 16 CTAs and a little for every CTA that fetches; records and their combine 11 us, 7 when there is one sequence (its schedule needs no
 // scan).  The choice it makes is within about 6 % of the best cut measured.
-static ListPlan list_plan(int T, int H, int R, int sel_stride, int splits, const float *part, bool q8, int grid_max) {
+// Clusters and the combine store o in 16-byte words; an o that is not aligned for them (`o_aligned`) leaves one CTA per sequence,
+// which stores single words.
+static ListPlan list_plan(int T, int H, int R, int sel_stride, int splits, const float *part, bool o_aligned, bool q8, int grid_max) {
     ListPlan best{0, 0, 1, true, 1e30f};
     auto offer = [&](int n, int64_t grid, int cluster, bool whole, float cost) {
         if (cost < best.cost) best = ListPlan{n, (int) grid, cluster, whole, cost};
@@ -1341,7 +1343,7 @@ static ListPlan list_plan(int T, int H, int R, int sel_stride, int splits, const
         const float t_cl = (Hg <= 32 ? 2.5f : Hg <= 48 ? 2.8f : 3.1f) + (q8 ? 0.2f : 0.f);
         const int64_t grid = n_seq_k < grid_max ? n_seq_k : grid_max;
         offer(n, grid, 1, true, (float) ((n_seq_k + grid - 1) / grid * tiles_seq) * t_one + 2.f);
-        for (int c = 2; c <= MAX_CLUSTER; c *= 2) {
+        for (int c = 2; o_aligned && c <= MAX_CLUSTER; c *= 2) {
             // CTAs of clusters of c that run at once on 148 SMs, one per SM
             const int resident = c == 2 ? 148 : c == 4 ? 132 : c == 8 ? 120 : 112;
             if (n_seq_k * c > (resident < grid_max ? resident : grid_max)) break;
@@ -1349,7 +1351,7 @@ static ListPlan list_plan(int T, int H, int R, int sel_stride, int splits, const
             offer(n, n_seq_k * c, c, true, (float) ((per + TILE - 1) / TILE) * t_cl + (Hg <= 48 ? 6.5f + 0.03f * (float) Hg : 17.f) +
                                                (c == 16 ? 2.5f : 0.f) + (q8 ? 2.f : 0.f) + 0.03f * (float) (n_seq_k * c));
         }
-        if (splits > 1 && part && !(reinterpret_cast<uintptr_t>(part) & 15)) {
+        if (o_aligned && splits > 1 && part && !(reinterpret_cast<uintptr_t>(part) & 15)) {
             // records that fit the caller's buffer
             const int64_t part_floats = (int64_t) T * H * splits * (R + 2);
             const int64_t desc_floats = (n_seq_k * 2 + 3) / 4 * 4;
@@ -1374,7 +1376,7 @@ int launch_decode_umma_list(const float *q, const void *C, const __half *C_scale
     if ((reinterpret_cast<uintptr_t>(C) & 15) || (reinterpret_cast<uintptr_t>(q) & 15) || (reinterpret_cast<uintptr_t>(C_scales) & 15)) return -1;
     int grid_max = sm_count < kMaxCtas ? sm_count : kMaxCtas;
     if (grid_max < 1) grid_max = 1;
-    const ListPlan L = list_plan(T, H, R, sel_stride, splits, part, C_scales != nullptr, grid_max);
+    const ListPlan L = list_plan(T, H, R, sel_stride, splits, part, !(reinterpret_cast<uintptr_t>(o) & 15), C_scales != nullptr, grid_max);
     if (L.n_groups == 0) return -1;
     const int n_groups = L.n_groups;
     const int64_t n_seq_k = (int64_t) T * n_groups;

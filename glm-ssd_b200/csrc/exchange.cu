@@ -229,6 +229,7 @@ __global__ void __launch_bounds__(CB_NT) k_exchange_combine(const __grid_constan
 
 int launch_exchange_combine(CombinePlan c, const gs_shard_exchange &x, float *o, int32_t *status, int sm_count,
                             cudaStream_t st) {
+    if (reinterpret_cast<uintptr_t>(o) & 15) return fail_invalid("gs_mla_decode: with an exchange, o must be 16-byte aligned");
     const int rows = c.n_seq * c.T * c.H;
     if (x.world < 2 || x.world > kMaxWorld || x.rank < 0 || x.rank >= x.world)
         return fail_invalid("exchange: world must be 2..8 and 0 <= rank < world");

@@ -320,6 +320,40 @@ def test_gs_mla_attn_lists_around_four_tiles(pkg, cuda, oracle, T, H):
     test_gs_mla_attn_list_cuts(pkg, cuda, oracle, False, T, H, [(255, 256, 257, 319, 321, 64, 0)[i % 7] for i in range(T)], 336)
 
 
+@pytest.mark.parametrize("T,splits", [(1, 16), (2, 4), (2, 1), (60, 1)])
+def test_gs_mla_attn_output_at_any_word(pkg, cuda, oracle, T, splits):
+    """An o that is aligned to a float only, at sizes where an aligned one is stored in 16-byte words."""
+    torch = cuda
+    H, ctx, n = 64, 3000, 2052
+    rng = np.random.default_rng(T)
+    q = rng.standard_normal((T, H, 512), dtype=np.float32)
+    Cc = (rng.standard_normal((ctx, 512), dtype=np.float32) * np.float32(0.5)).astype(np.float16)
+    sel, cnt = rng.integers(0, ctx, size=(T, n)).astype(np.int32), np.full(T, n, np.int32)
+    part = torch.empty(T * H * splits * 514, dtype=torch.float32, device="cuda") if splits > 1 else None
+    want = oracle.mla_attn_ref(q, Cc, sel, cnt, 1 / 16)
+    args = [to_dev(torch, a) for a in (q, Cc, sel, cnt)]
+    for off in (0, 1, 2):
+        buf = torch.full((T * H * 512 + 8,), 7.0, device="cuda")
+        o = buf[off:off + T * H * 512]
+        pkg.mla_attn(args[0], args[1], None, args[2], n, args[3], 1 / 16, o, part, T, H, 512, splits)
+        assert pkg.mla_attn_status() == 0
+        check_close(o.view(T, H, 512).cpu().numpy(), want, f"o at word {off}")
+        assert (buf[:off] == 7).all() and (buf[off + T * H * 512:] == 7).all()
+
+
+def test_outputs_the_merge_cannot_store_are_refused(pkg, cuda):
+    """Decode outputs and record blocks that are not 16-byte aligned come back as an error instead of a misaligned access."""
+    torch = cuda
+    q, c = (torch.zeros(s, dtype=torch.float16, device="cuda") for s in ((1, 1, 20, 576), (256, 576)))
+    lens = torch.full((1,), 256, dtype=torch.int32, device="cuda")
+    buf = torch.zeros(20 * 514 + 4, device="cuda")
+    with pytest.raises(pkg._lib.GsError):
+        pkg.mla_decode(q, c, lens, out=buf[1:1 + 20 * 512].view(1, 1, 20, 512))
+    with pytest.raises(pkg._lib.GsError):
+        pkg.mla_decode(q, c, lens, want_out=False, part_out=buf[2:])
+    torch.cuda.synchronize()
+
+
 @pytest.mark.parametrize("q8", [False, True])
 def test_gs_mla_attn_ragged_tail_behind_rows_that_are_not_finite(pkg, cuda, oracle, q8):
     """The rows past a list's end count as zeros, whatever an earlier list of the same CTA left in shared memory: 160 lists of
