@@ -420,34 +420,38 @@ __global__ void __launch_bounds__(st_threads(KB), 1) k_idx_score_umma(const Scor
             const int p = pt * ST_M + row;
             if (new_tile) {
                 new_tile = false;
-                // the MMAs of the old tile are over when its last unit's accumulators are complete
-                if (un > 0) (void) mbar_wait(&M.d_full[(un - 1) & 1], ((un - 1) >> 1) & 1, abort_flag, status, 4);
-                const float *src = S.P + (int64_t) p * S.Dk;
-                float4 x[KB][8];
+                // the MMAs of the old tile are over when its last unit's accumulators are complete; if that does not come, they
+                // may still be reading the old parts, which then stay (the waits for the new ones end with the abort flag)
+                const bool over = un == 0 || mbar_wait(&M.d_full[(un - 1) & 1], ((un - 1) >> 1) & 1, abort_flag, status, 4);
+                tc_fence_after();  // (group g has ordered itself behind its own units only)
+                if (over) {
+                    const float *src = S.P + (int64_t) p * S.Dk;
+                    float4 x[KB][8];
 #pragma unroll
-                for (int i = 0; i < KB; i++)
+                    for (int i = 0; i < KB; i++)
 #pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        const int c = (g * KB + i) * 32 + j * 4;
-                        x[i][j] = p < S.n_pools && c < S.Dk ? __ldcg(reinterpret_cast<const float4 *>(src + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        for (int j = 0; j < 8; j++) {
+                            const int c = (g * KB + i) * 32 + j * 4;
+                            x[i][j] = p < S.n_pools && c < S.Dk ? __ldcg(reinterpret_cast<const float4 *>(src + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        }
+#pragma unroll
+                    for (int i = 0; i < KB; i++) {
+                        uint32_t p1[16], p2[16], p3[16];
+#pragma unroll
+                        for (int j = 0; j < 8; j++) {
+                            split3(x[i][j].x, x[i][j].y, p1[2 * j], p2[2 * j], p3[2 * j]);
+                            split3(x[i][j].z, x[i][j].w, p1[2 * j + 1], p2[2 * j + 1], p3[2 * j + 1]);
+                        }
+                        const uint32_t a = tmem + lane_base + ST_A_COL + (g * KB + i) * 16;
+                        tmem_st16(a, p1);
+                        tmem_st16(a + 64, p2);
+                        tmem_st16(a + 128, p3);
                     }
-#pragma unroll
-                for (int i = 0; i < KB; i++) {
-                    uint32_t p1[16], p2[16], p3[16];
-#pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        split3(x[i][j].x, x[i][j].y, p1[2 * j], p2[2 * j], p3[2 * j]);
-                        split3(x[i][j].z, x[i][j].w, p1[2 * j + 1], p2[2 * j + 1], p3[2 * j + 1]);
-                    }
-                    const uint32_t a = tmem + lane_base + ST_A_COL + (g * KB + i) * 16;
-                    tmem_st16(a, p1);
-                    tmem_st16(a + 64, p2);
-                    tmem_st16(a + 128, p3);
+                    tmem_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&M.a_full);
                 }
-                tmem_wait_st();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&M.a_full);
             }
             if ((un & 1) != g) continue;
             const int t0 = tg * S.tok, n_tok = min(S.tok, S.T - t0);

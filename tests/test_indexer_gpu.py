@@ -98,7 +98,10 @@ def test_idx_score_vs_oracle_and_reference(pkg, cuda, oracle, T, pos0, Hq, Dk, k
     (5, 510, 32, 128, 4),      # two units of queries (4 + 1), one exact pool tile
     (4, 515, 32, 128, 4),      # the last query count below the tensor form
     (6, 509, 48, 128, 4),      # columns past the last whole query of a unit
-    (17, 1530, 80, 64, 4),     # one query per unit, one block of columns, three pool tiles
+    (17, 1530, 80, 64, 4),     # more heads than a unit has columns: the CUDA-core form
+    (17, 1530, 64, 64, 4),     # one query per unit, one block of columns, three pool tiles
+    (66, 30000, 64, 52, 4),    # one block with columns past Dk, 60 pool tiles: CTAs change theirs and go round the ring
+    (150, 9000, 16, 64, 1),    # four queries per unit, 72 pool tiles
     (9, 3, 16, 100, 1),        # fewer pools than a tile, columns past Dk
     (130, 20000, 64, 128, 4),  # many units per CTA: a CTA changes its pool tile
 ])
