@@ -254,6 +254,30 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t &w1, uint32_t 
     w3 = *reinterpret_cast<const uint32_t *>(&h3);
 }
 
+// One score in f32 on this thread, with the sums of the CUDA-core form: for values the split cannot hold.  An infinite or
+// near-maximal operand splits into infinity and x - infinity, every sum it enters is NaN, and relu makes that a 0 where an f32
+// sum keeps the infinity.  (Out of line: nobody should come here.)
+static __device__ __noinline__ float score_f32(const ScoreParams &S, int t, int p) {
+    const float *k = S.P + (int64_t) p * S.Dk;
+    float total = 0.f;
+    for (int h = 0; h < S.Hq; h++) {
+        const float *v = S.q + ((int64_t) t * S.Hq + h) * S.Dk;
+        float a[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int c = 0; c < S.Dk; c += 4)  // (Dk is a multiple of four in this form)
+#pragma unroll
+            for (int i = 0; i < 4; i++) a[i] = fmaf(v[c + i], k[c + i], a[i]);
+        total = fmaf(S.w[(int64_t) t * S.Hq + h], fmaxf(((a[0] + a[1]) + (a[2] + a[3])) * S.scale, 0.f), total);
+    }
+    return total;
+}
+
+// relu that passes a NaN on, so that it is seen in the total.
+__device__ __forceinline__ float relu_nan(float x) {
+    float r;
+    asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // KB: 64-column blocks of a row (Dk <= 64 * KB)
 template <int KB>
 __global__ void __launch_bounds__(st_threads(KB), 1) k_idx_score_umma(const ScoreParams S) {
@@ -468,7 +492,7 @@ __global__ void __launch_bounds__(st_threads(KB), 1) k_idx_score_umma(const Scor
             tmem_ld16(d_addr, r[0]);
             if (KB == 2) tmem_ld16(d_addr + ST_N, e[0]);
             float total = 0.f;
-            int k = 0, left = cpt;
+            int k = 0, left = cpt, redo = 0;
 #pragma unroll
             for (int c = 0; c < ST_N / 16; c++) {
                 tmem_wait_ld();
@@ -487,7 +511,7 @@ __global__ void __launch_bounds__(st_threads(KB), 1) k_idx_score_umma(const Scor
                     auto term = [&](int j, float wj) {
                         float d = __uint_as_float(r[c & 1][4 * i + j]);
                         if (KB == 2) d += __uint_as_float(e[c & 1][4 * i + j]);
-                        total = fmaf(wj, fmaxf(d * S.scale, 0.f), total);
+                        total = fmaf(wj, relu_nan(d * S.scale), total);
                     };
                     term(0, wv.x);
                     term(1, wv.y);
@@ -495,11 +519,18 @@ __global__ void __launch_bounds__(st_threads(KB), 1) k_idx_score_umma(const Scor
                     term(3, wv.w);
                 }
                 if (--left == 0) {  // the query's last chunk
-                    if (ok && k < n_tok && p < (S.pos0 + t0 + k + 1) / S.kpool) S.score[(int64_t) (t0 + k) * S.score_stride + p] = total;
+                    if (ok && k < n_tok && p < (S.pos0 + t0 + k + 1) / S.kpool) {
+                        S.score[(int64_t) (t0 + k) * S.score_stride + p] = total;
+                        if (!(fabsf(total) <= 3.402823466e+38f)) redo |= 1 << k;
+                    }
                     total = 0.f;
                     k++;
                     left = cpt;
                 }
+            }
+            if (redo) {  // (behind the loop: a call inside it would spill the columns in flight)
+                for (k = 0; k < n_tok; k++)
+                    if ((redo >> k) & 1) S.score[(int64_t) (t0 + k) * S.score_stride + p] = score_f32(S, t0 + k, p);
             }
         }
     }

@@ -83,7 +83,10 @@ int gs_idx_pool(const float *kc, const float *gc, float *rk, float *rg, const fl
                 int kpool, void *stream);
 /* Replaces gs_idx_score, ops.cu:675-712 (lib.rs:105-108): score[t][p] = sum_h w[t][h] * relu(scale * q[t][h] . P[p])
  * for the p < (pos0 + t + 1) / kpool complete pools; q f32 [T][Hq][Dk], w f32 [T][Hq], score f32 [T][score_stride].
- * Dk > 128 is rejected as in the reference. */
+ * Dk > 128 is rejected as in the reference.  Sums are f32, or - from five queries on, where the sizes allow - three-way bf16
+ * splits of the f32 values on the tensor cores, at the same precision but with other low bits: a query scored in a call of
+ * four and in one of five may differ there, and with it the choice among pools (nearly) tied at the k-th largest.
+ * Infinite and NaN operands give what the f32 sums give in either form (relu of NaN is 0). */
 int gs_idx_score(const float *q, const float *w, const float *P, float *score, int64_t score_stride, int pos0, int T,
                  int kpool, int Hq, int Dk, float scale, void *stream);
 /* Replaces gs_idx_select, ops.cu:714-791 (lib.rs:109-112).  Query t (position pos0 + t) with n_pool = (pos+1)/kpool

@@ -124,6 +124,46 @@ def test_idx_score_tensor_form_keeps_f32_precision(pkg, cuda, T, pos0, Hq, Dk, k
     assert (np.abs(got - want) / mag).max() <= 1e-6  # of the sum of magnitudes; entries past a query's pools untouched
 
 
+@pytest.mark.parametrize("T,Hq,Dk", [(4, 32, 128), (9, 32, 128), (9, 32, 64), (9, 16, 100)])
+def test_idx_score_values_that_are_not_finite(pkg, cuda, oracle, T, Hq, Dk):
+    """Infinite, NaN and near-maximal queries, keys and weights: what the f32 sums give, on either side of the tensor form's first
+    query count."""
+    rng = np.random.default_rng(T + Dk)
+    pos0, kpool = 1200, 4
+    pools = (pos0 + T) // kpool
+    q = rng.standard_normal((T, Hq, Dk), dtype=np.float32)
+    w = rng.standard_normal((T, Hq), dtype=np.float32)
+    P = rng.standard_normal((pools, Dk), dtype=np.float32)
+    scale = float(1 / np.sqrt(Dk))
+    P[3, 5], P[130, 0], P[131, Dk - 1], P[200] = np.inf, -np.inf, np.nan, 3.4e38
+    q[1, 2, 7], q[2, 0, 0], q[0, 1] = np.inf, np.nan, 1e-30
+    w[T - 1, 3] = np.inf
+    got = _scores(cuda, pkg._lib.load(), q, w, P, pos0, kpool, pools, scale)
+    def fma(a, b, c):  # one rounding (the product is exact in 64 bits): what overflows is decided by the sum
+        return (a.astype(np.float64) * b.astype(np.float64) + c.astype(np.float64)).astype(np.float32)
+
+    with np.errstate(all="ignore"):
+        want = np.full(got.shape, -123.0, np.float32)
+        for t in range(T):
+            n = (pos0 + t + 1) // kpool
+            acc = np.zeros((n, Hq, 4), np.float32)
+            for c in range(0, Dk, 4):
+                acc = fma(q[t][None, :, c:c + 4], P[:n, None, c:c + 4], acc)
+            d = (((acc[..., 0] + acc[..., 1]) + (acc[..., 2] + acc[..., 3])) * np.float32(scale))
+            r = np.where(np.isnan(d), np.float32(0), np.maximum(d, np.float32(0)))  # relu of NaN is 0, as in the reference
+            tot = np.zeros(n, np.float32)
+            for h in range(Hq):
+                tot = fma(w[t, h], r[:, h], tot)
+            want[t, :n] = tot
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    inf = np.isinf(want)
+    assert inf.any() and np.array_equal(got[inf], want[inf])
+    ok = np.isfinite(want)
+    assert np.array_equal(np.isfinite(got), ok)
+    small = ok & (np.abs(want) < 1e30)
+    assert np.abs(got[small] - want[small]).max() <= 1e-3 and np.allclose(got[ok], want[ok], rtol=1e-4, atol=1e-3)
+
+
 def _select(torch, lib, score, pos0, kpool, top_k, sel_stride):
     T, stride = score.shape
     sel = torch.full((T, sel_stride), -1, dtype=torch.int32, device="cuda")
