@@ -97,13 +97,19 @@ constexpr int SC_ROW = SC_C4 * 4 + 4;                   // rows padded by 16 byt
 constexpr int score_smem(int Hq) {
     return (SC_WARPS * (2 * SC_POOLS * SC_ROW + SC_HEADS * SC_POOLS) + Hq * (SC_ROW + 1)) * (int) sizeof(float);
 }
+// The query rows of a launch sit in shared memory; more heads than fit are worked off in launches of this many, each going
+// on with the sums the one before left in `score` (the heads are added in ascending order either way).
+constexpr int SC_MAX_HEADS = 9 * SC_HEADS;
+static_assert(score_smem(SC_MAX_HEADS) <= 232448, "shared memory of one CTA");
 __device__ __forceinline__ void fma_f32x2(uint64_t &d, uint64_t a, uint64_t b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
 
 __global__ void __launch_bounds__(SC_WARPS * 32) k_idx_score(const float *__restrict__ q, const float *__restrict__ w,
                                                              const float *__restrict__ P, float *__restrict__ score,
-                                                             int64_t score_stride, int pos0, int kpool, int Hq, int Dk, float scale) {
+                                                             int64_t score_stride, int pos0, int kpool, int Hq, int Dk, float scale,
+                                                             int Hq_all, int go_on) {
+    // q, w: this launch's Hq of the Hq_all heads of every query; go_on: after the heads in front of them
     extern __shared__ __align__(16) float sc_smem[];
     const int t = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float *sq = sc_smem;                                                             // [Hq][SC_ROW]
@@ -134,9 +140,9 @@ __global__ void __launch_bounds__(SC_WARPS * 32) k_idx_score(const float *__rest
     };
     const int step = gridDim.x * SC_WARPS;
     int tile = blockIdx.x * SC_WARPS + warp;
-    load_rows(sq, q + (int64_t) t * Hq * Dk, Hq, Hq - 1, tid, SC_WARPS * 32);
+    load_rows(sq, q + (int64_t) t * Hq_all * Dk, Hq, Hq - 1, tid, SC_WARPS * 32);
     if (tile < n_tiles) load_tile(tile, 0);
-    for (int i = tid; i < Hq; i += SC_WARPS * 32) sw[i] = w[(int64_t) t * Hq + i];
+    for (int i = tid; i < Hq; i += SC_WARPS * 32) sw[i] = w[(int64_t) t * Hq_all + i];
     sm100::cp_async_wait_all();
     __syncthreads();
     const int pg = lane >> 2, hg = lane & 3;       // pools pg + 8 j, heads hg + 4 i of a pass
@@ -145,7 +151,8 @@ __global__ void __launch_bounds__(SC_WARPS * 32) k_idx_score(const float *__rest
         __syncwarp();
         if (tile + step < n_tiles) load_tile(tile + step, buf ^ 1);
         const float *kt = sk + buf * SC_POOLS * SC_ROW + pg * SC_ROW;
-        float total = 0.f;
+        const int p = tile * SC_POOLS + lane;
+        float total = go_on && p < n_pool ? score[(int64_t) t * score_stride + p] : 0.f;
         for (int h0 = 0; h0 < Hq; h0 += SC_HEADS) {
             const int nh = min(SC_HEADS, Hq - h0);
             uint64_t acc[4][8][2];
@@ -183,7 +190,6 @@ __global__ void __launch_bounds__(SC_WARPS * 32) k_idx_score(const float *__rest
             for (int h = 0; h < nh; h++) total = fmaf(sw[h0 + h], sr[h * SC_POOLS + lane], total);
             __syncwarp();
         }
-        const int p = tile * SC_POOLS + lane;
         if (p < n_pool) score[(int64_t) t * score_stride + p] = total;
     }
 }
@@ -878,10 +884,17 @@ GS_EXPORT int gs_idx_score(const float *q, const float *w, const float *P, float
     }
     const int tiles = (max_pool + SC_POOLS - 1) / SC_POOLS, blocks = (tiles + SC_WARPS - 1) / SC_WARPS, want = (2 * sms + T - 1) / T;
     const dim3 grid(blocks < want ? blocks : want, T);
-    const int smem = score_smem(Hq);
-    GS_TRY(cudaFuncSetAttribute(k_idx_score, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    // attributes are set on every call: a cached flag would go stale across a device reset; always to the same value, since
+    // another thread may be between its own setting and its launch
+    GS_TRY(cudaFuncSetAttribute(k_idx_score, cudaFuncAttributeMaxDynamicSharedMemorySize, score_smem(SC_MAX_HEADS)));
     GS_TRY(cudaFuncSetAttribute(k_idx_score, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    return launch_pdl(k_idx_score, grid, SC_WARPS * 32, smem, (cudaStream_t) stream, q, w, P, score, score_stride, pos0, kpool, Hq, Dk, scale);
+    for (int h0 = 0; h0 < Hq; h0 += SC_MAX_HEADS) {
+        const int nh = Hq - h0 < SC_MAX_HEADS ? Hq - h0 : SC_MAX_HEADS;
+        if (int e = launch_pdl(k_idx_score, grid, SC_WARPS * 32, score_smem(nh), (cudaStream_t) stream, q + (int64_t) h0 * Dk, w + h0, P, score,
+                               score_stride, pos0, kpool, nh, Dk, scale, Hq, h0 > 0 ? 1 : 0))
+            return e;
+    }
+    return 0;
 }
 
 GS_EXPORT int gs_idx_select(const float *score, int64_t score_stride, int pos0, int T, int kpool, int top_k, int *sel,
