@@ -242,6 +242,7 @@ __device__ __forceinline__ bool combine_item_compute(const CombinePlan &C, const
 // one sequence, about n_ctas / n_seq + 1 with several): as many boxes as it needs are fetched.  Segments past the sequence's last one belong to other sequences or lie outside the tensor
 // (zero-filled) and get weight 0.
 constexpr int32_t ST_COMBINE = 1 << 18;  // status bit: the copy of the records did not complete in time
+constexpr int CB_BULK_SMEM = CB_NT * CB_COLS * 4 + 128;  // the largest tile a launch may ask for
 struct CombineBulk {
     CUtensorMap tm;
     CombinePlan c;

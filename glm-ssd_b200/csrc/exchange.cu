@@ -269,7 +269,7 @@ int launch_exchange_combine(CombinePlan c, const gs_shard_exchange &x, float *o,
                                        (uint64_t) c.d_v * 4, (uint64_t) c.seg_stride_acc * 4, CB_COLS, 1, (uint32_t) c.n_ctas))
             return e;
         smem = c.n_ctas * CB_COLS * 4 + 128;
-        GS_TRY(cudaFuncSetAttribute(k_exchange_combine, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        GS_TRY(cudaFuncSetAttribute(k_exchange_combine, cudaFuncAttributeMaxDynamicSharedMemorySize, CB_BULK_SMEM));  // (the most any call needs)
     }
     // blocks of one rank wait for blocks of the others: every block of the grid must be resident
     int per_sm = 0;

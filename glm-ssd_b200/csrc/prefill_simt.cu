@@ -127,12 +127,14 @@ int launch_prefill_simt(const __half *q, const __half *k, const __half *v, void 
     if (d % 8 != 0 || d > DMAX || d <= 0) return fail_invalid("prefill: need d % 8 == 0 and d <= 256");
     if (S <= 0 || H <= 0) return 0;
     const size_t smem = (size_t) BQ * d * 4 + 2 * (size_t) BK * d * 2 + (size_t) BQ * BK * 4;
+    // (the most any call needs: another thread may be between its own setting and its launch)
+    const int smem_max = BQ * DMAX * 4 + 2 * BK * DMAX * 2 + BQ * BK * 4;
     dim3 grid((S + BQ - 1) / BQ, H);
     if (o_f16) {
-        GS_TRY(cudaFuncSetAttribute(k_prefill_simt<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+        GS_TRY(cudaFuncSetAttribute(k_prefill_simt<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
         k_prefill_simt<true><<<grid, PNT, smem, st>>>(q, k, v, o, S, H, d, p0, scale);
     } else {
-        GS_TRY(cudaFuncSetAttribute(k_prefill_simt<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+        GS_TRY(cudaFuncSetAttribute(k_prefill_simt<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
         k_prefill_simt<false><<<grid, PNT, smem, st>>>(q, k, v, o, S, H, d, p0, scale);
     }
     GS_TRY(cudaGetLastError());

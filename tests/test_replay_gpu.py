@@ -148,3 +148,42 @@ def test_prefill_behind_itself_in_a_graph(pkg, cuda):
     torch.cuda.synchronize()
     for o, w in zip(outs, want):
         assert torch.equal(o, w)
+
+
+def test_calls_of_different_sizes_from_several_threads(pkg, cuda):
+    """Two host threads on streams of their own, with calls of the same kernels that need different amounts of shared memory."""
+    import threading
+    torch = cuda
+    n_big, H = 32768, 20
+    cache = (torch.randn((n_big, 576), device="cuda") * 0.5).half()
+    q = torch.randn((1, 1, H, 576), device="cuda").half()
+    qs, ps = torch.randn((3, 96, 64), device="cuda"), torch.randn((500, 64), device="cuda")
+    lens = {n: torch.full((1,), n, dtype=torch.int32, device="cuda") for n in (64, n_big)}
+    want = {n: pkg.mla_decode(q, cache[:n].contiguous(), lens[n], max_seq_len=n) for n in lens}
+    scores = {hq: torch.zeros((3, 500), device="cuda") for hq in (1, 96)}
+    L = pkg._lib.load()
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(n, hq):
+        try:
+            torch.cuda.set_device(0)
+            st = torch.cuda.Stream()
+            with torch.cuda.stream(st):
+                c, ws, out = cache[:n].contiguous(), pkg.new_workspace(1, 1, H), torch.empty((1, 1, H, 512), device="cuda")
+                w = torch.ones((3, hq), device="cuda")
+                for _ in range(1500):
+                    pkg.mla_decode(q, c, lens[n], workspace=ws, out=out, max_seq_len=n)
+                    pkg._lib.check(L.gs_idx_score(qs.data_ptr(), w.data_ptr(), ps.data_ptr(), scores[hq].data_ptr(), 500, 1000, 3, 4, hq, 64, 0.1,
+                                                  st.cuda_stream), "gs_idx_score")
+                st.synchronize()
+            assert pkg.decode_status(ws) == 0 and torch.equal(out, want[n])
+        except Exception as exc:
+            errors.append(exc)
+
+    threads = [threading.Thread(target=work, args=a) for a in ((64, 1), (n_big, 96))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
