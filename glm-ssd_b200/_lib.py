@@ -42,7 +42,21 @@ class DecodeArgs(C.Structure):
 # The bytes of a DecodeArgs from its fields in order (native alignment), in one call.
 _decode_struct = struct.Struct("@PPqPPPiifiPPPqiiiiiiiPiP")
 assert _decode_struct.size == C.sizeof(DecodeArgs)
-pack_decode_args = _decode_struct.pack
+_pack_decode_args = _decode_struct.pack
+
+
+def decode_args(*values) -> bytes:
+    """The bytes of a DecodeArgs.  What the packer refuses - an integer beyond its field, a ctypes handle - is stored field by field,
+    by the rules of ctypes."""
+    try:
+        return _pack_decode_args(*values)
+    except (struct.error, OverflowError, TypeError):
+        a = DecodeArgs()
+        for (name, _), v in zip(DecodeArgs._fields_, values):
+            if name == "exchange":
+                v = C.cast(C.c_void_p(v), C.POINTER(ShardExchange))
+            setattr(a, name, v)
+        return bytes(a)
 
 
 class FusedArgs(C.Structure):

@@ -49,8 +49,8 @@ def _need(t: torch.Tensor, dtype, name: str) -> torch.Tensor:
 
 def mla_attn(q, C_latent, C_scales, sel, sel_stride, cnt, scale, o, part, T, H, R, splits):
     """``gs_mla_attn`` with the reference's argument list (crates/cuda/src/lib.rs:97-100)."""
-    rc = _lib.load().gs_mla_attn(q.data_ptr(), C_latent.data_ptr(), _ptr(C_scales), sel.data_ptr(), sel_stride, cnt.data_ptr(), scale,
-                                 o.data_ptr(), _ptr(part), T, H, R, splits, _stream())
+    rc = _lib.load().gs_mla_attn(_ptr(q), _ptr(C_latent), _ptr(C_scales), _ptr(sel), sel_stride, _ptr(cnt), scale, _ptr(o), _ptr(part), T, H, R,
+                                 splits, _stream())
     if rc:
         _lib.check(rc, "gs_mla_attn")
 
@@ -104,13 +104,13 @@ def mla_decode(q, cache, seq_lens, *, scale=SCALE_256, d_v=512, seq_base=None, p
         workspace = new_workspace(n_seq, T, H, d_v, q.device)
     if want_out and out is None:
         out = torch.empty((n_seq, T, H, d_v), dtype=torch.float32, device=q.device)
-    a = _lib.pack_decode_args(
+    a = _lib.decode_args(
         q.data_ptr(), cache.data_ptr(), cache.shape[0], seq_lens.data_ptr(), 0 if seq_base is None else seq_base.data_ptr(),
         0 if page_table is None else page_table.data_ptr(), 0 if page_table is None else page_table.shape[1], page_rows, scale,
         1 if tail_causal else 0, out.data_ptr() if want_out else 0, 0 if part_out is None else part_out.data_ptr(),
         0 if static_scratch else workspace.data_ptr(), 0 if static_scratch else workspace.numel(),
         n_seq, T, H, d_qk, d_v, max_seq_len, impl,
-        ev_after_main or 0,  # raw cudaEvent_t handle (int) or None
+        ev_after_main or 0,  # raw cudaEvent_t handle (int, ctypes.c_void_p) or None
         1 if no_combine else 0,
         0 if exchange is None else C.addressof(exchange))  # a _lib.ShardExchange kept alive by the caller (see sharded.PeerExchange)
     if static_scratch:

@@ -100,3 +100,32 @@ def test_append_argument_validation(pkg):
     assert L.gs_rope_kv_append_at(None, None, 0, 0, 576, 64, 10000.0, None) == 0
     assert L.gs_prefill_attn(None, None, None, None, 0, 0, 20, 256, 0, 0.0625, 0, None) == 0
     assert L.gs_prefill_attn(None, None, None, None, 0, 8, 20, 256, 0, 0.0625, 0, None) == CUDA_ERROR_INVALID_VALUE
+
+
+def test_wrapper_arguments_the_packer_refuses(pkg, monkeypatch):
+    """decode_args takes what assignment to the ctypes fields takes: handles as c_void_p, integers beyond their field (cut off, as an
+    "unbounded" max_seq_len of sys.maxsize always was)."""
+    import sys
+    _lib = pkg._lib
+    plain = (0x1000, 0x2000, 131072, 0x3000, 0, 0x4000, 512, 64, 0.0625, 1, 0x5000, 0, 0x6000, 1 << 33, 3, 2, 20, 576, 512, 65536, 2, 0x7000, 1, 0x8000)
+
+    def fields(raw):
+        a = _lib.DecodeArgs.from_buffer_copy(raw)
+        return [C.cast(getattr(a, n), C.c_void_p).value if n == "exchange" else getattr(a, n) for n, _ in _lib.DecodeArgs._fields_]
+
+    want = [v if v != 0 or n not in ("seq_base", "part_out") else None for (n, _), v in zip(_lib.DecodeArgs._fields_, plain)]
+    assert fields(_lib.decode_args(*plain)) == want
+    ev = list(plain)
+    ev[21] = C.c_void_p(0x7000)
+    assert _lib.decode_args(*ev) == _lib.decode_args(*plain)
+    big = list(plain)
+    big[19] = sys.maxsize
+    assert fields(_lib.decode_args(*big))[19] == -1
+
+
+def test_wrapper_of_the_reference_entry_point_takes_null_pointers(pkg, monkeypatch):
+    """None is a null pointer: an error code for a call with work, nothing to do for one without."""
+    monkeypatch.setattr(pkg.attn, "_stream", lambda: 0)
+    pkg.mla_attn(None, None, None, None, 0, None, 0.0625, None, None, 0, 64, 512, 1)
+    with pytest.raises(pkg._lib.GsError):
+        pkg.mla_attn(None, None, None, None, 2052, None, 0.0625, None, None, 1, 64, 512, 1)
