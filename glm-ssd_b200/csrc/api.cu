@@ -40,6 +40,40 @@ static WsLayout ws_layout(int n_seq, int T, int H, int d_v) {
     return w;
 }
 
+int cluster_room(int slot, const void *kernel, int threads, int smem, ClusterRoom *out) {
+    static std::atomic<int> known[64][ROOM_SLOTS][kClusterSizes];  // CTAs + 1; zero-initialised: not asked yet
+    int dev = 0;
+    GS_TRY(cudaGetDevice(&dev));
+    out->ctas[0] = 0;
+    for (int i = 1; i < kClusterSizes; i++) {
+        const int v = dev < 64 ? known[dev][slot][i].load(std::memory_order_relaxed) : 0;
+        if (v > 0) {
+            out->ctas[i] = v - 1;
+            continue;
+        }
+        GS_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        GS_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1 << i);
+        cfg.blockDim = dim3(threads);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1 << i;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+            (void) cudaGetLastError();  // a size this device does not take at all
+            n = 0;
+        }
+        out->ctas[i] = n << i;
+        if (dev < 64) known[dev][slot][i].store((n << i) + 1, std::memory_order_relaxed);
+    }
+    return 0;
+}
+
 static int device_sm_count(int *out) {
     int dev = 0;
     GS_TRY(cudaGetDevice(&dev));
@@ -231,9 +265,11 @@ static int prefill_attn(const char *who, const void *q, const void *k, const voi
         set_error("%s: tcgen05 kernel does not take this shape: %s", who, why);
         return (int) cudaErrorInvalidValue;
     }
+    int sms = 0;
+    if (int e = device_sm_count(&sms)) return e;
     if (umma_ok && impl != 1)
         return launch_prefill_umma((const __half *) q, (const __half *) k, (const __half *) v, o, o_f16, S, H, d, p0,
-                                   scale, status, (cudaStream_t) stream);
+                                   scale, status, sms, (cudaStream_t) stream);
     return launch_prefill_simt((const __half *) q, (const __half *) k, (const __half *) v, o, o_f16, S, H, d, p0, scale,
                                (cudaStream_t) stream);
 }

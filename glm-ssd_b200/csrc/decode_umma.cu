@@ -1329,7 +1329,8 @@ struct ListPlan {
 // scan).  The choice it makes is within about 6 % of the best cut measured.
 // Clusters and the combine store o in 16-byte words; an o that is not aligned for them (`o_aligned`) leaves one CTA per sequence,
 // which stores single words.
-static ListPlan list_plan(int T, int H, int R, int sel_stride, int splits, const float *part, bool o_aligned, bool q8, int grid_max) {
+static ListPlan list_plan(int T, int H, int R, int sel_stride, int splits, const float *part, bool o_aligned, bool q8, int grid_max,
+                          const ClusterRoom &room) {
     ListPlan best{0, 0, 1, true, 1e30f};
     auto offer = [&](int n, int64_t grid, int cluster, bool whole, float cost) {
         if (cost < best.cost) best = ListPlan{n, (int) grid, cluster, whole, cost};
@@ -1343,10 +1344,9 @@ static ListPlan list_plan(int T, int H, int R, int sel_stride, int splits, const
         const float t_cl = (Hg <= 32 ? 2.5f : Hg <= 48 ? 2.8f : 3.1f) + (q8 ? 0.2f : 0.f);
         const int64_t grid = n_seq_k < grid_max ? n_seq_k : grid_max;
         offer(n, grid, 1, true, (float) ((n_seq_k + grid - 1) / grid * tiles_seq) * t_one + 2.f);
-        for (int c = 2; o_aligned && c <= MAX_CLUSTER; c *= 2) {
-            // CTAs of clusters of c that run at once on 148 SMs, one per SM
-            const int resident = c == 2 ? 148 : c == 4 ? 132 : c == 8 ? 120 : 112;
-            if (n_seq_k * c > (resident < grid_max ? resident : grid_max)) break;
+        for (int c = 2, i = 1; o_aligned && c <= MAX_CLUSTER; c *= 2, i++) {
+            // all clusters have to run at once (148 SMs: 148, 132, 120 and 112 CTAs in clusters of 2, 4, 8 and 16)
+            if (n_seq_k * c > (room.ctas[i] < grid_max ? room.ctas[i] : grid_max)) continue;
             const int64_t per = (sel_stride + c - 1) / c;
             offer(n, n_seq_k * c, c, true, (float) ((per + TILE - 1) / TILE) * t_cl + (Hg <= 48 ? 6.5f + 0.03f * (float) Hg : 17.f) +
                                                (c == 16 ? 2.5f : 0.f) + (q8 ? 2.f : 0.f) + 0.03f * (float) (n_seq_k * c));
@@ -1376,7 +1376,9 @@ int launch_decode_umma_list(const float *q, const void *C, const __half *C_scale
     if ((reinterpret_cast<uintptr_t>(C) & 15) || (reinterpret_cast<uintptr_t>(q) & 15) || (reinterpret_cast<uintptr_t>(C_scales) & 15)) return -1;
     int grid_max = sm_count < kMaxCtas ? sm_count : kMaxCtas;
     if (grid_max < 1) grid_max = 1;
-    const ListPlan L = list_plan(T, H, R, sel_stride, splits, part, !(reinterpret_cast<uintptr_t>(o) & 15), C_scales != nullptr, grid_max);
+    ClusterRoom room;  // (one CTA per SM in every form)
+    if (int e = cluster_room(ROOM_LIST, (const void *) k_decode_umma<64, 8, true, true>, LIST_NTHREADS, Smem<64, 8>::TOTAL, &room)) return e;
+    const ListPlan L = list_plan(T, H, R, sel_stride, splits, part, !(reinterpret_cast<uintptr_t>(o) & 15), C_scales != nullptr, grid_max, room);
     if (L.n_groups == 0) return -1;
     const int n_groups = L.n_groups;
     const int64_t n_seq_k = (int64_t) T * n_groups;

@@ -83,7 +83,17 @@ int launch_prefill_simt(const __half *q, const __half *k, const __half *v, void 
                         int p0, float scale, cudaStream_t st);
 bool prefill_umma_supported(int S, int H, int d, int p0, const char **why);
 int launch_prefill_umma(const __half *q, const __half *k, const __half *v, void *o, int o_f16, int S, int H, int d,
-                        int p0, float scale, int32_t *status, cudaStream_t st);
+                        int p0, float scale, int32_t *status, int sm_count, cudaStream_t st);
+
+// CTAs of clusters of 2, 4, 8 and 16 that run at once on the current device, one CTA per SM (index: log2 of the size; 0 where a
+// cluster of that size does not fit at all).  A property of the board - GPCs differ in their number of SMs - asked once per
+// device and kernel form (`slot`) and kept; racing first calls store the same values.
+constexpr int kClusterSizes = 5;
+struct ClusterRoom {
+    int ctas[kClusterSizes];
+};
+enum { ROOM_LIST = 0, ROOM_PREFILL = 1, ROOM_SLOTS = 2 };
+int cluster_room(int slot, const void *kernel, int threads, int smem, ClusterRoom *out);
 
 // Launch as a programmatic dependent of the kernel in front in the stream: the grid may be scheduled once every block of
 // that kernel has passed its launch_dependents (or ended), and waits for its results inside (griddepcontrol.wait before

@@ -494,33 +494,32 @@ __global__ void __launch_bounds__(PF_THREADS, 1) k_prefill_umma(const __grid_con
 struct PrefillPlan {
     int whole, cluster;
 };
-// A CTA takes an item from its first key tile to its last, and with one CTA per SM the items run in rounds of 148: a chunk
+// A CTA takes an item from its first key tile to its last, and with one CTA per SM the items run in rounds of (here) 148: a chunk
 // of 1000 tokens behind 7168 (160 items of 113 to 128 tiles) left 136 SMs idle for half its time, one of 128 tokens 128 of
 // them for all of it.  So when the items do not fill whole rounds, the last ones are split.  Estimated in key tiles (0.65 us);
 // a split item costs 18 tiles and more besides its share (its own start, the exchange and the sum; measured 11 us from 2 to 4
 // CTAs, 15 with 8, over 20 with 16).  Measured, whole / chosen: 1000 tokens behind 7168 188 / 135 us, 32 behind 4096 51 / 32 us,
 // 128 behind 32000 352 / 130 us (5 TB/s of keys and values), 900 behind 20000 482 / 332 us.
 constexpr int split_cost(int c) { return c <= 4 ? 18 : c == 8 ? 24 : 34; }
-static PrefillPlan prefill_plan(int S, int H, int p0) {
-    constexpr int SMS = 148;
+static PrefillPlan prefill_plan(int S, int H, int p0, int sms, const ClusterRoom &room) {
     const int nb = (S + BM - 1) / BM;
     const int64_t items = (int64_t) nb * H;
     // From five rounds on the last round is at most a few per cent.
-    if (items > 5 * SMS) return PrefillPlan{(int) items, 1};
+    if (items > 5 * sms) return PrefillPlan{(int) items, 1};
     auto tiles_of = [&](int64_t i) {
         const int qb = nb - 1 - (int) (i % nb);
         const int end = p0 + (S < (qb + 1) * BM ? S : (qb + 1) * BM);
         return (end + BN - 1) / BN;
     };
-    // when the SM that is free first has finished, items handed out in order: a heap of 148 finishing times
-    int busy[SMS] = {0};
+    // when the SM that is free first has finished, items handed out in order: a heap of the SMs' finishing times
+    int busy[kMaxCtas] = {0};
     auto give = [&](int t) {
         int i = 0;
         const int v = busy[0] + t;
         for (;;) {
             int c = 2 * i + 1;
-            if (c >= SMS) break;
-            if (c + 1 < SMS && busy[c + 1] < busy[c]) c++;
+            if (c >= sms) break;
+            if (c + 1 < sms && busy[c + 1] < busy[c]) c++;
             if (busy[c] >= v) break;
             busy[i] = busy[c];
             i = c;
@@ -529,13 +528,13 @@ static PrefillPlan prefill_plan(int S, int H, int p0) {
     };
     auto latest = [&]() {
         int m = 0;
-        for (int i = 0; i < SMS; i++) m = busy[i] > m ? busy[i] : m;
+        for (int i = 0; i < sms; i++) m = busy[i] > m ? busy[i] : m;
         return m;
     };
     PrefillPlan best{(int) items, 1};
-    const int64_t rounds = items / SMS;
+    const int64_t rounds = items / sms;
     int64_t at = 0;
-    for (; at < rounds * SMS; at++) give(tiles_of(at));
+    for (; at < rounds * sms; at++) give(tiles_of(at));
     const int done = latest();          // the full rounds
     int most = 0;
     for (int64_t i = at; i < items; i++) {
@@ -545,8 +544,9 @@ static PrefillPlan prefill_plan(int S, int H, int p0) {
     }
     int cost = latest();
     const int64_t rest = items - at;
-    for (int c = 2; rest > 0 && c <= PF_MAX_CLUSTER; c *= 2) {
-        const int resident = c == 2 ? 74 : c == 4 ? 33 : c == 8 ? 15 : 7;  // clusters that run at once, one CTA per SM
+    for (int c = 2, i = 1; rest > 0 && c <= PF_MAX_CLUSTER; c *= 2, i++) {
+        const int resident = room.ctas[i] / c;  // clusters that run at once, one CTA per SM (148 SMs: 74, 33, 15, 7)
+        if (resident < 1) continue;
         const int64_t turns = (rest + resident - 1) / resident;
         const int64_t t = done + turns * ((most + c - 1) / c + split_cost(c));
         if (t < cost) {
@@ -565,7 +565,7 @@ bool prefill_umma_supported(int S, int H, int d, int p0, const char **why) {
 }
 
 int launch_prefill_umma(const __half *q, const __half *k, const __half *v, void *o, int o_f16, int S, int H, int d,
-                        int p0, float scale, int32_t *status, cudaStream_t st) {
+                        int p0, float scale, int32_t *status, int sm_count, cudaStream_t st) {
     if (!(scale > 0.f)) return fail_invalid("prefill: the tcgen05 kernel needs a positive softmax scale");
     if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
          reinterpret_cast<uintptr_t>(o)) & 15)
@@ -585,7 +585,9 @@ int launch_prefill_umma(const __half *q, const __half *k, const __half *v, void 
     P.scale_log2 = scale * 1.4426950408889634f;
     P.status = status;  // may be nullptr: a wait that gives up is then not reported
     P.n_blocks = (S + BM - 1) / BM;
-    const PrefillPlan plan = prefill_plan(S, H, p0);
+    ClusterRoom room;
+    if (int e = cluster_room(ROOM_PREFILL, (const void *) k_prefill_umma<true>, PF_THREADS, PF_SMEM, &room)) return e;
+    const PrefillPlan plan = prefill_plan(S, H, p0, sm_count < kMaxCtas ? sm_count : kMaxCtas, room);
     if (plan.whole > 0) {
         GS_TRY(cudaFuncSetAttribute(k_prefill_umma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM));
         if (int e = launch_pdl(k_prefill_umma<false>, dim3(plan.whole), PF_THREADS, PF_SMEM, st, P)) return e;

@@ -187,3 +187,38 @@ def test_calls_of_different_sizes_from_several_threads(pkg, cuda):
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+def test_first_calls_of_a_process_inside_a_capture(cuda):
+    """Lists in clusters and split prefill items ask the device how many clusters it holds: also when a capture is the first to ask."""
+    import os
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+    code = """
+import importlib, torch
+pkg = importlib.import_module("glm-ssd_b200")
+T, H, n = 2, 64, 2052
+q, c = torch.randn((T, H, 512), device="cuda"), torch.randn((4000, 512), device="cuda").half()
+sel = torch.arange(n, device="cuda").repeat(T, 1).int().contiguous()
+cnt, o = torch.full((T,), n, dtype=torch.int32, device="cuda"), torch.zeros((T, H, 512), device="cuda")
+Q, K, V = (torch.randn((s, 20, 256), device="cuda").half() for s in (100, 3100, 3100))
+O = torch.zeros((100, 20, 256), device="cuda")
+def calls():
+    pkg.mla_attn(q, c, None, sel, n, cnt, 1 / 16, o, None, T, H, 512, 1)
+    pkg.prefill_attn(Q, K, V, p0=3000, out=O)
+s, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+s.wait_stream(torch.cuda.current_stream())
+with torch.cuda.stream(s):
+    with torch.cuda.graph(g, stream=s):
+        calls()
+torch.cuda.synchronize()
+g.replay()
+torch.cuda.synchronize()
+a, b = o.clone(), O.clone()
+calls()
+torch.cuda.synchronize()
+assert pkg.mla_attn_status() == 0 and torch.equal(a, o) and torch.equal(b, O) and a.abs().max() > 0 and b.abs().max() > 0
+"""
+    subprocess.run([sys.executable, "-c", code], cwd=ROOT, check=True, timeout=120)
