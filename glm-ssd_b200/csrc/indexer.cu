@@ -105,11 +105,12 @@ __device__ __forceinline__ void fma_f32x2(uint64_t &d, uint64_t a, uint64_t b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
 
+// q, w: this launch's Hq of the Hq_all heads of every query; GO_ON: after the heads in front of them
+template <bool GO_ON>
 __global__ void __launch_bounds__(SC_WARPS * 32) k_idx_score(const float *__restrict__ q, const float *__restrict__ w,
                                                              const float *__restrict__ P, float *__restrict__ score,
                                                              int64_t score_stride, int pos0, int kpool, int Hq, int Dk, float scale,
-                                                             int Hq_all, int go_on) {
-    // q, w: this launch's Hq of the Hq_all heads of every query; go_on: after the heads in front of them
+                                                             int Hq_all) {
     extern __shared__ __align__(16) float sc_smem[];
     const int t = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float *sq = sc_smem;                                                             // [Hq][SC_ROW]
@@ -151,8 +152,8 @@ __global__ void __launch_bounds__(SC_WARPS * 32) k_idx_score(const float *__rest
         __syncwarp();
         if (tile + step < n_tiles) load_tile(tile + step, buf ^ 1);
         const float *kt = sk + buf * SC_POOLS * SC_ROW + pg * SC_ROW;
-        const int p = tile * SC_POOLS + lane;
-        float total = go_on && p < n_pool ? score[(int64_t) t * score_stride + p] : 0.f;
+        float total = 0.f;
+        if (GO_ON && tile * SC_POOLS + lane < n_pool) total = score[(int64_t) t * score_stride + tile * SC_POOLS + lane];
         for (int h0 = 0; h0 < Hq; h0 += SC_HEADS) {
             const int nh = min(SC_HEADS, Hq - h0);
             uint64_t acc[4][8][2];
@@ -190,8 +191,44 @@ __global__ void __launch_bounds__(SC_WARPS * 32) k_idx_score(const float *__rest
             for (int h = 0; h < nh; h++) total = fmaf(sw[h0 + h], sr[h * SC_POOLS + lane], total);
             __syncwarp();
         }
+        const int p = tile * SC_POOLS + lane;
         if (p < n_pool) score[(int64_t) t * score_stride + p] = total;
     }
+}
+
+// Up to three heads (from 16 queries on, four): a key is used so little that staging it costs more than it saves.  Block = 64 pools x 4 column parts; thread
+// (pool, part) holds columns part, part + 4, ... of its pool's key in registers and joins the parts by two shuffles: the same
+// sums.  (One head x 128 columns, 64 queries x 8192 pools: 74 us this way, 230 with the register tiles; four heads
+// x 64 columns 93 / 107 us, of one query 5.4 / 5.1.)
+constexpr int SF_POOLS = 64, SF_PARTS = 4, SF_MAXI = 32, SF_HEADS = 4;  // Dk <= SF_PARTS * SF_MAXI
+__global__ void __launch_bounds__(SF_POOLS * SF_PARTS) k_idx_score_few(const float *__restrict__ q, const float *__restrict__ w,
+                                                                      const float *__restrict__ P, float *__restrict__ score,
+                                                                      int64_t score_stride, int pos0, int kpool, int Hq, int Dk, float scale) {
+    __shared__ float sq[SF_HEADS * SF_PARTS * SF_MAXI], sw[SF_HEADS];
+    const int t = blockIdx.y, n_pool = (pos0 + t + 1) / kpool, p_base = blockIdx.x * SF_POOLS;
+    sm100::griddep_wait();
+    sm100::griddep_launch_dependents();
+    if (p_base >= n_pool) return;
+    const float *qt = q + (int64_t) t * Hq * Dk;
+    for (int i = threadIdx.x; i < Hq * Dk; i += SF_POOLS * SF_PARTS) sq[i] = qt[i];
+    if (threadIdx.x < Hq) sw[threadIdx.x] = w[(int64_t) t * Hq + threadIdx.x];
+    const int part = threadIdx.x & (SF_PARTS - 1), p = p_base + threadIdx.x / SF_PARTS;
+    const float *pk = P + (int64_t) min(p, n_pool - 1) * Dk;  // (pools past the end work on a valid row and drop the result)
+    float key[SF_MAXI];
+#pragma unroll
+    for (int i = 0; i < SF_MAXI; i++) key[i] = i * SF_PARTS + part < Dk ? pk[i * SF_PARTS + part] : 0.f;
+    __syncthreads();
+    float total = 0.f;
+    for (int h = 0; h < Hq; h++) {
+        float d = 0.f;
+#pragma unroll
+        for (int i = 0; i < SF_MAXI; i++)
+            if (i * SF_PARTS < Dk) d = fmaf(i * SF_PARTS + part < Dk ? sq[h * Dk + i * SF_PARTS + part] : 0.f, key[i], d);
+        d += __shfl_xor_sync(0xffffffffu, d, 1);
+        d += __shfl_xor_sync(0xffffffffu, d, 2);
+        total = fmaf(sw[h], fmaxf(d * scale, 0.f), total);
+    }
+    if (part == 0 && p < n_pool) score[(int64_t) t * score_stride + p] = total;
 }
 
 // ---- scores of a prefill block on the tensor cores ----------------------------------------------------------
@@ -882,16 +919,22 @@ GS_EXPORT int gs_idx_score(const float *q, const float *w, const float *P, float
             return Dk <= 64 ? launch_score_umma<1>(S, sms, (cudaStream_t) stream) : launch_score_umma<2>(S, sms, (cudaStream_t) stream);
         }
     }
-    const int tiles = (max_pool + SC_POOLS - 1) / SC_POOLS, blocks = (tiles + SC_WARPS - 1) / SC_WARPS, want = (2 * sms + T - 1) / T;
+    if (Hq < SF_HEADS || (Hq == SF_HEADS && T >= 16))
+        return launch_pdl(k_idx_score_few, dim3((max_pool + SF_POOLS - 1) / SF_POOLS, T), SF_POOLS * SF_PARTS, 0, (cudaStream_t) stream, q, w, P, score,
+                          score_stride, pos0, kpool, Hq, Dk, scale);
+    // two blocks fit an SM: no more than they hold at once (one block over and a second, nearly empty round doubles the time:
+    // 16 queries x 8192 pools x 8 heads 73 us with 304 blocks, 39 with 288)
+    const int tiles = (max_pool + SC_POOLS - 1) / SC_POOLS, blocks = (tiles + SC_WARPS - 1) / SC_WARPS, want = 2 * sms > T ? 2 * sms / T : 1;
     const dim3 grid(blocks < want ? blocks : want, T);
     // attributes are set on every call: a cached flag would go stale across a device reset; always to the same value, since
     // another thread may be between its own setting and its launch
-    GS_TRY(cudaFuncSetAttribute(k_idx_score, cudaFuncAttributeMaxDynamicSharedMemorySize, score_smem(SC_MAX_HEADS)));
-    GS_TRY(cudaFuncSetAttribute(k_idx_score, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     for (int h0 = 0; h0 < Hq; h0 += SC_MAX_HEADS) {
         const int nh = Hq - h0 < SC_MAX_HEADS ? Hq - h0 : SC_MAX_HEADS;
-        if (int e = launch_pdl(k_idx_score, grid, SC_WARPS * 32, score_smem(nh), (cudaStream_t) stream, q + (int64_t) h0 * Dk, w + h0, P, score,
-                               score_stride, pos0, kpool, nh, Dk, scale, Hq, h0 > 0 ? 1 : 0))
+        auto kernel = h0 > 0 ? k_idx_score<true> : k_idx_score<false>;
+        GS_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, score_smem(SC_MAX_HEADS)));
+        GS_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+        if (int e = launch_pdl(kernel, grid, SC_WARPS * 32, score_smem(nh), (cudaStream_t) stream, q + (int64_t) h0 * Dk, w + h0, P, score,
+                               score_stride, pos0, kpool, nh, Dk, scale, Hq))
             return e;
     }
     return 0;

@@ -77,6 +77,8 @@ def _scores(torch, lib, q, w, P, pos0, kpool, stride, scale):
 
 @pytest.mark.parametrize("T,pos0,Hq,Dk,kpool", [(1, 4099, 32, 128, 4), (2, 700, 8, 128, 4), (256, 1000, 16, 64, 4), (3, 17, 4, 100, 8),
                                                  (1, 2, 8, 128, 4),
+                                                 # few heads: a block per 64 pools up to three (four from 16 queries on), register tiles above
+                                                 (7, 511, 1, 128, 4), (1, 256, 3, 77, 1), (16, 900, 4, 128, 4), (15, 900, 4, 128, 4), (33, 2000, 2, 4, 16),
                                                  # as many heads as 48 KB of query hold: more than one launch can stage
                                                  (1, 400, 288, 40, 4), (6, 400, 300, 32, 4), (2, 300, 1000, 11, 4), (1, 130, 6144, 1, 4)])
 def test_idx_score_vs_oracle_and_reference(pkg, cuda, oracle, T, pos0, Hq, Dk, kpool):
