@@ -200,7 +200,7 @@ def test_length_beyond_the_cache_is_taken_as_the_cache_size(pkg, cuda, oracle, T
 
 
 @pytest.mark.parametrize("T", [1, 2])
-@pytest.mark.parametrize("n", [74 * 64, 74 * 64 + 1, 75 * 64, 148 * 64, 148 * 64 + 1, 149 * 64 + 15, 296 * 64, 297 * 64 + 63])
+@pytest.mark.parametrize("n", [1, 16, 17, 63, 64, 65, 74 * 64, 74 * 64 + 1, 75 * 64, 148 * 64, 148 * 64 + 1, 149 * 64 + 15, 296 * 64, 297 * 64 + 63])
 def test_one_sequence_runs_of_whole_tiles(pkg, cuda, oracle, T, n):
     """Lengths around which the run of tiles per CTA, or the number of CTAs launched, changes; the bound exact, loose and unset."""
     q, cache = make_decode_inputs(n, 1, T, 20, n + 5)
@@ -211,3 +211,21 @@ def test_one_sequence_runs_of_whole_tiles(pkg, cuda, oracle, T, n):
         got = pkg.mla_decode(qd, cd, ld, max_seq_len=bound)
         cuda.cuda.synchronize()
         check_close(got.cpu().numpy(), want, f"n={n} T={T} bound={bound}")
+
+
+@pytest.mark.parametrize("lens,T,H", [
+    ([9000, 9000], 1, 20),                  # two sequences of 74 and more segments: one round of the merge
+    ([19000, 64, 1], 2, 20),                # one with nearly all of them, three blocks per SM
+    ([12000, 3, 500, 700, 2], 2, 20),       # more segments than its tile holds: further rounds
+    ([9000, 100, 9000, 4000], 1, 16),
+])
+def test_merge_of_few_sequences_with_many_segments(pkg, cuda, oracle, lens, T, H):
+    rng = np.random.default_rng(len(lens) + T)
+    lens = np.array(lens, np.int32)
+    pool, pt = paged_layout(rng, lens)
+    q = rng.standard_normal((len(lens), T, H, 576), dtype=np.float32).astype(np.float16)
+    ws = pkg.new_workspace(len(lens), T, H)
+    o = pkg.mla_decode(to_dev(cuda, q), to_dev(cuda, pool), to_dev(cuda, lens), page_table=to_dev(cuda, pt), workspace=ws, impl=2)
+    cuda.cuda.synchronize()
+    assert pkg.decode_status(ws) == 0
+    check_close(o.cpu().numpy(), oracle.mla_decode(q, np.nan_to_num(pool, nan=0.0), lens, 1 / 16, page_table=pt), "merge of few sequences")
