@@ -63,7 +63,9 @@ __global__ void __launch_bounds__(128) k_idx_pool(const float *__restrict__ kc, 
                 acc = fmaf(e, k[m], acc);
             }
         } else {
+#pragma unroll 4
             for (int m = 0; m < kpool; m++) mx = fmaxf(mx, idx_row(gc, rg, j * kpool + m, p0, Dk, kpool)[c] + ape[m * Dk + c]);
+#pragma unroll 4
             for (int m = 0; m < kpool; m++) {
                 const int64_t pos = j * kpool + m;
                 const float e = expf(idx_row(gc, rg, pos, p0, Dk, kpool)[c] + ape[m * Dk + c] - mx);
