@@ -603,8 +603,8 @@ __device__ __forceinline__ uint32_t f2ord(float f) {
 // k-th largest value lies in; the values of that bin (about 2 % of them) go to a list, from which further digits of 10 bits
 // are taken (from all values when it does not fit) until it is short enough for every value in it to count the larger and
 // the equal ones.  Then one ordered pass writes the list of positions: ballots of "greater" and "equal" flags of 32
-// consecutive pools each, one scan over the counts, and a thread per ballot writes the pools it holds - the pools appear in
-// ascending index and ties go to the lowest indices.
+// consecutive pools each, one scan over the counts, and a thread per ballot (a warp when they are few) writes the pools it
+// holds - the pools appear in ascending index and ties go to the lowest indices.
 // Latency-bound (32 KB of scores at 32K positions): what counts is the number of passes and barriers and the chains within
 // them.  The image is kept in shared memory when it fits, so memory is read once, eight loads in flight per thread; the
 // first digit is wide because eight bits of a float are little more than its sign and exponent - nearly all values then
@@ -616,12 +616,14 @@ constexpr int SEL_CACHE = 36864;          // scores of a query kept in shared me
 constexpr int SEL_LIST = 2048;            // values of the k-th largest value's bin kept in a list
 constexpr int SEL_RANK = 128;             // a list up to this long is ranked value by value (all against all), longer ones take a digit first
 constexpr int SEL_SLAB = 4 * SEL_NT;      // groups of 32 pools the ordered pass takes at once
+constexpr int SEL_WIDE = 64;              // with no more groups than this in a slab, a warp writes a group
 struct SelSmem {
     union {
         alignas(16) uint32_t hist[SEL_BINS];
         uint2 flags[SEL_SLAB];            // ordered pass: ballots of "greater" and "equal"
     };
     alignas(16) uint32_t list[SEL_LIST];
+    uint2 base[SEL_WIDE];                 // greater and equal values in front of a group
     uint32_t wsum[2][32];
     uint32_t digit, need, n_list;
 };
@@ -832,7 +834,24 @@ __global__ void __launch_bounds__(SEL_NT) k_idx_select(const float *__restrict__
             const uint32_t wg = warp_scan(lane < SEL_NW ? S.wsum[0][lane] : 0u, lane), we = warp_scan(lane < SEL_NW ? S.wsum[1][lane] : 0u, lane);
             const uint32_t pg = __shfl_sync(0xffffffffu, wg, warp > 0 ? warp - 1 : 0), pe = __shfl_sync(0xffffffffu, we, warp > 0 ? warp - 1 : 0);
             uint32_t gt = run_gt + (warp > 0 ? pg : 0u) + ig - __popc(f.x), eq = run_eq + (warp > 0 ? pe : 0u) + ie - __popc(f.y);
-            for (uint32_t m = f.x | f.y; m; m &= m - 1) {
+            if (groups <= SEL_WIDE) {
+                // few groups: every thread would write the pools of its group one by one (512 of 600: 27 each); a warp takes a
+                // group instead, a lane per pool
+                if (tid < SEL_WIDE) S.base[tid] = make_uint2(gt, eq);
+                __syncthreads();
+                for (int g = warp; g < groups; g += SEL_NW) {
+                    const uint2 m = S.flags[g], b = S.base[g];
+                    const uint32_t below = (1u << lane) - 1;
+                    const bool is_gt = (m.x >> lane) & 1, is_eq = (m.y >> lane) & 1;
+                    const uint32_t e = b.y + __popc(m.y & below);
+                    if (is_gt || (is_eq && e < need_eq)) {
+                        const int64_t slot = (int64_t) (b.x + __popc(m.x & below) + min(e, need_eq)) * kpool;
+                        const int first = (slab + g * 32 + lane) * kpool;
+                        if (vec4) *reinterpret_cast<int4 *>(out + slot) = make_int4(first, first + 1, first + 2, first + 3);
+                        else for (int i = 0; i < kpool; i++) out[slot + i] = first + i;
+                    }
+                }
+            } else for (uint32_t m = f.x | f.y; m; m &= m - 1) {
                 const int b = __ffs(m) - 1;
                 const bool is_gt = (f.x >> b) & 1;
                 if (is_gt || eq < need_eq) {

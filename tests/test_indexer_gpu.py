@@ -187,6 +187,10 @@ def _select(torch, lib, score, pos0, kpool, top_k, sel_stride):
     (3, 4097, 4, 512, True),      # many equal scores, also at the k-th largest: ties go to the lowest indices
     (4, 1000, 16, 7, True),
     (2, 131070, 4, 512, False),   # 128K context
+    (5, 2049, 4, 512, True),      # just beyond top_k: nearly every pool is taken
+    (3, 8190, 4, 512, True),      # around 64 groups of 32 pools: a warp per group up to there, a thread per group beyond
+    (2, 8193, 4, 2047, False),
+    (2, 700, 1, 600, True),
     (2, 170000, 4, 512, False),   # more scores than are kept in shared memory
     (1, 600000, 4, 2000, True),   # more than one slab of the ordered pass, ties across slabs
     (3, 50, 4, 0, False),         # top_k = 0: only the incomplete tail is attended
