@@ -52,33 +52,56 @@ __global__ void k_f32_to_f16_scalar(const float *__restrict__ x, __half *__restr
     if (i < n) y[i] = __float2half_rn(x[i]);
 }
 
-__global__ void k_f32_to_f16_rows(const float *__restrict__ x, __half *__restrict__ y, int64_t n) {
-    // two values per thread, 4-byte stores
+// Two values per access, U accesses in flight per thread.  U = 1 spreads a decode step's rows over the most blocks; in long
+// runs the dependency wait, which every block pays, has to be shared by more work (16.8 M values: 23.7 us without the wait,
+// 34.9 with it at U = 1).
+constexpr int CVT_NT = 256, CVT_U = 8;
+constexpr int64_t CVT_LONG = 1 << 20;  // values from which on U = 8 is used
+template <int U>
+__global__ void __launch_bounds__(CVT_NT) k_f32_to_f16_rows(const float *__restrict__ x, __half *__restrict__ y, int64_t n) {
     sm100::griddep_wait();
     sm100::griddep_launch_dependents();
-    const int64_t i = ((int64_t) blockIdx.x * blockDim.x + threadIdx.x) * 2;
-    if (i + 1 < n) {
-        const float2 v = *reinterpret_cast<const float2 *>(x + i);
-        *reinterpret_cast<__half2 *>(y + i) = __floats2half2_rn(v.x, v.y);
-    } else if (i < n) {
-        y[i] = __float2half_rn(x[i]);
+    const int64_t i0 = ((int64_t) blockIdx.x * (CVT_NT * U) + threadIdx.x) * 2;
+    float2 v[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int64_t i = i0 + (int64_t) u * CVT_NT * 2;
+        v[u] = make_float2(0.f, 0.f);
+        if (i + 1 < n) v[u] = *reinterpret_cast<const float2 *>(x + i);
+        else if (i < n) v[u].x = x[i];
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int64_t i = i0 + (int64_t) u * CVT_NT * 2;
+        if (i + 1 < n) *reinterpret_cast<__half2 *>(y + i) = __floats2half2_rn(v[u].x, v[u].y);
+        else if (i < n) y[i] = __float2half_rn(v[u].x);
     }
 }
 
 // Q8 latent rows: per block of 32 values d = amax / 127, q = round-to-nearest-even(x / d), d kept as f16.
-// One warp per block.  (Exact division and reciprocal: this file is not built with fast-math.)
-__global__ void k_quant_q8(const float *__restrict__ x, int8_t *__restrict__ q, __half *__restrict__ d, int64_t n_blocks) {
-    const int64_t b = (int64_t) blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+// One warp per block of 32, U of them in turn.  (Exact division and reciprocal: this file is not built with fast-math.)
+template <int U>
+__global__ void __launch_bounds__(CVT_NT) k_quant_q8(const float *__restrict__ x, int8_t *__restrict__ q, __half *__restrict__ d, int64_t n_blocks) {
+    const int64_t b0 = (int64_t) blockIdx.x * (CVT_NT / 32 * U) + threadIdx.x / 32;
     const int lane = threadIdx.x & 31;
     sm100::griddep_wait();
     sm100::griddep_launch_dependents();
-    if (b >= n_blocks) return;
-    const float v = x[b * 32 + lane];
-    const float amax = warp_max(fabsf(v));
-    const float dd = __fdiv_rn(amax, 127.f);
-    const float inv = dd > 0.f ? __fdiv_rn(1.f, dd) : 0.f;
-    q[b * 32 + lane] = (int8_t) __float2int_rn(__fmul_rn(v, inv));
-    if (lane == 0) d[b] = __float2half_rn(dd);
+    float v[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int64_t b = b0 + u * (CVT_NT / 32);
+        v[u] = b < n_blocks ? x[b * 32 + lane] : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const int64_t b = b0 + u * (CVT_NT / 32);
+        if (b >= n_blocks) return;
+        const float amax = warp_max(fabsf(v[u]));
+        const float dd = __fdiv_rn(amax, 127.f);
+        const float inv = dd > 0.f ? __fdiv_rn(1.f, dd) : 0.f;
+        q[b * 32 + lane] = (int8_t) __float2int_rn(__fmul_rn(v[u], inv));
+        if (lane == 0) d[b] = __float2half_rn(dd);
+    }
 }
 
 struct AppendParams {
@@ -323,14 +346,21 @@ GS_EXPORT int gs_f32_to_f16(const float *x, void *y, int64_t n, void *stream) {
         return launch_pdl(k_f32_to_f16_scalar, dim3((unsigned) ((n + 255) / 256)), 256, 0, (cudaStream_t) stream, x, (__half *) y, n);
     }
     const int64_t pairs = (n + 1) / 2;
-    return launch_pdl(k_f32_to_f16_rows, dim3((unsigned) ((pairs + 255) / 256)), 256, 0, (cudaStream_t) stream, x, (__half *) y, n);
+    if (n >= CVT_LONG)
+        return launch_pdl(k_f32_to_f16_rows<CVT_U>, dim3((unsigned) ((pairs + CVT_NT * CVT_U - 1) / (CVT_NT * CVT_U))), CVT_NT, 0,
+                          (cudaStream_t) stream, x, (__half *) y, n);
+    return launch_pdl(k_f32_to_f16_rows<1>, dim3((unsigned) ((pairs + CVT_NT - 1) / CVT_NT)), CVT_NT, 0, (cudaStream_t) stream, x, (__half *) y, n);
 }
 
 GS_EXPORT int gs_quant_q8_rows(const float *x, void *q, void *d, int64_t n, void *stream) {
     if (n % 32 != 0) return fail_invalid("gs_quant_q8_rows: n must be a multiple of 32");  // ops.cu:612
     const int64_t nb = n / 32;
     if (nb <= 0) return 0;
-    return launch_pdl(k_quant_q8, dim3((unsigned) ((nb + 7) / 8)), 256, 0, (cudaStream_t) stream, x, (int8_t *) q, (__half *) d, nb);
+    constexpr int W = CVT_NT / 32;
+    if (n >= CVT_LONG)
+        return launch_pdl(k_quant_q8<CVT_U>, dim3((unsigned) ((nb + W * CVT_U - 1) / (W * CVT_U))), CVT_NT, 0, (cudaStream_t) stream, x, (int8_t *) q,
+                          (__half *) d, nb);
+    return launch_pdl(k_quant_q8<1>, dim3((unsigned) ((nb + W - 1) / W)), CVT_NT, 0, (cudaStream_t) stream, x, (int8_t *) q, (__half *) d, nb);
 }
 
 GS_EXPORT int gs_rope_kv_append_at(const float *kv, void *cache_row0, int64_t pos0, int T, int d_row, int d_rope,

@@ -312,3 +312,21 @@ def test_prefill_checked_leaves_status_clear(pkg, cuda, oracle):
     assert int(st.item()) == 0
     check_close(o.cpu().numpy(), oracle.prefill(Q, K, V, 1 / 16), "prefill (checked entry)")
     assert L.gs_prefill_attn_checked(None, None, None, None, 0, 300, 2, 256, 0, 1 / 16, 2, None, None) == 1
+
+
+@pytest.mark.parametrize("n", [1, 511, (1 << 20) - 32, 1 << 20, (1 << 20) + 4096 + 32])
+def test_conversions_of_short_and_long_runs(pkg, cuda, oracle, n):
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal(n, dtype=np.float32)
+    xd, y = to_dev(cuda, x), cuda.full((n + 8,), 3.0, dtype=cuda.float16, device="cuda")
+    pkg.f32_to_f16(xd, y, n)
+    got = y.cpu().numpy()
+    assert np.array_equal(got[:n], x.astype(np.float16)) and (got[n:] == 3).all()
+    pkg.f32_to_f16(xd[1:], y, n - 1)  # a source aligned to one float
+    assert np.array_equal(y.cpu().numpy()[:n - 1], x[1:].astype(np.float16))
+    if n % 32 == 0:
+        q, d = cuda.zeros(n + 32, dtype=cuda.int8, device="cuda"), cuda.zeros(n // 32 + 1, dtype=cuda.float16, device="cuda")
+        pkg.quant_q8_rows(xd, q, d, n)
+        wq, wd = oracle.quant_q8_rows(x)
+        assert np.array_equal(q.cpu().numpy()[:n], wq) and np.array_equal(d.cpu().numpy()[:n // 32], wd)
+        assert int(q[n:].abs().sum()) == 0 and float(d[n // 32]) == 0
