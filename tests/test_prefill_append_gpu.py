@@ -330,3 +330,17 @@ def test_conversions_of_short_and_long_runs(pkg, cuda, oracle, n):
         wq, wd = oracle.quant_q8_rows(x)
         assert np.array_equal(q.cpu().numpy()[:n], wq) and np.array_equal(d.cpu().numpy()[:n // 32], wd)
         assert int(q[n:].abs().sum()) == 0 and float(d[n // 32]) == 0
+
+
+@pytest.mark.parametrize("T", [2368, 2369, 5000])
+def test_long_appends(pkg, cuda, oracle, T):
+    """A block per row up to 2368 rows, several rows per block beyond."""
+    rng = np.random.default_rng(T)
+    kv = rng.standard_normal((T, 576), dtype=np.float32)
+    cache = cuda.zeros((T + 20, 576), dtype=cuda.float16, device="cuda")
+    pkg.rope_kv_append_at(to_dev(cuda, kv), cache, 7)
+    got = cache.cpu().numpy().astype(np.float32)
+    want = np.asarray(oracle.rope_append(kv, 7)).astype(np.float32)
+    # one f16 rounding of a sum of two products below 2 max|x|; sine and cosine differ by an ulp or two of f32
+    assert np.abs(got[7:7 + T] - want).max() <= np.abs(kv).max() * 2.0 ** -9
+    assert (got[:7] == 0).all() and (got[7 + T:] == 0).all()
