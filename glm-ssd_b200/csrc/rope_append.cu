@@ -299,8 +299,10 @@ __global__ void __launch_bounds__(128) k_stage_append(const AppendParams P, vola
 // the rotated quarter of the rows, read and written once.  (8192 positions x 20 heads x 64 of 256 columns, 42 MB: 46 us with
 // a sincosf and a 4-byte access per pair, 9 us now.)
 constexpr int ROPE_NT = 256;
+// grid (positions / n_pos, head blocks of hb heads)
 template <typename V>  // V: one access, sizeof(V) / 4 pairs
-__global__ void __launch_bounds__(ROPE_NT) k_rope_f16(__half *x, int S, int H, int d, int d_rope, int64_t pos0, int n_pos, const RopeTable tab) {
+__global__ void __launch_bounds__(ROPE_NT) k_rope_f16(__half *x, int S, int H_all, int hb, int d, int d_rope, int64_t pos0, int n_pos,
+                                                      const RopeTable tab) {
     extern __shared__ float2 rope_cs[];  // [n_pos][d_rope / 2] (cos, sin)
     constexpr int PV = sizeof(V) / 4;
     const int s0 = blockIdx.x * n_pos, ns = min(n_pos, S - s0), ppr = d_rope / 2, vpr = ppr / PV;
@@ -313,8 +315,9 @@ __global__ void __launch_bounds__(ROPE_NT) k_rope_f16(__half *x, int S, int H, i
     __syncthreads();
     sm100::griddep_wait();
     sm100::griddep_launch_dependents();
+    const int h0 = blockIdx.y * hb, H = min(hb, H_all - h0);
     const int items = ns * H * vpr;
-    __half *const base = x + (int64_t) s0 * H * d + (d - d_rope);
+    __half *const base = x + ((int64_t) s0 * H_all + h0) * d + (d - d_rope);
     constexpr int U = 4;  // accesses in flight per thread
     for (int i0 = threadIdx.x; i0 < items; i0 += U * ROPE_NT) {
         V v[U];
@@ -323,9 +326,9 @@ __global__ void __launch_bounds__(ROPE_NT) k_rope_f16(__half *x, int S, int H, i
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int i = min(i0 + u * ROPE_NT, items - 1);
-            const int sh = i / vpr, c = i - sh * vpr;  // sh = position * H + head
-            p[u] = reinterpret_cast<V *>(base + (int64_t) sh * d) + c;
-            cs_at[u] = sh / H * ppr + c * PV;
+            const int sh = i / vpr, c = i - sh * vpr, s = sh / H;  // sh = position * H + head
+            p[u] = reinterpret_cast<V *>(base + ((int64_t) s * H_all + (sh - s * H)) * d) + c;
+            cs_at[u] = s * ppr + c * PV;
             v[u] = *p[u];
         }
 #pragma unroll
@@ -340,6 +343,22 @@ __global__ void __launch_bounds__(ROPE_NT) k_rope_f16(__half *x, int S, int H, i
             if (i0 + u * ROPE_NT < items) *p[u] = v[u];
         }
     }
+}
+
+// One head: no angle is used twice, so a thread forms its pair's (before the wait) and there is no table.  (8192 positions x 64
+// columns: 4.9 us with a table.)
+__global__ void __launch_bounds__(ROPE_NT) k_rope_f16_one(__half *x, int64_t n_pairs, int d, int d_rope, int64_t pos0, const RopeTable tab) {
+    const int ppr = d_rope / 2;
+    const int64_t i = (int64_t) blockIdx.x * ROPE_NT + threadIdx.x, s = i / ppr;
+    const int pair = (int) (i - s * ppr);
+    float sn, cs;
+    sincosf((float) (pos0 + s) * tab.inv_freq[pair], &sn, &cs);
+    sm100::griddep_wait();
+    sm100::griddep_launch_dependents();
+    if (i >= n_pairs) return;
+    __half2 *p = reinterpret_cast<__half2 *>(x + s * d + (d - d_rope)) + pair;
+    const float2 r = rotate(__half22float2(*p), cs, sn);
+    *p = __floats2half2_rn(r.x, r.y);
 }
 
 int check_rope(int d_row, int d_rope) {
@@ -472,14 +491,25 @@ GS_EXPORT int gs_rope_f16_inplace(void *x, int S, int H, int d, int d_rope, int6
     if (S <= 0 || H <= 0 || d_rope == 0) return 0;
     RopeTable tab;
     fill_table(tab, d_rope, rope_base);
+    if (H == 1) {
+        const int64_t n_pairs = (int64_t) S * (d_rope / 2);
+        return launch_pdl(k_rope_f16_one, dim3((unsigned) ((n_pairs + ROPE_NT - 1) / ROPE_NT)), ROPE_NT, 0, (cudaStream_t) stream, (__half *) x, n_pairs, d,
+                          d_rope, pos0, tab);
+    }
     // positions per block: enough for a few accesses per thread, fewer when the blocks would not fill the GPU
     int n_pos = 8;
     while (n_pos > 1 && (S + n_pos - 1) / n_pos < 296) n_pos >>= 1;
-    const dim3 grid((S + n_pos - 1) / n_pos);
+    const bool wide = d % 8 == 0 && d_rope % 8 == 0 && !(reinterpret_cast<uintptr_t>(x) & 15);
+    // a few positions of many heads: blocks of as many heads as make one round of accesses (1 position x 128 heads x 128
+    // columns 3.2 us in one block, 2.3 this way)
+    const int blocks = (S + n_pos - 1) / n_pos, per_head = n_pos * (d_rope / (wide ? 8 : 2));
+    int hb = H;
+    if (blocks < 148 && (int64_t) H * per_head > 2 * ROPE_NT) hb = 2 * ROPE_NT / per_head > 0 ? 2 * ROPE_NT / per_head : 1;
+    if ((H + hb - 1) / hb > 65535) hb = (H + 65534) / 65535;
+    const dim3 grid(blocks, (H + hb - 1) / hb);
     const size_t smem = (size_t) n_pos * (d_rope / 2) * sizeof(float2);
-    if (d % 8 == 0 && d_rope % 8 == 0 && !(reinterpret_cast<uintptr_t>(x) & 15))
-        return launch_pdl(k_rope_f16<uint4>, grid, ROPE_NT, smem, (cudaStream_t) stream, (__half *) x, S, H, d, d_rope, pos0, n_pos, tab);
-    return launch_pdl(k_rope_f16<uint32_t>, grid, ROPE_NT, smem, (cudaStream_t) stream, (__half *) x, S, H, d, d_rope, pos0, n_pos, tab);
+    if (wide) return launch_pdl(k_rope_f16<uint4>, grid, ROPE_NT, smem, (cudaStream_t) stream, (__half *) x, S, H, hb, d, d_rope, pos0, n_pos, tab);
+    return launch_pdl(k_rope_f16<uint32_t>, grid, ROPE_NT, smem, (cudaStream_t) stream, (__half *) x, S, H, hb, d, d_rope, pos0, n_pos, tab);
 }
 
 // ---- one decode step of a layer with host buffers ---------------------------------------------------

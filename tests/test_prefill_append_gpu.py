@@ -344,3 +344,19 @@ def test_long_appends(pkg, cuda, oracle, T):
     # one f16 rounding of a sum of two products below 2 max|x|; sine and cosine differ by an ulp or two of f32
     assert np.abs(got[7:7 + T] - want).max() <= np.abs(kv).max() * 2.0 ** -9
     assert (got[:7] == 0).all() and (got[7 + T:] == 0).all()
+
+
+@pytest.mark.parametrize("S,H,d,d_rope", [
+    (1, 1, 64, 64), (300, 1, 64, 64), (9, 1, 130, 6),      # one head: angles per thread
+    (1, 128, 256, 128), (2, 130, 64, 64), (7, 33, 256, 128),  # few positions, heads over several blocks
+    (500, 3, 256, 64), (3000, 2, 66, 10),                  # angles once per position; rows of odd words
+])
+def test_rope_in_place_forms(pkg, cuda, oracle, S, H, d, d_rope):
+    rng = np.random.default_rng(S + H)
+    x = rng.standard_normal((S, H, d), dtype=np.float32).astype(np.float16)
+    xd = to_dev(cuda, x)
+    pkg.rope_f16_inplace(xd, d_rope=d_rope, pos0=77)
+    got, want = xd.cpu().numpy().astype(np.float32), oracle.rope_f16(x, pos0=77, d_rope=d_rope).astype(np.float32)
+    # one f16 rounding of a sum of two products below 2 max|x|; sine and cosine differ by an ulp or two of f32
+    assert np.abs(got - want).max() <= np.abs(x.astype(np.float32)).max() * 2.0 ** -9
+    assert np.array_equal(got[..., :d - d_rope], want[..., :d - d_rope])
