@@ -183,6 +183,11 @@ struct Barriers {
 // NQ <= 48: stages and query rows sized for the widest row (576 columns), one layout for both row widths.  NQ = 64 (only
 // built for 512-column rows): sized by the row width, or two stages, the query rows and P would not fit.
 constexpr int MAX_CLUSTER = 16;
+// f16 lists of up to so many rows are attended by the first CTA of their cluster alone: the exchange costs more than the tiles it
+// saves (20 rows, two tokens, 64 heads: 16 us in a cluster, 12 alone).  Not with a Q8 cache, whose tiles take twice as long and
+// whose kernel has no register to spare for it (65536 rows, two tokens +1 us), nor with 64 query columns, which clusters
+// are hardly ever chosen for.
+constexpr int ALONE_ROWS = 3 * TILE;
 template <int NQ, int NBLK = NBLK_MAX>
 struct Smem {
     static constexpr int SBLK = NQ > 48 ? NBLK : NBLK_MAX;   // 64-column blocks a stage and the query rows are sized for
@@ -201,6 +206,7 @@ struct Smem {
         Barriers bar;
         uint32_t tmem_base;
         int abort_flag;
+        int alone;                         // cluster form: the list is short, the first CTA attends it alone
         int flag[2];
         union {
             struct {
@@ -254,19 +260,20 @@ struct Sched {
     int len0, base0;  // single sequence: its (capped) length and first row
     bool single;
     bool whole;       // sequences are not dealt by rows: CTA c attends sequences c, c + grid, ... from their first row to their
-                      // last, or - share > 1 - every CTA of cluster b the rank-th part of sequence b
-    int share, rank;
+                      // last, or - cluster > 1 - every CTA of cluster b the rank-th part of sequence b, or the
+                      // first one all of it when it is short (alone)
+    int cluster, rank;
 };
 
 // Walks the segments of this CTA's unit range [pos, end); `b` is a cursor over sequences.
 __device__ __forceinline__ bool next_segment(int &pos, int &b, int end, const int *cum, int unit_rows,
-                                             const int *seq_lens, Segment &sg, const Sched &sc) {
+                                             const int *seq_lens, Segment &sg, const Sched &sc, bool alone) {
     if (sc.whole) {
         int len = 0;
-        if (sc.share > 1) {  // an equal share of the sequence's rows, possibly none
+        if (sc.cluster > 1 && !alone) {  // an equal share of the sequence's rows, possibly none
             if (b >= sc.total) return false;
             len = sc.len0;
-            const int per = (len + sc.share - 1) / sc.share;
+            const int per = (len + sc.cluster - 1) / sc.cluster;
             sg.b = b;
             sg.len = len;
             sg.r0 = min(len, sc.rank * per);
@@ -342,6 +349,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
     constexpr int NTHR = LIST ? LIST_NTHREADS : NTHREADS;
     constexpr int NI = issuers_for(NQ);   // issuing MMA warps
     constexpr int O_SLOT0 = 2 * NI;       // first O^T slot in tensor memory
+    constexpr bool ALONE = LIST && !Q8 && NQ <= 48;
     constexpr int STAGE_BYTES = SM::STAGE;
     static_assert((O_SLOT0 + 4) * NQ <= TMEM_COLS, "tensor memory columns");
     extern __shared__ uint8_t smem_raw[];
@@ -413,10 +421,10 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
     }
     // The schedule: units per sequence, their running sum, this CTA's chunk and the sequence it starts in.
     Sched sc;
-    sc.single = P.n_seq == 1;
     sc.whole = LIST && P.whole_seq;
-    sc.share = LIST && P.whole_seq ? P.cluster : 1;
-    sc.rank = sc.share > 1 ? (int) blockIdx.x % sc.share : 0;
+    sc.cluster = LIST ? P.cluster : 1;
+    sc.single = P.n_seq == 1 || (ALONE && sc.cluster > 1);  // one length per CTA, in len0
+    sc.rank = sc.cluster > 1 ? (int) blockIdx.x % sc.cluster : 0;
     sc.total = 0;
     sc.chunk = 1;
     sc.start = sc.end = sc.b0 = 0;
@@ -429,13 +437,13 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
         // are final - the schedule stays monotone and every index derived from it stays in range.
         const int64_t len_cap = min(P.paged ? (int64_t) P.page_table_stride * TILE : P.cache_rows,
                                     (int64_t) 0x7fffffff - 64);  // the rounding up to units below stays in an int
-        if (sc.single) {
+        if (sc.single && sc.cluster == 1) {
             // one sequence: every thread reads the one length word itself and derives its CTA's range in registers
             sc.len0 = (int) min((int64_t) max(ld_global_hint(P.seq_lens, pol_keep), 0), len_cap);
             sc.base0 = P.seq_base ? ld_global_hint(P.seq_base, pol_keep) : 0;
             sc.total = (sc.len0 + unit_rows - 1) / unit_rows;
-        } else if (LIST && sc.share > 1) {  // one sequence per cluster: every thread reads its length itself
-            sc.len0 = (int) min((int64_t) max(ld_global_hint(P.seq_lens + (int) blockIdx.x / sc.share / P.seq_div, pol_keep), 0), len_cap);
+        } else if (LIST && sc.cluster > 1) {  // one sequence per cluster: every thread reads its length itself
+            sc.len0 = (int) min((int64_t) max(ld_global_hint(P.seq_lens + (int) blockIdx.x / sc.cluster / P.seq_div, pol_keep), 0), len_cap);
         } else if (LIST && sc.whole) {  // no units to deal, only the lengths
             for (int b = tid; b < P.n_seq; b += NTHR)
                 M.len[b] = (int) min((int64_t) max(ld_global_hint(P.seq_lens + b / P.seq_div, pol_keep), 0), len_cap);
@@ -474,7 +482,12 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
         sc.b0 = 0;
         if (sc.whole) {  // sequences dealt round-robin; `total` counts sequences, the cursor starts at this CTA's first
             sc.total = P.n_seq;
-            sc.b0 = (int) blockIdx.x / sc.share;
+            sc.b0 = (int) blockIdx.x / sc.cluster;
+            if (ALONE && sc.cluster > 1) {
+                const int alone = sc.len0 <= ALONE_ROWS;  // the same decision in every thread of the cluster
+                M.alone = alone;  // (in shared memory: the softmax warps have no register to spare for it)
+                if (alone && sc.rank > 0) sc.b0 = sc.total;
+            }
             return;
         }
         if (!sc.single) {
@@ -496,7 +509,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
     if (!LIST && warp == 0) {
         int pp = sc.start, bb = sc.b0, asked = 0;
         Segment s2;
-        while (asked < AHEAD && next_segment(pp, bb, sc.end, M.cum, unit_rows, M.len, s2, sc)) {
+        while (asked < AHEAD && next_segment(pp, bb, sc.end, M.cum, unit_rows, M.len, s2, sc, false)) {
             for (int j = 0; j < s2.n_tiles && asked < AHEAD; j++, asked++) {
                 const int row = s2.r0 + j * TILE;
                 int64_t grow = -1;
@@ -516,7 +529,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (LIST && sc.share > 1) cluster_sync();  // every CTA's barriers are initialised before another CTA arrives on them
+    if (LIST && sc.cluster > 1) cluster_sync();  // every CTA's barriers are initialised before another CTA arrives on them
     griddep_wait();
     if (tid == 0) GS_CTA_STAMP(1);
     build_schedule();
@@ -555,7 +568,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
         // The whole warp runs the loop (uniform control flow); one elected lane issues each copy.
         bool ok = true, lane_ok = true;  // (of the warp; of this lane's waits)
         const uint64_t pol_stream = l2_policy_evict_first();  // every cache row is read once per step
-        while (ok && next_segment(pos, b_cur, end, M.cum, unit_rows, M.len, sg, sc)) {
+        while (ok && next_segment(pos, b_cur, end, M.cum, unit_rows, M.len, sg, sc, ALONE && M.alone)) {
             const int64_t base_row = sc.single ? sc.base0 : M.base[sg.b];
             for (int j = 0; ok && j < sg.n_tiles; j++, it++) {
                 const int s = it & 1;
@@ -639,7 +652,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
         const uint64_t d_pt = make_smem_desc(0, 128, 1024, kSwizzleNone);          // P^T, MN-major
         const uint32_t q_lo = smem_desc_addr(q_smem), p_lo0 = smem_desc_addr(p_smem), kv_lo0 = smem_desc_addr(kv_smem);
         bool ok = true, lane_ok = true;  // (of the warp; of this lane's waits)
-        while (ok && next_segment(pos, b_cur, end, M.cum, unit_rows, M.len, sg, sc)) {
+        while (ok && next_segment(pos, b_cur, end, M.cum, unit_rows, M.len, sg, sc, ALONE && M.alone)) {
             if (LIST && sg.n_tiles == 0) continue;  // (cluster form: no share of the rows)
             lane_ok &= bar_wait<LIST>(&B.q_full, sgc & 1, abort_flag, status_w, ST_MMA);
             // S of tile j+1 is issued ahead of P.V of tile j whenever its data has already landed, so it
@@ -708,6 +721,8 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                     }
                 }
                 // ---- O^T[my tiles] += V^T . P^T ----
+                ok = __all_sync(0xffffffffu, !gave_up(lane_ok));  // (here, where the softmax is still at work)
+                if (!ok) break;
                 lane_ok &= bar_wait<LIST>(&B.p_full[s], ph, abort_flag, status_w, ST_MMA);
                 // P.V reads every value block of the tile: all groups (they have landed: the scores the softmax
                 // just turned into P needed them; the waits return at once and make that landing visible here)
@@ -732,7 +747,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                         umma_commit(&B.q_empty);
                     }
                 }
-                ok = __all_sync(0xffffffffu, !gave_up(lane_ok));
+                __syncwarp();
                 if (mw == 0 && lane == 0) GS_STAMP(it, PF_PV_ISSUED);
             }
             sgc++;
@@ -755,15 +770,15 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
         float l_part[HQ];                             // row sums of this thread's cache row, per query row
         float nm[HQ];                                 // minus the reference maximum (log2 units) per query row
         bool ok = true, lane_ok = true;               // (of the group; of this lane's waits)
-        if (LIST && sc.whole && sc.share == 1) {
+        if (LIST && sc.whole && (sc.cluster == 1 || (ALONE && M.alone))) {
             // a query that attends nothing gets zeros (crates/cuda/kernels/ops.cu:535); such sequences yield no segment
-            for (int b = (int) blockIdx.x; b < P.n_seq; b += (int) gridDim.x) {
+            for (int b = sc.b0; b < P.n_seq; b += (int) gridDim.x) {
                 if ((sc.single ? sc.len0 : M.len[b]) > 0) continue;
                 float *dst = P.o + ((int64_t) (b / P.seq_div) * P.H_out + (b % P.seq_div) * P.H) * P.d_v;
                 for (int i = wg_tid; i < P.rows_q * P.d_v; i += 128) dst[i] = 0.f;
             }
         }
-        while (ok && next_segment(pos, b_cur, end, M.cum, unit_rows, M.len, sg, sc)) {
+        while (ok && next_segment(pos, b_cur, end, M.cum, unit_rows, M.len, sg, sc, ALONE && M.alone)) {
             if (LIST && sg.n_tiles > 0) {
                 // f32 queries: the four warps round this sequence's rows to f16 straight into the operand layout the
                 // TMA would have produced (64-column blocks of [NQ rows][128 bytes], 16-byte chunk j of row r at chunk
@@ -979,7 +994,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                 if ((lane & 15) == 0) M.sl[qt][col0 + i] = v;
             }
             named_bar_sync(1, 128);
-            if (LIST && sc.share > 1) {
+            if (LIST && sc.cluster > 1 && !(ALONE && M.alone)) {
                 // ---- the CTAs of the cluster merge their parts through distributed shared memory -----------------------
                 // Every CTA tells all others that its MMAs are done with its stages, stages its accumulators column block
                 // by column block, and sends each CTA its 512 / cluster columns (and everybody its (m, l)) by bulk copies;
@@ -987,7 +1002,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                 // ops.cu:552-574), and stores them.
                 // (About 5 us for 16 CTAs x 64 KB, half of it the copies at 27 GB/s per SM.  With 4-byte stores to the other CTAs instead of bulk copies 6.4 us, with
                 // 16-byte stores a row apart 9 us, and 3.3 us more for exchanging the maxima first.)
-                const int share = sc.share, cols = 512 / share;
+                const int share = sc.cluster, cols = 512 / share;
                 float *const x_acc = reinterpret_cast<float *>(kv_smem), *const x_out = reinterpret_cast<float *>(smem + SM::OFF_XOUT);
                 // "ready" of a round: this CTA takes the copies of the round and has everything of the round before, so that the
                 // others may fill their staging area again (one round up to 48 query rows, two for 64)
@@ -1158,7 +1173,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
         // two 183, four 166 us, four through registers 228 us.)
         const int pw = warp - 8;
         bool ok = true, lane_ok = true;  // (of the warp; of this lane's waits)
-        while (ok && next_segment(pos, b_cur, end, M.cum, unit_rows, M.len, sg, sc)) {
+        while (ok && next_segment(pos, b_cur, end, M.cum, unit_rows, M.len, sg, sc, ALONE && M.alone)) {
             const int32_t *lp = P.sel + (int64_t) (sg.b / P.seq_div) * P.sel_stride + sg.r0;
             const int n_rows = sg.r1 - sg.r0;
             int n_left = n_rows;
@@ -1230,15 +1245,26 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                     lane_ok &= bar_wait<LIST>(&B.kv_empty[s], ((it >> 1) & 1) ^ 1, abort_flag, status_w, ST_PRODUCER);
                     if (pw == 0 && lane == 0) GS_STAMP(it, PF_LOAD_ISSUE);
                     const char *cbase = reinterpret_cast<const char *>(P.list_cache) + lane * 16;
+                    auto place = [&](int r, int h) {
+                        const int c = h * 32 + lane;
+                        return dst + (c >> 3) * BLK_BYTES + r * 128 + (((c & 7) ^ (r & 7)) << 4);
+                    };
+                    if (n_left >= TILE) {
 #pragma unroll
-                    for (int k = 0; k < RPW; k++) {
-                        const int r = k * 4 + pw;
-                        const char *src = cbase + row_of(r) * (NBLK * 128);
+                        for (int k = 0; k < RPW; k++) {
+                            const int r = k * 4 + pw;
+                            const char *src = cbase + row_of(r) * (NBLK * 128);
 #pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            const int c = h * 32 + lane;
-                            // (rows past the segment's end become zeros; their entries name row 0, which is not read)
-                            cp_async16_or_zero(dst + (c >> 3) * BLK_BYTES + r * 128 + (((c & 7) ^ (r & 7)) << 4), src + h * 512, r < n_left);
+                            for (int h = 0; h < 2; h++) cp_async16(place(r, h), src + h * 512);
+                        }
+                    } else {
+                        // rows past the segment's end become zeros; their entries name row 0, which is not read
+#pragma unroll 1
+                        for (int k = 0; k < RPW; k++) {
+                            const int r = k * 4 + pw;
+                            const char *src = cbase + row_of(r) * (NBLK * 128);
+#pragma unroll
+                            for (int h = 0; h < 2; h++) cp_async16_or_zero(place(r, h), src + h * 512, r < n_left);
                         }
                     }
                     cp_async_mbar_arrive(&B.kv_full[s][0]);
@@ -1260,7 +1286,7 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
         }
     }
     __syncthreads();
-    if (LIST && sc.share > 1) cluster_sync();  // no CTA leaves while another may still write to its shared memory
+    if (LIST && sc.cluster > 1) cluster_sync();  // no CTA leaves while another may still write to its shared memory
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, TMEM_COLS);
@@ -1322,11 +1348,13 @@ struct ListPlan {
 //  * a cluster of 2 to 16 CTAs per sequence, which merge through distributed shared memory - when all clusters run at once;
 //  * the rows of all sequences dealt to CTAs as in the dense form, records in `part` (as many segments as its
 //    T*H*splits*(R+2) floats hold), a combine launch - long lists with a large `part`.
-// The estimate: a CTA's longest run of 64-row tiles times the time of a tile, plus what the merge costs.  Measured over 2052-row
-// lists, 1 to 256 tokens, 16 to 64 heads, every cut (f16 / Q8 cache): a tile 2.2 / 3.0 us with up to 32 query columns and
-// 2.85 / 3.4 with 64, 2.5 and 3.1 in a cluster; a cluster's start and merge 7.5 / 9.5 us, 17 with 64 columns (two rounds of the
-// exchange), 2.5 more with 16 CTAs and a little for every CTA that fetches; records and their combine 11 us, 7 when there is one sequence (its schedule needs no
-// scan).  The choice it makes is within about 6 % of the best cut measured.
+// The estimate, in microseconds: what a list of one tile takes, which follows the query rows of the group (their conversion, and
+// the exchange or the merge), and a time per further tile of the longest run, which grows a little with the CTAs at
+// work.  Fitted to lists of 20 to 2052 rows, 1 to 256 tokens, 16 to 64 heads, f16 and Q8 (f16, first tile: one CTA 10 to 14,
+// a cluster 13.2 / 15.2 / 19.6 / 24.8 with up to 16 / 32 / 48 / 64 query rows, records 10.4 / 10.6 / 13.4 / 15.9 when there is one
+// sequence, whose schedule needs no scan, else 15.6).  The host knows the stride and not the lengths: it plans for lists as long
+// as the stride, and short ones in clusters are left to one CTA on the device (ALONE_ROWS).  One token, 64 heads, 2052
+// rows: 18.3 us in four groups, 19.3 in one.
 // Clusters and the combine store o in 16-byte words; an o that is not aligned for them (`o_aligned`) leaves one CTA per sequence,
 // which stores single words.
 static ListPlan list_plan(int T, int H, int R, int sel_stride, int splits, const float *part, bool o_aligned, bool q8, int grid_max,
@@ -1340,16 +1368,19 @@ static ListPlan list_plan(int T, int H, int R, int sel_stride, int splits, const
         const int Hg = H / n;
         const int64_t n_seq_k = (int64_t) T * n, tiles_seq = (sel_stride + TILE - 1) / TILE;
         if (n_seq_k > MAX_SEQ) break;
-        const float t_one = (Hg <= 32 ? 2.2f : Hg <= 48 ? 2.5f : 2.85f) + (q8 ? (Hg <= 48 ? 0.8f : 0.55f) : 0.f);
-        const float t_cl = (Hg <= 32 ? 2.5f : Hg <= 48 ? 2.8f : 3.1f) + (q8 ? 0.2f : 0.f);
+        const int w = Hg <= 16 ? 0 : Hg <= 32 ? 1 : Hg <= 48 ? 2 : 3;
+        static const float one_first[2][4] = {{9.5f, 9.8f, 11.5f, 14.f}, {12.f, 12.f, 14.f, 16.5f}};
+        static const float cl_first[2][4] = {{13.2f, 15.2f, 19.6f, 24.8f}, {12.9f, 14.9f, 19.4f, 24.9f}};
+        static const float rec_first[2][4] = {{10.4f, 10.6f, 13.4f, 15.9f}, {12.5f, 12.5f, 14.8f, 17.6f}};
+        static const float tile[2][4] = {{1.35f, 1.35f, 1.5f, 1.85f}, {2.8f, 2.8f, 2.8f, 2.85f}};
+        auto further = [&](int64_t tiles, int64_t ctas) { return (float) (tiles > 1 ? tiles - 1 : 0) * (tile[q8][w] + 0.0035f * (float) ctas); };
         const int64_t grid = n_seq_k < grid_max ? n_seq_k : grid_max;
-        offer(n, grid, 1, true, (float) ((n_seq_k + grid - 1) / grid * tiles_seq) * t_one + 2.f);
+        offer(n, grid, 1, true, one_first[q8][w] + further((n_seq_k + grid - 1) / grid * tiles_seq, grid));
         for (int c = 2, i = 1; o_aligned && c <= MAX_CLUSTER; c *= 2, i++) {
             // all clusters have to run at once (148 SMs: 148, 132, 120 and 112 CTAs in clusters of 2, 4, 8 and 16)
             if (n_seq_k * c > (room.ctas[i] < grid_max ? room.ctas[i] : grid_max)) continue;
             const int64_t per = (sel_stride + c - 1) / c;
-            offer(n, n_seq_k * c, c, true, (float) ((per + TILE - 1) / TILE) * t_cl + (Hg <= 48 ? 6.5f + 0.03f * (float) Hg : 17.f) +
-                                               (c == 16 ? 2.5f : 0.f) + (q8 ? 2.f : 0.f) + 0.03f * (float) (n_seq_k * c));
+            offer(n, n_seq_k * c, c, true, cl_first[q8][w] + further((per + TILE - 1) / TILE, n_seq_k * c) + (c == 16 ? 1.f : 0.f));
         }
         if (o_aligned && splits > 1 && part && !(reinterpret_cast<uintptr_t>(part) & 15)) {
             // records that fit the caller's buffer
@@ -1360,7 +1391,7 @@ static ListPlan list_plan(int T, int H, int R, int sel_stride, int splits, const
             int64_t g = segs - n_seq_k;
             if (g > grid_max) g = grid_max;
             if (g > tiles) g = tiles;
-            if (g > 0) offer(n, g, 1, false, (float) ((tiles + g - 1) / g) * t_cl + (n_seq_k == 1 ? 7.f : 11.f) + (q8 ? 2.f : 0.f));
+            if (g > 0) offer(n, g, 1, false, (n_seq_k == 1 ? rec_first[q8][w] : 15.6f) + further((tiles + g - 1) / g, g));
         }
     }
     return best;

@@ -289,6 +289,8 @@ def test_gs_mla_attn_tensor_kernel_vs_oracle_and_cuda_core_kernel(pkg, cuda, ora
     (32, 64, [65 * i for i in range(32)], 2052),          # 64 query columns in a cluster: two rounds of the exchange
     (33, 48, [63 + i for i in range(33)], 130),           # 48 columns, clusters of 4 with less than a tile each
     (60, 64, [900 + i for i in range(60)], 960),          # clusters of 2
+    (2, 64, [64, 65], 2052),             # around the lengths one CTA of a cluster attends alone (f16)
+    (3, 32, [192, 193, 1], 2052),
 ])
 def test_gs_mla_attn_list_cuts(pkg, cuda, oracle, q8, T, H, cnts, stride):
     """One call per way of dealing (token, head group) lists to CTAs and clusters, single split: no part buffer at all."""
