@@ -1245,26 +1245,15 @@ __global__ void __launch_bounds__(LIST ? LIST_NTHREADS : NTHREADS, 1) k_decode_u
                     lane_ok &= bar_wait<LIST>(&B.kv_empty[s], ((it >> 1) & 1) ^ 1, abort_flag, status_w, ST_PRODUCER);
                     if (pw == 0 && lane == 0) GS_STAMP(it, PF_LOAD_ISSUE);
                     const char *cbase = reinterpret_cast<const char *>(P.list_cache) + lane * 16;
-                    auto place = [&](int r, int h) {
-                        const int c = h * 32 + lane;
-                        return dst + (c >> 3) * BLK_BYTES + r * 128 + (((c & 7) ^ (r & 7)) << 4);
-                    };
-                    if (n_left >= TILE) {
 #pragma unroll
-                        for (int k = 0; k < RPW; k++) {
-                            const int r = k * 4 + pw;
-                            const char *src = cbase + row_of(r) * (NBLK * 128);
+                    for (int k = 0; k < RPW; k++) {
+                        const int r = k * 4 + pw;
+                        const char *src = cbase + row_of(r) * (NBLK * 128);
 #pragma unroll
-                            for (int h = 0; h < 2; h++) cp_async16(place(r, h), src + h * 512);
-                        }
-                    } else {
-                        // rows past the segment's end become zeros; their entries name row 0, which is not read
-#pragma unroll 1
-                        for (int k = 0; k < RPW; k++) {
-                            const int r = k * 4 + pw;
-                            const char *src = cbase + row_of(r) * (NBLK * 128);
-#pragma unroll
-                            for (int h = 0; h < 2; h++) cp_async16_or_zero(place(r, h), src + h * 512, r < n_left);
+                        for (int h = 0; h < 2; h++) {
+                            const int c = h * 32 + lane;
+                            // (rows past the segment's end become zeros; their entries name row 0, which is not read)
+                            cp_async16_or_zero(dst + (c >> 3) * BLK_BYTES + r * 128 + (((c & 7) ^ (r & 7)) << 4), src + h * 512, r < n_left);
                         }
                     }
                     cp_async_mbar_arrive(&B.kv_full[s][0]);
