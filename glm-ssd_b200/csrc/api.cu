@@ -192,7 +192,7 @@ GS_EXPORT int gs_mla_attn(const float *q, const void *C, const void *C_scales, c
     DecodeProblem p{};
     if (int e = device_sm_count(&p.sm_count)) return e;
     // The tcgen05 kernel's producer warps fetch the listed rows themselves (f16 rows, or int8 rows and their scales, which
-    // the kernel widens in shared memory) and the kernel rounds the queries to f16 itself; it needs nothing beyond the
+    // they widen on the way into shared memory) and the kernel rounds the queries to f16 itself; it needs nothing beyond the
     // reference's own arguments.  Shapes it does not take run on the CUDA-core kernel below.
     const int impl = g_attn_impl.load(std::memory_order_relaxed);
     if (impl != 1) {

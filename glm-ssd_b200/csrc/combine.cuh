@@ -26,17 +26,12 @@ struct CombineSmem {
     float4 part[CB_LANES][CB_COLS / 4];
 };
 
-// Address helpers of the generalised record layout (see CombinePlan).
-__device__ __forceinline__ int64_t combine_row_stride_acc(const CombinePlan &C) { return C.row_stride_acc ? C.row_stride_acc : C.d_v; }
-__device__ __forceinline__ int64_t combine_chunk_stride_acc(const CombinePlan &C) { return C.chunk_stride_acc ? C.chunk_stride_acc : CB_COLS; }
-__device__ __forceinline__ int64_t combine_row_stride_ml(const CombinePlan &C) { return C.row_stride_ml ? C.row_stride_ml : 2; }
-// column `col` of row `row_in_seg` of segment `seg`
+// Column `col` of row `row_in_seg` of segment `seg`, and that row's (m, l) pair.
 __device__ __forceinline__ const float *combine_acc_ptr(const CombinePlan &C, int64_t seg, int row_in_seg, int col) {
-    return C.acc + seg * C.seg_stride_acc + (int64_t) row_in_seg * combine_row_stride_acc(C) +
-           (int64_t) (col / CB_COLS) * combine_chunk_stride_acc(C) + (col % CB_COLS);
+    return C.acc + seg * C.seg_stride_acc + (int64_t) row_in_seg * C.d_v + col;
 }
 __device__ __forceinline__ const float *combine_ml_ptr(const CombinePlan &C, int64_t seg, int row_in_seg) {
-    return C.ml + seg * C.seg_stride_ml + (int64_t) row_in_seg * combine_row_stride_ml(C);
+    return C.ml + seg * C.seg_stride_ml + (int64_t) row_in_seg * 2;
 }
 
 // Where the segments of output row `row` lie.

@@ -46,11 +46,7 @@ struct CombinePlan {
     int regular_segments;  // desc == nullptr: segments per (sequence, token) group, consecutive
     int64_t seg_stride_acc;  // floats between the accumulator blocks of consecutive segments
     int64_t seg_stride_ml;   // floats between the (m, l) blocks of consecutive segments
-    // Generalised addressing (0 = the plain record layout [segment][row][d_v] / [segment][row][2]): column c of row r of
-    // segment s lies at acc + s*seg_stride_acc + r*row_stride_acc + (c/128)*chunk_stride_acc + c%128, its (m, l) pair at
-    // ml + s*seg_stride_ml + r*row_stride_ml.  The tcgen05 kernel keeps its records as [row][128-column chunk][segment][128],
-    // so that everything one (row, chunk) item of the combine needs is one contiguous run of memory.
-    int64_t row_stride_acc, chunk_stride_acc, row_stride_ml;
+    // column c of row r of segment s lies at acc + s*seg_stride_acc + r*d_v + c, its (m, l) pair at ml + s*seg_stride_ml + r*2
     bool bulk;             // fetch an item's accumulators with one tiled TMA copy into shared memory (k_combine_bulk)
     int n_segments;        // bulk: segments the record arrays hold (extent of the tensor map)
     int n_seq, T, H, d_v;  // H: heads in the records being merged
